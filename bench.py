@@ -687,7 +687,7 @@ def run_dynamic27(args):
 
 def run_big29(args, force_exact):
     """n = 2^29 (beyond one FP32 pass), fresh seed per block: 2^27-bit FP32 chunk blocks under the
-    residual guard, or (force_exact) the exact NTT path."""
+    residual guard, or (force_exact) the exact path."""
     import numpy as np
     import torch
     import privacyamplification_gb300 as pa
@@ -721,7 +721,7 @@ def run_big29(args, force_exact):
         ev1.synchronize()
     st = eng.sync(check=False)
     t = ev0.elapsed_time(ev1) / 1e3
-    path = "exact NTT path mod 3*2^30+1" if force_exact else "FP32 path in 2^27-bit chunk blocks, residual guard"
+    path = "exact path over GF(2)" if force_exact else "FP32 path in 2^27-bit chunk blocks, residual guard"
     _line(METRIC, args.steps * n / t / 1e9, UNIT, args.steps, args.warmup, t / args.steps * 1e3,
           "n=2^29 (h=n/2+n/8, v=n/4+n/8), dynamic seed, " + path,
           {"exact": st.exact, "max_residual": st.max_residual, "clocks": clk.summary(),

@@ -18,8 +18,8 @@
  *     (PrivacyAmplification.cu:1197).
  *   - Result: out[i] = (sum_{j=0..h} key_start[j] * seed[(i-j) mod n] mod 2) XOR key_rest[i].
  *   - Precision: the FP32 FFT path measures every block's largest distance of an output value to the
- *     nearest integer; above residual_limit pa_process recomputes the block on the exact integer
- *     (NTT mod 3*2^30+1) path.  Blocks with n > 2^27 (up to 2^30) run as 2^27-bit FP32 chunk blocks
+ *     nearest integer; above residual_limit pa_process recomputes the block on the exact path, which
+ *     forms the product over GF(2) itself (additive FFT).  Blocks with n > 2^27 (up to 2^30) run as 2^27-bit FP32 chunk blocks
  *     (large-block decomposition) under the same guard.
  *
  * All functions return 0 (PA_OK) or a negative PA_ERR_* code; nothing exits the process.
@@ -50,7 +50,7 @@ extern "C" {
 
 #define PA_FLAG_XOR_KEY_REST 1u   /* do_xor_key_rest (config.yaml, key-server message) */
 #define PA_FLAG_COMPRESS 2u       /* do_compress */
-#define PA_FLAG_EXACT 4u          /* force the exact integer (NTT) path for this block */
+#define PA_FLAG_EXACT 4u          /* force the exact (GF(2)) path for this block */
 
 typedef struct pa_engine pa_engine;
 

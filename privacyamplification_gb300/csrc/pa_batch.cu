@@ -79,7 +79,7 @@ struct Slot {
     int cap = 0;  // log2 of the largest cyclic length the buffers hold
     size_t bytes = 0;
     cudaStream_t s = nullptr;
-    float2* work = nullptr;   // pass A output / exact-path residues
+    float2* work = nullptr;   // pass A output / exact-path elements
     float2* work2 = nullptr;  // pass B output / exact-path scratch
     float2* spec = nullptr;   // dynamic seed spectrum / exact seed transform
     uint32_t* planes = nullptr;
@@ -90,7 +90,6 @@ struct Slot {
     Mirror* host = nullptr;
     pa::PassMaps maps{};
     int maps_key = -1;
-    pa::NttTables* ntt = nullptr;
     cudaEvent_t done = nullptr, join = nullptr;
     // served block in flight
     bool busy = false;
@@ -209,7 +208,6 @@ void free_slot(Pool* p, Slot* sl) {
     cudaFree(sl->kr);
     cudaFree(sl->out);
     cudaFreeHost(sl->host);
-    pa::free_ntt_tables(sl->ntt);
     if (sl->done) cudaEventDestroy(sl->done);
     if (sl->join) cudaEventDestroy(sl->join);
     if (sl->s) cudaStreamDestroy(sl->s);
@@ -356,8 +354,8 @@ int exact_in_slot(pa_engine* e, Slot* sl, const BlockGeom& g, const uint32_t* d_
     uint32_t* hat = reinterpret_cast<uint32_t*>(sl->spec);
     uint32_t* a = reinterpret_cast<uint32_t*>(sl->work);
     uint32_t* tmp = reinterpret_cast<uint32_t*>(sl->work2);
-    int rc = pa::launch_exact_seed(g, d_seed, hat, tmp, &sl->ntt, s);
-    if (!rc) rc = pa::launch_exact_block(g, ks, kr, flags, hat, a, tmp, out, &sl->ntt, s);
+    int rc = pa::launch_exact_seed(g, d_seed, hat, tmp, s);
+    if (!rc) rc = pa::launch_exact_block(g, ks, kr, flags, hat, a, tmp, out, s);
     return rc ? cuda_fail(e, (cudaError_t)rc) : PA_OK;
 }
 

@@ -46,7 +46,7 @@ int make_geom(uint32_t n, uint32_t v, uint32_t flags, const int8_t* split, Block
         if (l2 < split_min(g->log_n) || l2 > split_max(g->log_n)) l2 = split_default(g->log_n);
         g->log_n2 = l2;  // rows 2^10..2^14, columns 2^5..2^12
         g->log_n1 = g->log_n - g->log_n2;
-    } else {  // beyond the FP32 path: exact NTT only
+    } else {  // beyond the one-pass FP32 path: chunk blocks or the exact path
         g->log_n1 = g->log_n2 = 0;
         g->exact_only = 1;
         if (g->log_np > 30) return PA_ERR_TOO_LARGE;
@@ -60,11 +60,16 @@ bool same_seed_geom(const BlockGeom& a, const BlockGeom& b) {
     return a.seed_direct == b.seed_direct && a.h == b.h;
 }
 
+bool same_exact_geom(const BlockGeom& a, const BlockGeom& b) {
+    return a.n == b.n && a.h == b.h && a.out_bits == b.out_bits;
+}
+
 }  // namespace pa_host
 
 namespace {
 
 using pa_host::make_geom;
+using pa_host::same_exact_geom;
 using pa_host::same_seed_geom;
 
 int ensure_maps(pa_engine* e, const BlockGeom& g) {
@@ -78,7 +83,7 @@ int ensure_maps(pa_engine* e, const BlockGeom& g) {
 pa::Scratch scratch(pa_engine* e) { return {e->d_work, e->d_work2, e->d_planes, e->d_err, &e->maps}; }
 
 int build_exact_seed(pa_engine* e, const BlockGeom& g, cudaStream_t s) {
-    int rc = pa::launch_exact_seed(g, e->d_seed, e->d_exact_seed, reinterpret_cast<uint32_t*>(e->d_work2), &e->ntt, s);
+    int rc = pa::launch_exact_seed(g, e->d_seed, e->d_exact_seed, reinterpret_cast<uint32_t*>(e->d_work2), s);
     if (rc) return cuda_fail(e, (cudaError_t)rc);
     e->exact_geom = g;
     e->exact_valid = true;
@@ -183,15 +188,15 @@ int chunked_block(pa_engine* e, const uint32_t* d_ks, const uint32_t* d_kr, cons
     return PA_OK;
 }
 
-// Exact path for one block (the seed's NTT is built on first use and cached with the seed).
+// Exact path for one block (the seed's transform is built on first use and cached with the seed).
 int exact_block(pa_engine* e, const uint32_t* d_ks, const uint32_t* d_kr, const BlockGeom& g, uint32_t flags,
                 uint32_t* d_out, cudaStream_t s) {
-    if (!e->exact_valid || !same_seed_geom(e->exact_geom, g)) {
+    if (!e->exact_valid || !same_exact_geom(e->exact_geom, g)) {
         int rc = build_exact_seed(e, g, s);
         if (rc) return rc;
     }
     int rc = pa::launch_exact_block(g, d_ks, d_kr, flags, e->d_exact_seed, reinterpret_cast<uint32_t*>(e->d_work),
-                                    reinterpret_cast<uint32_t*>(e->d_work2), d_out, &e->ntt, s);
+                                    reinterpret_cast<uint32_t*>(e->d_work2), d_out, s);
     if (rc) return cuda_fail(e, (cudaError_t)rc);
     // the exact path leaves no residual: report 0 and the reference popcounts are not needed
     PA_CUDA(e, cudaMemsetAsync(e->d_resid, 0, sizeof(unsigned int), s));
@@ -385,7 +390,6 @@ void pa_destroy(pa_engine* e) {
     cudaFree(e->d_work);
     cudaFree(e->d_spec);
     cudaFree(e->d_exact_seed);
-    pa::free_ntt_tables(e->ntt);
     cudaFree(e->d_work2);
     cudaFree(e->d_err);
     cudaFree(e->d_planes);

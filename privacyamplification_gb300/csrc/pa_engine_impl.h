@@ -35,8 +35,7 @@ struct pa_engine {
     float2* d_work2 = nullptr;  // pass B output (tile-major)
     float2* d_spec = nullptr;
     int* d_err = nullptr;       // device error word of the bounded TMA waits
-    uint32_t* d_exact_seed = nullptr;  // NTT of the placed seed (exact path), Np words
-    pa::NttTables* ntt = nullptr;      // exact-path twiddle tables
+    uint32_t* d_exact_seed = nullptr;  // the seed's transform (exact path), Np words
     bool exact_valid = false;          // d_exact_seed matches the current seed for exact_geom
     bool last_exact = false;           // the last block ran on the exact path
     bool last_chunked = false;         // the last block ran as FP32 chunk blocks (n > 2^27)
@@ -114,6 +113,8 @@ inline int split_default(int log_n) {
 int make_geom(uint32_t n, uint32_t v, uint32_t flags, const int8_t* split, pa::BlockGeom* g);
 // Two geometries whose seed spectra are interchangeable (placement and layout).
 bool same_seed_geom(const pa::BlockGeom& a, const pa::BlockGeom& b);
+// Two geometries whose exact-path seed transforms are interchangeable (the windows start at -h).
+bool same_exact_geom(const pa::BlockGeom& a, const pa::BlockGeom& b);
 // Key used to cache tensor maps: (log_n, log_n2).
 inline int maps_key(const pa::BlockGeom& g) { return g.log_n * 32 + g.log_n2; }
 

@@ -15,7 +15,7 @@ struct BlockGeom {
     int log_n;             // complex length N = Np/2
     int log_n1, log_n2;    // three-pass split N = N1 * N2 (0, 0 for the single-CTA path)
     uint32_t seed_direct;  // seed positions < seed_direct map to themselves (see seed_source)
-    int exact_only;        // 1: beyond the FP32 path (n > 2^27), only the exact NTT path applies
+    int exact_only;        // 1: beyond one pass of the FP32 path (n > 2^27): chunk blocks or the exact path
 };
 
 // Seed placement in the cyclic length Np.  For Np == n this is the identity.  For a padded Np the
@@ -160,14 +160,14 @@ int launch_pass_c(const BlockGeom& g, const PassMaps& maps, const float2* Z, con
 int launch_finish(const BlockGeom& g, const uint32_t* planes, const uint32_t* key_rest, uint32_t flags,
                   uint32_t* out, cudaStream_t s, const Group& gp = kOneBlock);
 
-// Exact path (pa_ntt.cu): integer convolution modulo 3*2^30+1.  seed_hat, a, tmp: Np words each.
-struct NttTables;
-void free_ntt_tables(NttTables* t);
-int launch_exact_seed(const BlockGeom& g, const uint32_t* seed, uint32_t* seed_hat, uint32_t* tmp,
-                      NttTables** tables, cudaStream_t s);
+// Exact path (pa_exact.cu): the product over GF(2) by an additive FFT, or for short blocks (direct_geom,
+// pa_direct.cu) word by word.  seed_hat, a, tmp: Np words each; seed_hat holds for the same n, h and out_bits.
+int launch_exact_seed(const BlockGeom& g, const uint32_t* seed, uint32_t* seed_hat, uint32_t* tmp, cudaStream_t s);
 int launch_exact_block(const BlockGeom& g, const uint32_t* key_start, const uint32_t* key_rest, uint32_t flags,
-                       const uint32_t* seed_hat, uint32_t* a, uint32_t* tmp, uint32_t* out_words, NttTables** tables,
-                       cudaStream_t s);
+                       const uint32_t* seed_hat, uint32_t* a, uint32_t* tmp, uint32_t* out_words, cudaStream_t s);
+bool direct_geom(const BlockGeom& g);
+int launch_direct(const BlockGeom& g, const uint32_t* seed, const uint32_t* key_start, const uint32_t* key_rest,
+                  uint32_t flags, uint32_t* out_words, cudaStream_t s);
 int exact_kernel_count(const BlockGeom& g);
 
 // Blocks beyond the single-pass FP32 size (pa_chunk.cu): side x side chunk blocks (n' = 2 side) on the

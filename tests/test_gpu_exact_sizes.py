@@ -1,0 +1,44 @@
+"""The exact path (PA_FLAG_EXACT) at the edges of its forms, whole outputs against the exact CPU oracle: the
+word-by-word product of short blocks (one and eight result words per CTA, a partial last word, the key's last bit
+in a word of its own), its boundary at 2^34 bit products, and every transform length's split into passes (2^16
+points and up), with odd sizes, extreme ratios and every flag."""
+import numpy as np
+import pytest
+
+import privacyamplification_gb300 as pa
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+DEFAULT = pa.DEFAULT_FLAGS
+# (n, v, flags)
+SHORT = [(1024, 32, DEFAULT), (1024, 992, DEFAULT), (1056, 480, 0), (2080, 1024, pa.FLAG_XOR_KEY_REST),
+         (19200, 19168, DEFAULT), (19264, 19232, DEFAULT), (65536, 24576, DEFAULT), (65568, 40032, pa.FLAG_COMPRESS),
+         (100000, 32, DEFAULT), (262144, 98304, DEFAULT), (262144, 131072, 0)]
+# around the boundary: (h + 1) v <= 2^34 is word by word; then 2^16 .. 2^21 points
+LONG = [(262144, 131040, DEFAULT), (262176, 131104, DEFAULT), (524288, 196608, DEFAULT), (786432, 32768, 0),
+        (1048576, 524288, DEFAULT), (1048608, 524320, DEFAULT), (3000032, 1000032, DEFAULT),
+        (4194304, 1572864, pa.FLAG_COMPRESS), (4194336, 4128768, pa.FLAG_XOR_KEY_REST), (8388608, 3145728, DEFAULT),
+        (16777248, 6291456, 0), (33554432, 12582912, DEFAULT)]
+
+
+@pytest.mark.parametrize("n,v,flags", SHORT + LONG)
+def test_exact_flag_whole_output(gpu_engine, n, v, flags):
+    seed, recv = O.random_block(n, v, n % 9973 + v + flags)
+    ks, kr = O.key_split(recv, n, v)
+    gpu_engine.set_seed(seed, n, -1)
+    out = gpu_engine.process(ks, kr, n, v, flags | pa.FLAG_EXACT)
+    assert gpu_engine.last_stats.exact == 1
+    assert np.array_equal(out, O.ntt(seed, ks, kr, n, v, flags))
+
+
+@pytest.mark.parametrize("n", [65536, 1048576])
+def test_exact_seed_transform_follows_the_output_length(gpu_engine, n):
+    """One static seed, blocks of different v: the exact path's seed transform depends on h and the output length."""
+    v1, v2 = n // 4, n // 2
+    seed, recv = O.random_block(n, v1, 77)
+    gpu_engine.set_seed(seed, n, -1)
+    for v, flags in ((v1, DEFAULT), (v2, DEFAULT), (v1, pa.FLAG_XOR_KEY_REST), (v1, DEFAULT)):
+        ks, kr = O.key_split(recv, n, v)
+        out = gpu_engine.process(ks, kr, n, v, flags | pa.FLAG_EXACT)
+        assert np.array_equal(out, O.ntt(seed, ks, kr, n, v, flags))
