@@ -870,7 +870,14 @@ int launch_exact_seed(const BlockGeom& g, const uint32_t* seed, uint32_t* seed_h
 
 int launch_exact_block(const BlockGeom& g, const uint32_t* key_start, const uint32_t* key_rest, uint32_t flags,
                        const uint32_t* seed_hat, uint32_t* a, uint32_t* tmp, uint32_t* out_words, cudaStream_t s) {
-    if (direct_geom(g)) return launch_direct(g, seed_hat, key_start, key_rest, flags, out_words, s);
+    if (direct_geom(g)) {
+        if (direct_overlap(g, key_start, out_words)) {  // every result word reads the whole key
+            cudaError_t err = cudaMemcpyAsync(a, key_start, 4u * (size_t)(g.h / 32u + 1u), cudaMemcpyDeviceToDevice, s);
+            if (err != cudaSuccess) return (int)err;
+            key_start = a;
+        }
+        return launch_direct(g, seed_hat, key_start, key_rest, flags, out_words, s);
+    }
     const Shape sh = shape_of(g);
     const size_t half = size_t(16) * sh.pw;
     k_exact_planes<false><<<(sh.pw + 127u) / 128u, 128, 0, s>>>(key_start, g, sh.pw, tmp);

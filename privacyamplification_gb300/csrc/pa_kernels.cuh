@@ -166,6 +166,7 @@ int launch_exact_seed(const BlockGeom& g, const uint32_t* seed, uint32_t* seed_h
 int launch_exact_block(const BlockGeom& g, const uint32_t* key_start, const uint32_t* key_rest, uint32_t flags,
                        const uint32_t* seed_hat, uint32_t* a, uint32_t* tmp, uint32_t* out_words, cudaStream_t s);
 bool direct_geom(const BlockGeom& g);
+bool direct_overlap(const BlockGeom& g, const uint32_t* key_start, const uint32_t* out_words);
 int launch_direct(const BlockGeom& g, const uint32_t* seed, const uint32_t* key_start, const uint32_t* key_rest,
                   uint32_t flags, uint32_t* out_words, cudaStream_t s);
 int exact_kernel_count(const BlockGeom& g);

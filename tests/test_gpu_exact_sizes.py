@@ -42,3 +42,20 @@ def test_exact_seed_transform_follows_the_output_length(gpu_engine, n):
         ks, kr = O.key_split(recv, n, v)
         out = gpu_engine.process(ks, kr, n, v, flags | pa.FLAG_EXACT)
         assert np.array_equal(out, O.ntt(seed, ks, kr, n, v, flags))
+
+
+@pytest.mark.parametrize("n,v,where", [(1024, 384, "key"), (4096, 1536, "seed"), (32768, 12288, "key"),
+                                       (32768, 32736, "key_rest"), (20480, 7680, "seed")])
+def test_noalloc_output_over_an_input(n, v, where):
+    """The result may be written over the seed, the key or key_rest: every input is read first."""
+    torch = pytest.importorskip("torch")
+    seed, recv = O.random_block(n, v, n + v)
+    ks, kr = O.key_split(recv, n, v)
+    bufs = {k: torch.from_numpy(np.ascontiguousarray(a, dtype=np.uint32).view(np.int32).copy()).cuda()
+            for k, a in (("seed", seed), ("key", ks), ("key_rest", kr))}
+    torch.cuda.synchronize()
+    pa.process_noalloc(bufs["seed"].data_ptr(), bufs["key"].data_ptr(), bufs["key_rest"].data_ptr(), n, v,
+                       bufs[where].data_ptr())
+    torch.cuda.synchronize()
+    got = bufs[where].cpu().numpy().view(np.uint8)[: v // 8]
+    assert np.array_equal(got, O.direct(seed, ks, kr, n, v))
