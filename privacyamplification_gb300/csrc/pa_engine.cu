@@ -142,7 +142,7 @@ int fused_block(pa_engine* e, const uint32_t* d_ks, const uint32_t* d_kr, const 
 
 // n > 2^27: the block as 2^27-bit FP32 chunk blocks (pa_chunk.cu).  The exact seed transform's buffer
 // is the chunks' staging area and the chunk spectra go through d_spec, so both caches are invalidated.
-// Block popcounts are not formed on this path (read_stats reports 0).
+// Block popcounts are not formed on this path (take_stats reports 0).
 //
 // Two lanes take the diagonals in turn.  The second lane's three-pass buffers are the upper halves of
 // d_work / d_work2 (each holds Np / 2 >= 2^27 complex here, a chunk block needs 2^26); its staging, bit
@@ -258,26 +258,22 @@ int block_common(pa_engine* e, const uint32_t* d_ks, const uint32_t* d_kr, const
     return PA_OK;
 }
 
-int read_stats(pa_engine* e, pa_stats* st, float* resid_out) {
-    unsigned long long cnt[2] = {0, 0};
-    unsigned int rb = 0;
-    PA_CUDA(e, cudaMemcpy(cnt, e->d_cnt, sizeof(cnt), cudaMemcpyDeviceToHost));
-    PA_CUDA(e, cudaMemcpy(&rb, e->d_resid, sizeof(rb), cudaMemcpyDeviceToHost));
-    int derr = 0;
-    PA_CUDA(e, cudaMemcpy(&derr, e->d_err, sizeof(derr), cudaMemcpyDeviceToHost));
-    if (derr) {  // a bounded device wait expired: the block's result is not valid
+// Statistics from the block's words on the host (h_words); `s` has finished.
+int take_stats(pa_engine* e, pa_stats* st, float* resid_out) {
+    const pa_engine::Words w = *e->h_words;
+    if (w.err) {  // a bounded device wait expired: the block's result is not valid
         cudaMemset(e->d_err, 0, sizeof(int));
         e->last_cuda = (int)cudaErrorLaunchTimeout;
         return PA_ERR_CUDA;
     }
     float resid;
-    std::memcpy(&resid, &rb, sizeof(resid));
+    std::memcpy(&resid, &w.resid, sizeof(resid));
     *resid_out = resid;
     if (st) {
         st->max_residual = resid;
         const bool counted = !e->last_exact && !e->last_chunked;  // popcounts exist on the one-pass FP32 path
-        st->popcount_key = counted ? cnt[0] : 0;
-        st->popcount_seed = counted ? cnt[1] : 0;
+        st->popcount_key = counted ? w.cnt[0] : 0;
+        st->popcount_seed = counted ? w.cnt[1] : 0;
         float ms = 0.f;
         cudaEventElapsedTime(&ms, e->ev0, e->ev1);
         st->gpu_ms = ms;
@@ -362,18 +358,19 @@ int pa_create(const pa_config* cfg, pa_engine** out) {
     if ((err = cudaMalloc(&e->d_spec, (np_fp32 / 2) * sizeof(float2))) != cudaSuccess) return fail(err);
     if ((err = cudaMalloc(&e->d_exact_seed, np * sizeof(uint32_t))) != cudaSuccess) return fail(err);
     if ((err = cudaMalloc(&e->d_work2, (np / 2) * sizeof(float2))) != cudaSuccess) return fail(err);
-    if ((err = cudaMalloc(&e->d_err, sizeof(int))) != cudaSuccess) return fail(err);
-    cudaMemset(e->d_err, 0, sizeof(int));
+    if ((err = cudaMalloc(&e->d_words, sizeof(pa_engine::Words))) != cudaSuccess) return fail(err);
+    cudaMemset(e->d_words, 0, sizeof(pa_engine::Words));
+    e->d_cnt = e->d_words->cnt;
+    e->d_resid = &e->d_words->resid;
+    e->d_err = &e->d_words->err;
+    if ((err = cudaMallocHost((void**)&e->h_words, 64 + pa_engine::kStageBytes)) != cudaSuccess) return fail(err);
+    e->h_stage = reinterpret_cast<uint8_t*>(e->h_words) + 64;
     if ((err = cudaMalloc(&e->d_planes, np_fp32 / 8 + 256)) != cudaSuccess) return fail(err);
-    if ((err = cudaMalloc(&e->d_cnt, 2 * sizeof(unsigned long long))) != cudaSuccess) return fail(err);
-    if ((err = cudaMalloc(&e->d_resid, sizeof(unsigned int))) != cudaSuccess) return fail(err);
     if (e->cap_log_np >= 21) {  // blocks with columns of 2^10 and more: the fused column pass's park
         // one spectrum tile per CTA: two CTAs per SM, at most one per tile of the largest block
         e->park_ctas = std::min<uint32_t>(2u * (uint32_t)e->num_sms, (uint32_t)((np / 2) / 8192u));
         if ((err = cudaMalloc(&e->d_park, e->park_ctas * pa::kParkBytes)) != cudaSuccess) return fail(err);
     }
-    cudaMemset(e->d_cnt, 0, 2 * sizeof(unsigned long long));
-    cudaMemset(e->d_resid, 0, sizeof(unsigned int));
     *out = e;
     return PA_OK;
 }
@@ -391,10 +388,9 @@ void pa_destroy(pa_engine* e) {
     cudaFree(e->d_spec);
     cudaFree(e->d_exact_seed);
     cudaFree(e->d_work2);
-    cudaFree(e->d_err);
+    cudaFree(e->d_words);
+    cudaFreeHost(e->h_words);
     cudaFree(e->d_planes);
-    cudaFree(e->d_cnt);
-    cudaFree(e->d_resid);
     cudaFree(e->d_park);
     for (auto& a : e->tev)
         for (auto ev : a) cudaEventDestroy(ev);
@@ -458,38 +454,50 @@ int pa_process(pa_engine* e, const uint32_t* key_start, const uint32_t* key_rest
     PA_CUDA(e, cudaSetDevice(e->device));
     cudaStream_t s = e->stream;
     PA_CUDA(e, cudaMemcpyAsync(e->d_key_start, key_start, (size_t)(g.h / 32u + 1u) * 4u, cudaMemcpyHostToDevice, s));
-    // key_rest is first read by the block's last kernel: it is copied on the side stream (after
-    // whatever the engine stream had queued) while the passes run
+    // key_rest is first read by the block's last kernel: a long one is copied on the side stream (after
+    // whatever the engine stream had queued) while the passes run; a short one costs less than the events
     cudaEvent_t kr_ready = nullptr;
-    if (flags & PA_FLAG_XOR_KEY_REST) {
+    const size_t kr_bytes = (size_t)(v / 32u) * 4u;
+    if ((flags & PA_FLAG_XOR_KEY_REST) && kr_bytes <= pa_engine::kStageBytes) {
+        PA_CUDA(e, cudaMemcpyAsync(e->d_key_rest, key_rest, kr_bytes, cudaMemcpyHostToDevice, s));
+    } else if (flags & PA_FLAG_XOR_KEY_REST) {
         PA_CUDA(e, cudaEventRecord(e->main_ready, s));
         PA_CUDA(e, cudaStreamWaitEvent(e->side, e->main_ready, 0));
-        PA_CUDA(e, cudaMemcpyAsync(e->d_key_rest, key_rest, (size_t)(v / 32u) * 4u, cudaMemcpyHostToDevice, e->side));
+        PA_CUDA(e, cudaMemcpyAsync(e->d_key_rest, key_rest, kr_bytes, cudaMemcpyHostToDevice, e->side));
         PA_CUDA(e, cudaEventRecord(e->kr_ready, e->side));
         kr_ready = e->kr_ready;
     }
     rc = block_common(e, e->d_key_start, e->d_key_rest, g, flags, e->d_out, s, kr_ready);
     if (rc) {
-        if (kr_ready) cudaStreamSynchronize(e->side);  // the caller's key_rest is not read after we return
+        cudaStreamSynchronize(kr_ready ? e->side : s);  // the caller's key_rest is not read after we return
         return rc;
     }
-    size_t ob = pa_output_bytes(n, v, flags);
-    PA_CUDA(e, cudaStreamSynchronize(s));
+    // The words, and a short result, come back behind the kernels and are waited for once; the caller's buffer is
+    // written when the words say that the result holds (a 2^16-bit call: 111 -> 88 us; it was a wait, three copies of
+    // a word and one of the result, each a round trip).
+    const size_t ob = pa_output_bytes(n, v, flags);
+    const bool staged = ob <= pa_engine::kStageBytes;
+    auto collect = [&](pa_stats* st, float* resid) -> int {
+        PA_CUDA(e, cudaMemcpyAsync(e->h_words, e->d_words, sizeof(pa_engine::Words), cudaMemcpyDeviceToHost, s));
+        if (staged) PA_CUDA(e, cudaMemcpyAsync(e->h_stage, e->d_out, ob, cudaMemcpyDeviceToHost, s));
+        PA_CUDA(e, cudaStreamSynchronize(s));
+        return take_stats(e, st, resid);
+    };
     float resid = 0.f;
-    rc = read_stats(e, stats, &resid);
+    rc = collect(stats, &resid);
     if (rc) return rc;
     if (!(resid <= e->residual_limit)) {
         // FP32 rounding budget exceeded: recompute this block exactly (same inputs, same seed use)
         if (e->seed_left >= 0) ++e->seed_left;
         rc = block_common(e, e->d_key_start, e->d_key_rest, g, flags | PA_FLAG_EXACT, e->d_out, s);
         if (rc) return rc;
-        PA_CUDA(e, cudaStreamSynchronize(s));
         float r2 = 0.f;
-        rc = read_stats(e, stats, &r2);
+        rc = collect(stats, &r2);
         if (rc) return rc;
         if (stats) stats->max_residual = resid;  // report what the FP32 path measured
     }
-    PA_CUDA(e, cudaMemcpy(out, e->d_out, ob, cudaMemcpyDeviceToHost));
+    if (staged) std::memcpy(out, e->h_stage, ob);
+    else PA_CUDA(e, cudaMemcpy(out, e->d_out, ob, cudaMemcpyDeviceToHost));
     return PA_OK;
 }
 
@@ -512,8 +520,9 @@ int pa_sync(pa_engine* e, pa_stats* stats) {
     PA_CUDA(e, cudaSetDevice(e->device));
     PA_CUDA(e, cudaDeviceSynchronize());
     e->pending = false;
+    PA_CUDA(e, cudaMemcpy(e->h_words, e->d_words, sizeof(pa_engine::Words), cudaMemcpyDeviceToHost));
     float resid = 0.f;
-    int rc = read_stats(e, stats, &resid);
+    int rc = take_stats(e, stats, &resid);
     if (rc) return rc;
     return resid <= e->residual_limit ? PA_OK : PA_ERR_PRECISION;
 }

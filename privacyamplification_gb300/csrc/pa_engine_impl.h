@@ -34,7 +34,7 @@ struct pa_engine {
     float2* d_work = nullptr;   // pass A output (row-major)
     float2* d_work2 = nullptr;  // pass B output (tile-major)
     float2* d_spec = nullptr;
-    int* d_err = nullptr;       // device error word of the bounded TMA waits
+    int* d_err = nullptr;       // device error word of the bounded TMA waits (in d_words)
     uint32_t* d_exact_seed = nullptr;  // the seed's transform (exact path), Np words
     bool exact_valid = false;          // d_exact_seed matches the current seed for exact_geom
     bool last_exact = false;           // the last block ran on the exact path
@@ -54,8 +54,19 @@ struct pa_engine {
     float2* d_park = nullptr;
     uint32_t park_ctas = 0;
     uint32_t* d_planes = nullptr;
-    unsigned long long* d_cnt = nullptr;  // [0] key popcount, [1] seed popcount
-    unsigned int* d_resid = nullptr;
+    // a block's words, in one allocation (d_words) that one copy brings to the host
+    struct Words {
+        unsigned long long cnt[2];  // key popcount, seed popcount
+        unsigned int resid;         // largest residual (float bits)
+        int err;                    // bounded device waits that expired
+    };
+    Words* d_words = nullptr;
+    unsigned long long* d_cnt = nullptr;  // d_words->cnt
+    unsigned int* d_resid = nullptr;      // &d_words->resid
+    // pinned: the words, then short results (kStageBytes), which are handed over once the words are read
+    static constexpr size_t kStageBytes = size_t(256) << 10;
+    Words* h_words = nullptr;
+    uint8_t* h_stage = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     // seed state
     bool seed_valid = false;
