@@ -40,8 +40,7 @@ int launch_pass_b_fused_k(dim3 grid, size_t smem_base, size_t box, int max_early
     }();
     const size_t bytes = smem_base + (size_t)early * box;
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    kernel<<<grid, 256, bytes, s>>>(mapYs, mapY, Z, g, park, err, early);
-    return (int)cudaGetLastError();
+    return (int)launch_pdl(kernel, grid, 256, bytes, s, mapYs, mapY, Z, g, park, err, early);
 }
 
 #define PA_FUSED_B(LG)                                                                                           \

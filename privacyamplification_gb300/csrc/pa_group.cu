@@ -27,14 +27,9 @@ template <int LOGL>
 int launch_pass_b_group(bool seed, dim3 grid, size_t smem, const CUtensorMap& mapY, float2* Y, float2* Z,
                         float2* spec, const BlockGeom& g, int* err, int early, const Group& gp, cudaStream_t s) {
     if (!gp.e) return (int)cudaErrorInvalidValue;
-    if (seed) {
-        cudaFuncSetAttribute(k_pass_b_group<LOGL, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k_pass_b_group<LOGL, true><<<grid, 256, smem, s>>>(mapY, Y, Z, g, spec, err, early, gp);
-    } else {
-        cudaFuncSetAttribute(k_pass_b_group<LOGL, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k_pass_b_group<LOGL, false><<<grid, 256, smem, s>>>(mapY, Y, Z, g, spec, err, early, gp);
-    }
-    return (int)cudaGetLastError();
+    auto kernel = seed ? k_pass_b_group<LOGL, true> : k_pass_b_group<LOGL, false>;
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return (int)launch_pdl(kernel, grid, 256, smem, s, mapY, Y, Z, g, spec, err, early, gp);
 }
 
 #define PA_GROUP_B(LG)                                                                                            \

@@ -16,6 +16,7 @@
 //       finish    bit planes -> reference byte order, XOR key_rest
 #include "pa_device.cuh"
 #include "pa_kernels.cuh"
+#include "pa_launch.cuh"
 
 #include <algorithm>
 
@@ -130,6 +131,7 @@ __global__ void __launch_bounds__(NT) k_mono_seed(const uint32_t* __restrict__ s
                                                   float2* __restrict__ spec, unsigned long long* cnt_seed, Group gp) {
     extern __shared__ float2 sm[];
     __shared__ unsigned long long red[32];
+    pdl_wait();
     if (gp.e) {
         seed = gp.e[blockIdx.x].seed;
         spec += (size_t)blockIdx.x * gp.work;
@@ -165,6 +167,7 @@ __global__ void __launch_bounds__(NT) k_mono_key(const uint32_t* __restrict__ ke
     __shared__ unsigned long long red[32];
     __shared__ float redf[32];
     __shared__ float s_corr;
+    pdl_wait();
     if (gp.e) {
         const GroupEntry& en = gp.e[blockIdx.x];
         key_start = en.key_start;
@@ -225,7 +228,7 @@ __global__ void __launch_bounds__(NT) k_mono_key(const uint32_t* __restrict__ ke
         }
     }
     float bm = block_max(res, redf);
-    if (threadIdx.x == 0) atomicMax(resid_bits, __float_as_uint(bm));
+    if (threadIdx.x == 0) *resid_bits = __float_as_uint(bm);  // one CTA is the whole block
 }
 
 // ============================================================================ host launchers
@@ -243,8 +246,7 @@ static int mono_seed(const BlockGeom& g, const uint32_t* seed, float2* spec, uns
     constexpr int NT = mono_threads<N>();
     size_t smem = (size_t)Padded<N>::value * sizeof(float2);
     set_smem(k_mono_seed<N, NT>, smem);
-    k_mono_seed<N, NT><<<gp.count, NT, smem, s>>>(seed, g, spec, cnt_seed, gp);
-    return (int)cudaGetLastError();
+    return (int)launch_pdl(k_mono_seed<N, NT>, gp.count, NT, smem, s, seed, g, spec, cnt_seed, gp);
 }
 
 template <int N>
@@ -254,8 +256,7 @@ static int mono_key(const BlockGeom& g, const uint32_t* ks, const uint32_t* kr, 
     constexpr int NT = mono_threads<N>();
     size_t smem = (size_t)Padded<N>::value * sizeof(float2);
     set_smem(k_mono_key<N, NT>, smem);
-    k_mono_key<N, NT><<<gp.count, NT, smem, s>>>(ks, kr, g, flags, spec, cnt, resid, out, gp);
-    return (int)cudaGetLastError();
+    return (int)launch_pdl(k_mono_key<N, NT>, gp.count, NT, smem, s, ks, kr, g, flags, spec, cnt, resid, out, gp);
 }
 
 #define PA_DISPATCH_MONO(L, CALL)          \
@@ -276,8 +277,7 @@ int launch_seed_spectrum(const BlockGeom& g, const uint32_t* seed, float2* spec,
         PA_DISPATCH_MONO(g.log_n, C)
 #undef C
     }
-    cudaMemsetAsync(cnt_seed, 0, sizeof(unsigned long long), s);
-    int rc = launch_bit_rows(g, seed, true, sc.planes, s);
+    int rc = launch_bit_rows(g, seed, true, sc.planes, s, kOneBlock, cnt_seed);
     if (!rc) rc = launch_pass_a(g, sc.planes, true, sc.work, cnt_seed, num_sms, s);
     if (!rc) rc = launch_pass_b(g, true, *sc.maps, sc.work, sc.work2, spec, sc.err, num_sms, s);
     return rc;
@@ -289,7 +289,6 @@ int launch_key_block(const BlockGeom& g, const uint32_t* key_start, const uint32
     auto mark = [&](int i) {
         if (ev) cudaEventRecord(ev[i], s);
     };
-    cudaMemsetAsync(resid_bits, 0, sizeof(unsigned int), s);
     if (g.log_n1 == 0) {
         if (key_rest_ready) cudaStreamWaitEvent(s, key_rest_ready, 0);
         mark(0);
@@ -300,9 +299,8 @@ int launch_key_block(const BlockGeom& g, const uint32_t* key_start, const uint32
         mark(1);
         return rc;
     }
-    cudaMemsetAsync(cnt, 0, sizeof(unsigned long long), s);  // key popcount; cnt[1] is the seed's
     mark(0);
-    int rc = launch_bit_rows(g, key_start, false, sc.planes, s);
+    int rc = launch_bit_rows(g, key_start, false, sc.planes, s, kOneBlock, cnt, resid_bits);  // cnt[1] is the seed's
     if (!rc) rc = launch_pass_a(g, sc.planes, false, sc.work, cnt, num_sms, s);
     mark(1);
     if (!rc) rc = launch_pass_b(g, false, *sc.maps, sc.work, sc.work2, const_cast<float2*>(spec), sc.err, num_sms, s);
@@ -323,12 +321,10 @@ int launch_fused_block(const BlockGeom& g, const uint32_t* seed, const uint32_t*
     auto mark = [&](int i) {
         if (ev) cudaEventRecord(ev[i], s);
     };
-    cudaMemsetAsync(resid_bits, 0, sizeof(unsigned int), s);
-    cudaMemsetAsync(cnt, 0, 2 * sizeof(unsigned long long), s);  // key and seed popcounts
     mark(0);
-    int rc = launch_bit_rows(g, seed, true, sc.planes, s);
+    int rc = launch_bit_rows(g, seed, true, sc.planes, s, kOneBlock, cnt + 1);
     if (!rc) rc = launch_pass_a(g, sc.planes, true, seed_y, cnt + 1, num_sms, s);
-    if (!rc) rc = launch_bit_rows(g, key_start, false, sc.planes, s);
+    if (!rc) rc = launch_bit_rows(g, key_start, false, sc.planes, s, kOneBlock, cnt, resid_bits);
     if (!rc) rc = launch_pass_a(g, sc.planes, false, sc.work, cnt, num_sms, s);
     mark(1);
     if (!rc) rc = launch_pass_b_fused(g, seed_maps, *sc.maps, sc.work2, park, park_ctas, sc.err, num_sms, s);

@@ -123,8 +123,10 @@ int launch_group_mono_key(const BlockGeom& g, const Group& gp, uint32_t flags, c
 // Three-pass kernels (pa_passes.cu).  `rows` and the parity planes share one buffer of Np/8 bytes.
 // With a group, the pointer arguments are the group's bases (rows, Y, Z, the own spectra) or are
 // replaced by the entries (bits, key_rest, out, cnt, resid, the key pass's spectrum).
+// zero_cnt, zero_resid (may be null): words of the block that this first kernel clears.
 int launch_bit_rows(const BlockGeom& g, const uint32_t* bits, bool seed, uint32_t* rows, cudaStream_t s,
-                    const Group& gp = kOneBlock);
+                    const Group& gp = kOneBlock, unsigned long long* zero_cnt = nullptr,
+                    unsigned int* zero_resid = nullptr);
 int launch_pass_a(const BlockGeom& g, const uint32_t* rows, bool seed, float2* Y, unsigned long long* cnt,
                   int num_sms, cudaStream_t s, const Group& gp = kOneBlock);
 struct PassMaps {

@@ -1,0 +1,36 @@
+// pa_launch.cuh -- programmatic dependent launch of a block's kernels.
+//
+// A block is a chain of kernels that each need the whole of the one before.  Launched with programmatic stream
+// serialisation, a kernel's CTAs take the SMs as its predecessor's leave, compute their twiddle tables and set up
+// their barriers, and wait in pdl_wait() for the predecessor to finish: the launch gap and the prologue run under
+// the predecessor's tail.  Every kernel launched so calls pdl_wait() before its first access to data of the block,
+// reads and writes alike, so that completion is transitive along the chain; in a kernel launched otherwise it does
+// nothing.  The trigger is the implicit one, a CTA's exit: with an explicit one at the kernels' start, the
+// successors' waiting CTAs took shared memory and warp slots from the running kernel (n = 2^27: 909 us a block
+// without early launches, 922 with the explicit trigger, 897 with the implicit one; 2^20: 56.7, 48.9, 45.3 us; a
+// batch of 64 uneven blocks: 6.15, 6.24, 5.94 ms).
+#pragma once
+#include <cuda_runtime.h>
+
+namespace pa {
+
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... P, class... A>
+inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    const cudaError_t err = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    if (err != cudaSuccess) cudaGetLastError();  // reported here, not by a later call
+    return err;
+}
+
+}  // namespace pa

@@ -17,6 +17,7 @@
 #include "pa_device.cuh"
 #include "pa_fft.cuh"
 #include "pa_kernels.cuh"
+#include "pa_launch.cuh"
 #include "pa_tma.cuh"
 
 namespace pa {
@@ -150,8 +151,9 @@ __device__ __forceinline__ void pass_a_rows(const uint32_t* __restrict__ rows, c
             else t2[b][i - 16 - T1N] = w;
         }
     };
-    fetch_row(first, 0);
     row_tables(first, 0);
+    pdl_wait();  // the bit rows; Y may still be read by the block before
+    fetch_row(first, 0);
     int buf = 0;
     for (uint32_t m1 = first; m1 < n1; m1 += stride, buf ^= 1) {
         cp_async_wait_group<0>();  // this thread's copy of row m1 (the only one in flight) has landed
@@ -411,6 +413,7 @@ __device__ __forceinline__ void pass_b_tiles(const CUtensorMap* mapY, const floa
     }
     __syncthreads();
     uint32_t parity_spec = 0;
+    pdl_wait();  // pass A's rows, the spectrum; Z may still be read by the block before
     fence_proxy_async();
     load_tile((int)first, FUSED ? mapYs : mapY);
     for (int unit = (int)first; unit < nunits; unit += (int)stride) {
@@ -768,6 +771,7 @@ __device__ __forceinline__ void pass_c_rows(const CUtensorMap* mapZ, const float
         for (int q = 0; q < QL; ++q) tws[q][t] = w[q];
         if (P::NSTAGE == 2) fill_stage_table<P::RB, 16, +1>(tab2);
     }
+    pdl_wait();  // pass B's tiles and the popcounts; the planes are the bit rows that pass A read
     float corr;
     {
         unsigned long long ck = cnt[0], cs = cnt[1];

@@ -16,9 +16,22 @@
 #include <cudaTypedefs.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 
 namespace pa {
+
+// A block's popcount and residual words, cleared by its first kernel (later kernels add to them).
+struct Zeroed {
+    unsigned long long* cnt;
+    unsigned int* resid;
+    __device__ __forceinline__ void clear() const {
+        if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) {
+            if (cnt) *cnt = 0ull;
+            if (resid) *resid = 0u;
+        }
+    }
+};
 
 // ============================================================================ bit-plane transposes
 // Input bit planes.  Warp (a, c): rows m1 = 16a .. 16a+15, columns m2 = 32c .. 32c+31 (lane = m2 - 32c).
@@ -27,7 +40,9 @@ namespace pa {
 // 32c + 16h .. 32c + 16h + 15 -- one word of the row plane.
 template <bool SEED>
 __global__ void __launch_bounds__(256) k_bit_rows(const uint32_t* __restrict__ src, BlockGeom g,
-                                                  uint32_t* __restrict__ rows, Group gp) {
+                                                  uint32_t* __restrict__ rows, Zeroed z, Group gp) {
+    pdl_wait();
+    z.clear();
     if (gp.e) {  // block blockIdx.z of a group
         src = SEED ? gp.e[blockIdx.z].seed : gp.e[blockIdx.z].key_start;
         rows += (size_t)blockIdx.z * gp.planes;
@@ -60,8 +75,10 @@ __global__ void __launch_bounds__(256) k_bit_rows(const uint32_t* __restrict__ s
 // transpose on distinct banks.  SEED with a padded Np: each word comes from its placed source word.
 template <bool SEED>
 __global__ void __launch_bounds__(256) k_bit_rows_tiled(const uint32_t* __restrict__ src, BlockGeom g,
-                                                        uint32_t* __restrict__ rows, Group gp) {
+                                                        uint32_t* __restrict__ rows, Zeroed z, Group gp) {
     __shared__ uint32_t tile[256][17];  // [m2 - m20][a - a0], then [m1 - 16 a0][(m2 - m20) / 16]
+    pdl_wait();
+    z.clear();
     if (gp.e) {
         src = SEED ? gp.e[blockIdx.z].seed : gp.e[blockIdx.z].key_start;
         rows += (size_t)blockIdx.z * gp.planes;
@@ -154,6 +171,7 @@ __global__ void __launch_bounds__((1 << LOGL) / 32, 1)
 __global__ void __launch_bounds__(1024) k_finish(const uint32_t* __restrict__ planes, BlockGeom g,
                                                  const uint32_t* __restrict__ key_rest, uint32_t flags,
                                                  uint32_t* __restrict__ out, uint32_t nwords, Group gp) {
+    pdl_wait();
     if (gp.e) {  // block blockIdx.z of a group
         planes += (size_t)blockIdx.z * gp.planes;
         key_rest = gp.e[blockIdx.z].key_rest;
@@ -190,6 +208,7 @@ __global__ void __launch_bounds__(256) k_finish_tiled(const uint32_t* __restrict
                                                       uint32_t* __restrict__ out, uint32_t nwords, Group gp) {
     __shared__ uint32_t se[256][9], so[256][9];  // [m1 - m10][c - c0], even / odd samples
     __shared__ uint32_t sw[256][17];             // [m2 - 32 c0][(m1 - m10) / 16]
+    pdl_wait();
     if (gp.e) {
         planes += (size_t)blockIdx.z * gp.planes;
         key_rest = gp.e[blockIdx.z].key_rest;
@@ -272,18 +291,16 @@ static int group_ctas(uint32_t units, int per_wave, const Group& gp) {
 }
 
 int launch_bit_rows(const BlockGeom& g, const uint32_t* bits, bool seed, uint32_t* rows, cudaStream_t s,
-                    const Group& gp) {
+                    const Group& gp, unsigned long long* zero_cnt, unsigned int* zero_resid) {
+    const Zeroed z{zero_cnt, zero_resid};
     const uint32_t n1 = 1u << g.log_n1, n2 = 1u << g.log_n2;
     if (n1 >= 256u && n2 >= 256u) {
         dim3 grid(n1 / 256u, n2 / 256u, gp.count);
-        if (seed) k_bit_rows_tiled<true><<<grid, 256, 0, s>>>(bits, g, rows, gp);
-        else k_bit_rows_tiled<false><<<grid, 256, 0, s>>>(bits, g, rows, gp);
-        return (int)cudaGetLastError();
+        return (int)launch_pdl(seed ? k_bit_rows_tiled<true> : k_bit_rows_tiled<false>, grid, 256, 0, s, bits, g, rows,
+                               z, gp);
     }
     dim3 grid((n1 / 16u + 7u) / 8u, n2 / 32u, gp.count);
-    if (seed) k_bit_rows<true><<<grid, 256, 0, s>>>(bits, g, rows, gp);
-    else k_bit_rows<false><<<grid, 256, 0, s>>>(bits, g, rows, gp);
-    return (int)cudaGetLastError();
+    return (int)launch_pdl(seed ? k_bit_rows<true> : k_bit_rows<false>, grid, 256, 0, s, bits, g, rows, z, gp);
 }
 
 template <int LOGL>
@@ -297,11 +314,9 @@ static int pass_a_l(const BlockGeom& g, const uint32_t* rows, bool seed, float2*
         smem_attr(kernel, smem);
         static const int per_sm = resident_ctas(kernel, NT, smem);
         const dim3 grid(group_ctas(1u << g.log_n1, num_sms * per_sm, gp), gp.count);
-        kernel<<<grid, NT, smem, s>>>(rows, g, Y, cnt, gp);
+        return (int)launch_pdl(kernel, grid, NT, smem, s, rows, g, Y, cnt, gp);
     };
-    if (seed) go(k_pass_a<LOGL, true>);
-    else go(k_pass_a<LOGL, false>);
-    return (int)cudaGetLastError();
+    return seed ? go(k_pass_a<LOGL, true>) : go(k_pass_a<LOGL, false>);
 }
 
 // Pass B's shared memory without the early boxes: tile / exchange buffer, column tables, stage bases, and
@@ -346,14 +361,9 @@ static int pass_b_l(const BlockGeom& g, bool seed, const PassMaps& maps, float2*
     const int early = seed ? early_seed : early_key;
     const size_t bytes = smem + (size_t)early * box;
     if (gp.e) return launch_pass_b_group<LOGL>(seed, grid, bytes, maps.y, Y, Z, spec, g, err, early, gp, s);
-    if (seed) {
-        smem_attr(k_pass_b<LOGL, true>, bytes);
-        k_pass_b<LOGL, true><<<grid, 256, bytes, s>>>(maps.y, Y, Z, g, spec, err, early);
-    } else {
-        smem_attr(k_pass_b<LOGL, false>, bytes);
-        k_pass_b<LOGL, false><<<grid, 256, bytes, s>>>(maps.y, Y, Z, g, spec, err, early);
-    }
-    return (int)cudaGetLastError();
+    auto kernel = seed ? k_pass_b<LOGL, true> : k_pass_b<LOGL, false>;
+    smem_attr(kernel, bytes);
+    return (int)launch_pdl(kernel, grid, 256, bytes, s, maps.y, Y, Z, g, spec, err, early);
 }
 
 // Per-block shared memory limit of the current device (opt-in maximum).
@@ -395,10 +405,13 @@ static int pass_c_k(const BlockGeom& g, const PassMaps& maps, const float2* Z, c
     const size_t box_bytes = (size_t)(ntiles < 256u ? ntiles : 256u) * cpt * sizeof(float2);
     const size_t smem = exch + (size_t)early * box_bytes;
     smem_attr(k_pass_c<LOGL, KEEP8>, smem);
-    const int per_sm = resident_ctas(k_pass_c<LOGL, KEEP8>, NT, smem);  // smem depends on the geometry
+    // by the number of early boxes and the box size (pass B's tile width), which fix the shared memory
+    static std::atomic<int> resident[33][16];
+    std::atomic<int>& known = resident[early][g.log_n1 & 15];
+    int per_sm = known.load(std::memory_order_relaxed);
+    if (!per_sm) known.store(per_sm = resident_ctas(k_pass_c<LOGL, KEEP8>, NT, smem), std::memory_order_relaxed);
     const dim3 grid(group_ctas(1u << g.log_n1, num_sms * per_sm, gp), gp.count);
-    k_pass_c<LOGL, KEEP8><<<grid, NT, smem, s>>>(maps.z, Z, g, cnt, planes, resid, err, early, gp);
-    return (int)cudaGetLastError();
+    return (int)launch_pdl(k_pass_c<LOGL, KEEP8>, grid, NT, smem, s, maps.z, Z, g, cnt, planes, resid, err, early, gp);
 }
 
 // Eighths of the last stage's outputs that hold samples below out_bits: samples m2 < ceil(out_bits / 2N1)
@@ -554,12 +567,10 @@ int launch_finish(const BlockGeom& g, const uint32_t* planes, const uint32_t* ke
     const uint32_t cols = std::min<uint32_t>(wpr, (m2max + 31u) / 32u);
     if (n1 >= 256u) {
         dim3 grid(n1 / 256u, (cols + 7u) / 8u, gp.count);
-        k_finish_tiled<<<grid, 256, 0, s>>>(planes, g, key_rest, flags, out, nwords, gp);
-        return (int)cudaGetLastError();
+        return (int)launch_pdl(k_finish_tiled, grid, 256, 0, s, planes, g, key_rest, flags, out, nwords, gp);
     }
     dim3 grid((n1 / 32u + 3u) / 4u, (cols + 7u) / 8u, gp.count);
-    k_finish<<<grid, 1024, 0, s>>>(planes, g, key_rest, flags, out, nwords, gp);
-    return (int)cudaGetLastError();
+    return (int)launch_pdl(k_finish, grid, 1024, 0, s, planes, g, key_rest, flags, out, nwords, gp);
 }
 
 }  // namespace pa
