@@ -22,8 +22,10 @@
 // block is 32 MB and stays in L2.
 #include "pa_gf2.cuh"
 #include "pa_kernels.cuh"
+#include "pa_launch.cuh"
 
 #include <algorithm>
+#include <utility>
 
 namespace pa {
 
@@ -35,6 +37,10 @@ enum Op { kF, kT, kIT };  // transform, its transpose, the inverse of its transp
 template <Op OP>
 struct OpTag {
     static constexpr Op value = OP;
+};
+template <int N>
+struct IntTag {
+    static constexpr int value = N;
 };
 
 // ============================================================================ segments <-> bit planes
@@ -83,18 +89,19 @@ __global__ void __launch_bounds__(128) k_exact_planes(const uint32_t* __restrict
                                                       uint32_t* __restrict__ V) {
     const uint32_t s = blockIdx.x * 128u + threadIdx.x;
     if (s >= pw) return;
+    pdl_wait();
     const uint32_t H = g.h / 32u, nw = g.n / 32u;
     const uint64_t tbits = (uint64_t)g.h + g.out_bits;
     auto word = [&](uint64_t q) -> uint32_t {
         if (SEED) {
             if (32ull * q >= tbits) return 0u;
             const uint32_t i = q < H ? (uint32_t)q + nw - H : (uint32_t)q - H;  // (32 q - h) mod n, in words
-            const uint32_t v = __brev(__ldg(src + i));
+            const uint32_t v = __brev(load(src + i));
             const uint64_t left = tbits - 32ull * q;
             return left >= 32u ? v : v & ((1u << left) - 1u);
         }
         if (q > H) return 0u;
-        return (__ldg(src + (H - q)) >> 31) | (q < H ? __ldg(src + (H - q - 1u)) << 1 : 0u);
+        return (load(src + (H - q)) >> 31) | (q < H ? load(src + (H - q - 1u)) << 1 : 0u);
     };
     uint32_t w[17], a[16];
 #pragma unroll
@@ -119,9 +126,10 @@ __global__ void __launch_bounds__(128) k_exact_words(const uint32_t* __restrict_
                                                      uint32_t* __restrict__ out, uint32_t nwords) {
     const uint32_t s = blockIdx.x * 128u + threadIdx.x;
     if (s >= pw || 16u * s >= nwords) return;
+    pdl_wait();
     uint32_t a[16];
 #pragma unroll
-    for (int p = 0; p < 16; ++p) a[p] = gather2(__ldg(V + (size_t)p * pw + s));
+    for (int p = 0; p < 16; ++p) a[p] = gather2(load(V + (size_t)p * pw + s));
     transpose16(a);
 #pragma unroll
     for (int k = 0; k < 16; ++k) {
@@ -131,7 +139,7 @@ __global__ void __launch_bounds__(128) k_exact_words(const uint32_t* __restrict_
         const uint32_t left = g.out_bits - 32u * q;
         if (left < 32u) w &= (1u << left) - 1u;
         w = __brev(w);
-        if ((flags & 1u) && 32ull * q < g.v) w ^= __ldg(key_rest + q);
+        if ((flags & 1u) && 32ull * q < g.v) w ^= load(key_rest + q);
         out[q] = __byte_perm(w, 0, 0x0123);
     }
 }
@@ -330,6 +338,7 @@ __global__ void __launch_bounds__(kBcThreads) k_exact_bc16(uint32_t* __restrict_
         r[4] = b.x; r[5] = b.y; r[6] = b.z; r[7] = b.w;
     };
     uint32_t* xp = x;
+    pdl_wait();
     unpack(g4);
     if (OP == kT) all_rounds<0, 8, OP>(r);
     pack(s4);
@@ -352,6 +361,7 @@ __global__ void __launch_bounds__(256) k_exact_taylor(const uint32_t* __restrict
                                                       uint32_t pw, int r, int e) {
     const uint32_t w = blockIdx.x * 256u + threadIdx.x;
     if (w >= pw) return;
+    pdl_wait();
     in += (size_t)blockIdx.y * pw;
     out += (size_t)blockIdx.y * pw;
     const uint32_t RW = 1u << (r - 5), o = w & (2u * RW - 1u);
@@ -362,30 +372,30 @@ __global__ void __launch_bounds__(256) k_exact_taylor(const uint32_t* __restrict
     uint32_t v;
     if (OP == kF) {
         auto nh = [&](uint32_t k) {  // hi after the wrap
-            uint32_t x = __ldg(hi + k);
+            uint32_t x = load(hi + k);
             if (DW) {
-                if (k < DW) x ^= __ldg(hi + (RW - DW + k));
+                if (k < DW) x ^= load(hi + (RW - DW + k));
             } else if (k == 0) {
-                x ^= __ldg(hi + (RW - 1u)) >> (32 - S);
+                x ^= load(hi + (RW - 1u)) >> (32 - S);
             }
             return x;
         };
         if (o >= RW) {
             v = nh(o - RW);
         } else {
-            v = __ldg(lo + o);
+            v = load(lo + o);
             if (DW) v ^= o >= DW ? nh(o - DW) : 0u;
             else v ^= (nh(o) << S) | (o ? nh(o - 1u) >> (32 - S) : 0u);
         }
     } else if (o < RW) {
-        v = __ldg(lo + o);
+        v = load(lo + o);
     } else {
         const uint32_t k = o - RW;
         auto down = [&](uint32_t j) -> uint32_t {  // lo >> d
-            if (DW) return j + DW < RW ? __ldg(lo + j + DW) : 0u;
-            return (__ldg(lo + j) >> S) | (j + 1u < RW ? __ldg(lo + j + 1u) << (32 - S) : 0u);
+            if (DW) return j + DW < RW ? load(lo + j + DW) : 0u;
+            return (load(lo + j) >> S) | (j + 1u < RW ? load(lo + j + 1u) << (32 - S) : 0u);
         };
-        auto h1 = [&](uint32_t j) { return OP == kT ? __ldg(hi + j) ^ down(j) : __ldg(hi + j); };
+        auto h1 = [&](uint32_t j) { return OP == kT ? load(hi + j) ^ down(j) : load(hi + j); };
         v = h1(k);
         if (DW) {
             if (k >= RW - DW) v ^= h1(k - (RW - DW));
@@ -405,6 +415,7 @@ __global__ void __launch_bounds__(256) k_exact_bc_rows(uint32_t* __restrict__ V,
     extern __shared__ uint32_t xr[];  // [row][kBcCols]
     const uint32_t rows = pw / 2048u, c = threadIdx.x % kBcCols, r0 = threadIdx.x / kBcCols, step = 256u / kBcCols;
     uint32_t* base = V + (size_t)blockIdx.y * pw + blockIdx.x * kBcCols + c;
+    pdl_wait();
     for (uint32_t i = r0; i < rows; i += step) xr[i * kBcCols + c] = base[(size_t)i * 2048u];
     __syncthreads();
     for (int k = 0; k < rs.count; ++k) {
@@ -443,6 +454,156 @@ __global__ void __launch_bounds__(256) k_exact_bc_rows(uint32_t* __restrict__ V,
     for (uint32_t i = r0; i < rows; i += step) base[(size_t)i * 2048u] = xr[i * kBcCols + c];
 }
 
+// The rounds above bit 16 of up to 2^23 coefficients in one pass: R = 2^up rows of 2048 words, a tile of columns in
+// shared memory.  The Taylor rounds (r, r - 16) shift a row by less than R bits in all, so that a tile needs H words
+// of halo.  Leaving out the wrap, the rows grow by an overflow O_c of R - 1 bits past x^65536; reducing that once,
+//   row c += x O_c + O_(c-1)
+// is the same as wrapping in every round, and only the first H words of a row see it: the CTA of the first columns
+// forms the overflows for itself from the last H words (kF).  Transposed, the halo is on the right, and the overflows
+// O_c[k] = g_c[k + 1] + g_(c+1)[k] are what the last columns continue with (kT); undoing that (kIT) first undoes the
+// rounds on the first 2 H + 1 words, which need no overflow, then runs the overflows forward and continues with those.
+// The rounds among rows (the polynomial in x^65536 + x) follow or precede where `rs` has some.
+// Out of place: tiles read each other's columns.  In place of one launch per Taylor round and one for the rows (52 us
+// each way at 2^25 bits), and with the chain launched dependently, a 2^25-bit block takes 156 instead of 243 us.
+constexpr int kUpThreads = 256;
+constexpr int kMaxUp = 7;
+constexpr int kUpRow = 64;   // words of a row of the tile, halo included
+constexpr int kUpEdge = 16;  // words of a row of the edge tile
+template <Op OP>
+__global__ void __launch_bounds__(kUpThreads) k_exact_upper(const uint32_t* __restrict__ in,
+                                                            uint32_t* __restrict__ out, int up, Rounds rs) {
+    extern __shared__ uint32_t xu[];
+    pdl_wait();
+    const int R = 1 << up, H = (R + 31) / 32, W = kUpRow - H, t = threadIdx.x;
+    const int w0 = (int)blockIdx.x * W, cols = min(W, 2048 - w0);  // the last tile has at least H columns
+    // blockIdx.y: a run of 2^(16 + up) coefficients of some plane
+    in += (size_t)blockIdx.y * (2048u << up);
+    out += (size_t)blockIdx.y * (2048u << up);
+    const bool edge = OP == kF ? w0 == 0 : w0 + cols == 2048;
+    // tile: kF H words of halo, then the columns; otherwise the columns, then the halo.
+    // edge tile: kF columns 2048 - H .. 2047 and H words past the end; otherwise columns 0 .. 2 H.
+    uint32_t* xa = xu;
+    uint32_t* xe = xu + R * kUpRow;
+    for (int i = t; i < R * kUpRow; i += kUpThreads) {
+        const int col = w0 + (i & (kUpRow - 1)) - (OP == kF ? H : 0);
+        xa[i] = col >= 0 && col < 2048 ? load(in + (size_t)(i / kUpRow) * 2048u + col) : 0u;
+    }
+    if (edge)
+        for (int i = t; i < R * kUpEdge; i += kUpThreads) {
+            const int col = (i & (kUpEdge - 1)) + (OP == kF ? 2048 - H : 0);
+            xe[i] = col < 2048 ? load(in + (size_t)(i / kUpEdge) * 2048u + col) : 0u;
+        }
+    __syncthreads();
+    // Taylor rounds on words [first, last) of rows of S words: kF lo ^= hi << d, d = R/2 .. 1; otherwise
+    // hi ^= lo >> d (`rising`: d from 1 up, the transpose; else from R/2 down, its inverse).  Bits from outside the
+    // words count as zero.
+    auto taylor = [&](uint32_t* x, auto stride, int first, int last, bool rising) {
+        constexpr int S = decltype(stride)::value;
+        for (int k = 0; k < up; ++k) {
+            const int q = rising ? k : up - 1 - k;
+            const int dw = q >= 5 ? 1 << (q - 5) : 0, bs = q >= 5 ? 0 : 1 << q;
+            for (int i = t; i < (R / 2) * S; i += kUpThreads) {
+                const int p = i / S, w = i & (S - 1);
+                if (w < first || w >= last) continue;
+                const int c = ((p >> q) << (q + 1)) | (p & ((1 << q) - 1));
+                uint32_t *lo = x + c * S, *hi = lo + (S << q);
+                if (OP == kF) {
+                    if (bs) lo[w] ^= __funnelshift_l(w > first ? hi[w - 1] : 0u, hi[w], bs);
+                    else if (w - dw >= first) lo[w] ^= hi[w - dw];
+                } else {
+                    if (bs) hi[w] ^= __funnelshift_r(lo[w], w + 1 < last ? lo[w + 1] : 0u, bs);
+                    else if (w + dw < last) hi[w] ^= lo[w + dw];
+                }
+            }
+            __syncthreads();
+        }
+    };
+    // The rounds among rows, on whole rows of S words.
+    auto among_rows = [&](uint32_t* x, auto stride) {
+        constexpr int S = decltype(stride)::value;
+        for (int k = 0; k < rs.count; ++k) {
+            const int q = OP == kT ? rs.count - 1 - k : k;
+            const int lr = rs.r[q], le = rs.e[q], RW = 1 << lr, D = 1 << le;
+            auto wrap = [&] {
+                for (int i = t; i < (R >> (lr + 1)) * D * S; i += kUpThreads) {
+                    const int u = i / S, j = u & (D - 1);
+                    uint32_t* hi = x + (((u >> le) << (lr + 1)) + RW) * S + (i & (S - 1));
+                    if (OP == kF) hi[j * S] ^= hi[(RW - D + j) * S];
+                    else hi[(RW - D + j) * S] ^= hi[j * S];
+                }
+                __syncthreads();
+            };
+            auto shift = [&] {
+                for (int i = t; i < (R / 2) * S; i += kUpThreads) {
+                    const int u = i / S, j = u & (RW - 1);
+                    uint32_t* lo = x + ((u >> lr) << (lr + 1)) * S + (i & (S - 1));
+                    uint32_t* hi = lo + RW * S;
+                    if (OP == kF) {
+                        if (j >= D) lo[j * S] ^= hi[(j - D) * S];
+                    } else if (j + D < RW) {
+                        hi[j * S] ^= lo[(j + D) * S];
+                    }
+                }
+                __syncthreads();
+            };
+            if (OP == kT) {
+                shift();
+                wrap();
+            } else {
+                wrap();
+                shift();
+            }
+        }
+    };
+    // Transposed overflows, from the edge tile's first words into the words after the last column.
+    auto overflow = [&] {
+        for (int i = t; i < R * kUpEdge; i += kUpThreads) {
+            const int k = i & (kUpEdge - 1);
+            if (k >= H) continue;
+            const uint32_t next = i / kUpEdge + 1 < R ? xe[i + kUpEdge] : 0u;
+            xa[(i / kUpEdge) * kUpRow + cols + k] = __funnelshift_r(xe[i], xe[i + 1], 1) ^ next;
+        }
+        __syncthreads();
+    };
+    using Row = IntTag<kUpRow>;
+    using Edge = IntTag<kUpEdge>;
+    if (OP == kF) {
+        taylor(xa, Row(), 0, kUpRow, false);
+        if (edge) {
+            taylor(xe, Edge(), 0, 2 * H, false);
+            for (int i = t; i < R * kUpEdge; i += kUpThreads) {
+                const int k = i & (kUpEdge - 1);
+                if (k >= H) continue;
+                const uint32_t* o = xe + i + H;
+                uint32_t v = (*o << 1) | (k ? o[-1] >> 31 : 0u);
+                if (i >= kUpEdge) v ^= o[-kUpEdge];
+                xa[(i / kUpEdge) * kUpRow + H + k] ^= v;
+            }
+            __syncthreads();
+        }
+        among_rows(xa, Row());
+    } else if (OP == kT) {
+        among_rows(xa, Row());
+        if (edge) {
+            among_rows(xe, Edge());
+            overflow();
+        }
+        taylor(xa, Row(), 0, edge ? cols + H : kUpRow, true);
+    } else {
+        if (edge) {
+            taylor(xe, Edge(), 0, 2 * H + 1, false);  // valid in the first H + 1 words
+            overflow();
+            taylor(xa, Row(), cols, cols + H, true);  // the overflows alone, through the transposed rounds
+        }
+        taylor(xa, Row(), 0, edge ? cols + H : kUpRow, false);
+        among_rows(xa, Row());
+    }
+    for (int i = t; i < R * kUpRow; i += kUpThreads) {
+        const int w = (i & (kUpRow - 1)) - (OP == kF ? H : 0);
+        if (w >= 0 && w < cols) out[(size_t)(i / kUpRow) * 2048u + w0 + w] = xa[i];
+    }
+}
+
 // ============================================================================ planes <-> field elements
 // Elements: W[slice][32 words], word c = bit c of the slice's 32 elements.  A warp converts 32 slices and
 // moves its 4 KB of elements through shared memory, so that both sides are coalesced.
@@ -456,15 +617,16 @@ __global__ void __launch_bounds__(kConvThreads) k_exact_to_field(const uint32_t*
     const uint32_t s = blockIdx.x * kConvThreads + threadIdx.x;
     const int lane = threadIdx.x & 31;
     uint32_t o[32];
+    pdl_wait();
     if constexpr (SEED) {
         uint32_t in[32];
 #pragma unroll
-        for (int p = 0; p < 32; ++p) in[p] = __ldg(V + (size_t)p * pw + s);
+        for (int p = 0; p < 32; ++p) in[p] = load(V + (size_t)p * pw + s);
         gf2::apply<gf2::kMapTraceToField, 32, 32>(in, o);
     } else {
         uint32_t in[16];
 #pragma unroll
-        for (int p = 0; p < 16; ++p) in[p] = __ldg(V + (size_t)p * pw + s);
+        for (int p = 0; p < 16; ++p) in[p] = load(V + (size_t)p * pw + s);
         gf2::apply<gf2::kMapSegToField, 32, 16>(in, o);
     }
     uint4* row = reinterpret_cast<uint4*>(sm + threadIdx.x * kRow);
@@ -487,10 +649,11 @@ __global__ void __launch_bounds__(kConvThreads) k_exact_to_traces(const uint32_t
     const int lane = threadIdx.x & 31;
     const uint4* src = reinterpret_cast<const uint4*>(W) + (size_t)(s - lane) * 8u;
     uint32_t* wrow = sm + (threadIdx.x - lane) * kRow;
+    pdl_wait();
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
         const int f = 32 * k + lane;
-        *reinterpret_cast<uint4*>(wrow + (f >> 3) * kRow + 4 * (f & 7)) = __ldg(src + f);
+        *reinterpret_cast<uint4*>(wrow + (f >> 3) * kRow + 4 * (f & 7)) = load(src + f);
     }
     __syncwarp();
     uint32_t in[32], o[16];
@@ -611,6 +774,7 @@ __global__ void __launch_bounds__(512) k_exact_top(uint32_t* __restrict__ W, int
     const uint32_t rows = 1u << T, half = blockIdx.x & 1u, col = blockIdx.x >> 1;
     const uint32_t cols = 1u << (lo - 5);
     uint32_t* base = W + ((size_t)blockIdx.y * rows * cols + col) * 32u + 16u * half;
+    pdl_wait();
     for (uint32_t i = threadIdx.x; i < rows * 4u; i += blockDim.x)
         *reinterpret_cast<uint4*>(xt + (i >> 2) * kTopRow + 4u * (i & 3u)) =
             *reinterpret_cast<const uint4*>(base + (size_t)(i >> 2) * cols * 32u + 4u * (i & 3u));
@@ -653,7 +817,6 @@ __global__ void __launch_bounds__(1 << (LOWB - 5), LOWB >= 13 ? 2 : 1)
     __shared__ uint32_t tc[LOWB];                  // the part of the CTA's index bits, per level
     const int t = threadIdx.x;
     uint4* g4 = reinterpret_cast<uint4*>(W) + (size_t)blockIdx.x * (NS * 8);
-    for (int f = t; f < NS * 8; f += NT) *reinterpret_cast<uint4*>(xl + (f >> 3) * kRow + 4 * (f & 7)) = g4[f];
     tt.fill();
     for (int i = t; i < 6 * 32; i += NT) {
         const int lev = i >> 5, m = i & 31;
@@ -672,6 +835,8 @@ __global__ void __launch_bounds__(1 << (LOWB - 5), LOWB >= 13 ? 2 : 1)
             if ((blockIdx.x >> b) & 1u) v ^= c_cantor[LOWB + b - t];
         tc[t] = v;
     }
+    pdl_wait();
+    for (int f = t; f < NS * 8; f += NT) *reinterpret_cast<uint4*>(xl + (f >> 3) * kRow + 4 * (f & 7)) = g4[f];
     __syncthreads();
     // Level i between slices differing in slice bit q; transposed: after the block transposes.
     auto level = [&](auto op, int i, bool transposed) {
@@ -734,7 +899,7 @@ __global__ void __launch_bounds__(1 << (LOWB - 5), LOWB >= 13 ? 2 : 1)
             load_words<32>(px, a);
 #pragma unroll
             for (int k = 0; k < 8; ++k) {
-                const uint4 q = __ldg(sp + k);
+                const uint4 q = load(sp + k);
                 b[4 * k] = q.x;
                 b[4 * k + 1] = q.y;
                 b[4 * k + 2] = q.z;
@@ -783,37 +948,60 @@ Shape shape_of(const BlockGeom& g) {
     return s;
 }
 
+// The launches of one transform, in order on a stream; the first error ends them.
+struct Chain {
+    cudaStream_t s;
+    cudaError_t err = cudaSuccess;
+    template <class... P, class... A>
+    void run(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A&&... args) {
+        if (err == cudaSuccess) err = launch_pdl(kernel, grid, block, smem, s, std::forward<A>(args)...);
+    }
+};
+
 template <class K>
 void smem_limit(K kernel, size_t bytes) {
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
 // The basis conversion on `planes` planes in a (b: scratch of the same size); returns where the result is.
+// Up to 2^23 coefficients a plane: the rounds above bit 16 in one pass; longer planes' first Taylor rounds one by one
+// and the rounds among their rows in a pass of their own.
 template <Op OP>
-uint32_t* convert_basis(const Shape& sh, uint32_t* a, uint32_t* b, uint32_t planes, cudaStream_t s) {
-    const int up = sh.l - 16;
-    auto taylor = [&] {
-        for (int k = 0; k < up; ++k) {
-            const int r = OP == kT ? 16 + k : sh.l - 1 - k;
-            k_exact_taylor<OP><<<dim3((sh.pw + 255u) / 256u, planes), 256, 0, s>>>(a, b, sh.pw, r, r - 16);
+uint32_t* convert_basis(const Shape& sh, uint32_t* a, uint32_t* b, uint32_t planes, Chain& ch) {
+    const int up = sh.l - 16, low = std::min(up, kMaxUp);
+    Rounds rs{}, none{};
+    add_rounds(&rs, 0, up);
+    auto long_taylor = [&] {
+        for (int k = 0; k < up - low; ++k) {
+            const int r = OP == kT ? 16 + low + k : sh.l - 1 - k;
+            ch.run(k_exact_taylor<OP>, dim3((sh.pw + 255u) / 256u, planes), 256, 0, a, b, sh.pw, r, r - 16);
             std::swap(a, b);
         }
     };
+    auto upper = [&] {
+        if (!low) return;
+        const int R = 1 << low, W = kUpRow - (R + 31) / 32;
+        const size_t smem = (size_t)R * (kUpRow + kUpEdge) * sizeof(uint32_t);
+        smem_limit(k_exact_upper<OP>, smem);
+        ch.run(k_exact_upper<OP>, dim3((2048u + W - 1u) / W, planes << (up - low)), kUpThreads, smem, a, b, low,
+               up == low ? rs : none);
+        std::swap(a, b);
+    };
     auto rows = [&] {
-        Rounds rs{};
-        add_rounds(&rs, 0, up);
-        if (!rs.count) return;
+        if (up == low) return;
         const size_t smem = (size_t)(sh.pw / 2048u) * kBcCols * sizeof(uint32_t);
         smem_limit(k_exact_bc_rows<OP>, smem);
-        k_exact_bc_rows<OP><<<dim3(2048u / kBcCols, planes), 256, smem, s>>>(a, sh.pw, rs);
+        ch.run(k_exact_bc_rows<OP>, dim3(2048u / kBcCols, planes), 256, smem, a, sh.pw, rs);
     };
-    auto runs = [&] { k_exact_bc16<OP><<<dim3(sh.pw / 2048u, planes), kBcThreads, 0, s>>>(a, sh.pw); };
+    auto runs = [&] { ch.run(k_exact_bc16<OP>, dim3(sh.pw / 2048u, planes), kBcThreads, 0, a, sh.pw); };
     if (OP == kT) {
         runs();
         rows();
-        taylor();
+        upper();
+        long_taylor();
     } else {
-        taylor();
+        long_taylor();
+        upper();
         rows();
         runs();
     }
@@ -821,28 +1009,28 @@ uint32_t* convert_basis(const Shape& sh, uint32_t* a, uint32_t* b, uint32_t plan
 }
 
 template <Op OP>
-void top_levels(const Shape& sh, uint32_t* W, cudaStream_t s) {
+void top_levels(const Shape& sh, uint32_t* W, Chain& ch) {
     for (int k = 0; k < sh.passes; ++k) {
         const int p = OP == kT ? sh.passes - 1 - k : k, T = sh.T[p], lo = sh.lo[p];
         if (T == 0) continue;
         const size_t smem = ((size_t)kTopRow << T) * sizeof(uint32_t);
         smem_limit(k_exact_top<OP>, smem);
         const int nt = std::max(32, std::min(512, 1 << (T - 1)));
-        k_exact_top<OP><<<dim3(2u << (lo - 5), 1u << (sh.l - lo - T)), nt, smem, s>>>(W, sh.l, lo, T);
+        ch.run(k_exact_top<OP>, dim3(2u << (lo - 5), 1u << (sh.l - lo - T)), nt, smem, W, sh.l, lo, T);
     }
 }
 
 template <int LOWB, bool KEY>
-void low_levels_k(const Shape& sh, uint32_t* W, const uint32_t* spec, cudaStream_t s) {
+void low_levels_k(const Shape& sh, uint32_t* W, const uint32_t* spec, Chain& ch) {
     const size_t smem = ((size_t)kRow << (LOWB - 5)) * sizeof(uint32_t);
     smem_limit(k_exact_low<LOWB, KEY>, smem);
-    k_exact_low<LOWB, KEY><<<1u << (sh.l - LOWB), 1 << (LOWB - 5), smem, s>>>(W, spec, sh.l);
+    ch.run(k_exact_low<LOWB, KEY>, 1u << (sh.l - LOWB), 1 << (LOWB - 5), smem, W, spec, sh.l);
 }
 template <bool KEY>
-void low_levels(const Shape& sh, uint32_t* W, const uint32_t* spec, cudaStream_t s) {
-    if (sh.lowb == 11) low_levels_k<11, KEY>(sh, W, spec, s);
-    else if (sh.lowb == 12) low_levels_k<12, KEY>(sh, W, spec, s);
-    else low_levels_k<13, KEY>(sh, W, spec, s);
+void low_levels(const Shape& sh, uint32_t* W, const uint32_t* spec, Chain& ch) {
+    if (sh.lowb == 11) low_levels_k<11, KEY>(sh, W, spec, ch);
+    else if (sh.lowb == 12) low_levels_k<12, KEY>(sh, W, spec, ch);
+    else low_levels_k<13, KEY>(sh, W, spec, ch);
 }
 
 }  // namespace
@@ -850,8 +1038,8 @@ void low_levels(const Shape& sh, uint32_t* W, const uint32_t* spec, cudaStream_t
 int exact_kernel_count(const BlockGeom& g) {
     if (direct_geom(g)) return 1;
     const Shape sh = shape_of(g);
-    const int up = sh.l - 16;
-    return 5 + 2 * (up + (up > 1 ? 1 : 0) + 1 + sh.passes);
+    const int up = sh.l - 16, extra = up > kMaxUp ? up - kMaxUp + 1 : 0;
+    return 5 + 2 * (extra + (up ? 1 : 0) + 1 + sh.passes);
 }
 
 // Buffers: P = 2^l field elements are at most Np / 8 words, 32 planes as much.
@@ -859,13 +1047,14 @@ int launch_exact_seed(const BlockGeom& g, const uint32_t* seed, uint32_t* seed_h
     if (direct_geom(g))  // the block kernel reads the seed itself
         return (int)cudaMemcpyAsync(seed_hat, seed, (size_t)(g.n / 32u) * 4u, cudaMemcpyDeviceToDevice, s);
     const Shape sh = shape_of(g);
+    Chain ch{s};
     const size_t P = size_t(32) * sh.pw;
-    k_exact_planes<true><<<(sh.pw + 127u) / 128u, 128, 0, s>>>(seed, g, sh.pw, tmp);
-    const uint32_t* V = convert_basis<kIT>(sh, tmp, tmp + P, 32, s);
-    k_exact_to_field<true><<<sh.pw / kConvThreads, kConvThreads, 0, s>>>(V, sh.pw, seed_hat);
-    top_levels<kIT>(sh, seed_hat, s);
-    low_levels<false>(sh, seed_hat, nullptr, s);
-    return (int)cudaGetLastError();
+    ch.run(k_exact_planes<true>, (sh.pw + 127u) / 128u, 128, 0, seed, g, sh.pw, tmp);
+    const uint32_t* V = convert_basis<kIT>(sh, tmp, tmp + P, 32, ch);
+    ch.run(k_exact_to_field<true>, sh.pw / kConvThreads, kConvThreads, 0, V, sh.pw, seed_hat);
+    top_levels<kIT>(sh, seed_hat, ch);
+    low_levels<false>(sh, seed_hat, nullptr, ch);
+    return (int)ch.err;
 }
 
 int launch_exact_block(const BlockGeom& g, const uint32_t* key_start, const uint32_t* key_rest, uint32_t flags,
@@ -879,18 +1068,20 @@ int launch_exact_block(const BlockGeom& g, const uint32_t* key_start, const uint
         return launch_direct(g, seed_hat, key_start, key_rest, flags, out_words, s);
     }
     const Shape sh = shape_of(g);
+    Chain ch{s};
     const size_t half = size_t(16) * sh.pw;
-    k_exact_planes<false><<<(sh.pw + 127u) / 128u, 128, 0, s>>>(key_start, g, sh.pw, tmp);
-    const uint32_t* V = convert_basis<kF>(sh, tmp, tmp + half, 16, s);
-    k_exact_to_field<false><<<sh.pw / kConvThreads, kConvThreads, 0, s>>>(V, sh.pw, a);
-    top_levels<kF>(sh, a, s);
-    low_levels<true>(sh, a, seed_hat, s);
-    top_levels<kT>(sh, a, s);
-    k_exact_to_traces<<<sh.pw / kConvThreads, kConvThreads, 0, s>>>(a, sh.pw, tmp);
-    V = convert_basis<kT>(sh, tmp, tmp + half, 16, s);
+    ch.run(k_exact_planes<false>, (sh.pw + 127u) / 128u, 128, 0, key_start, g, sh.pw, tmp);
+    const uint32_t* V = convert_basis<kF>(sh, tmp, tmp + half, 16, ch);
+    ch.run(k_exact_to_field<false>, sh.pw / kConvThreads, kConvThreads, 0, V, sh.pw, a);
+    top_levels<kF>(sh, a, ch);
+    low_levels<true>(sh, a, seed_hat, ch);
+    top_levels<kT>(sh, a, ch);
+    ch.run(k_exact_to_traces, sh.pw / kConvThreads, kConvThreads, 0, a, sh.pw, tmp);
+    V = convert_basis<kT>(sh, tmp, tmp + half, 16, ch);
     const uint32_t nwords = (g.out_bits + 31u) / 32u;
-    k_exact_words<<<((nwords + 15u) / 16u + 127u) / 128u, 128, 0, s>>>(V, g, sh.pw, key_rest, flags, out_words, nwords);
-    return (int)cudaGetLastError();
+    ch.run(k_exact_words, ((nwords + 15u) / 16u + 127u) / 128u, 128, 0, V, g, sh.pw, key_rest, flags, out_words,
+           nwords);
+    return (int)ch.err;
 }
 
 }  // namespace pa

@@ -26,14 +26,14 @@ namespace pa {
 #define PA_FLAG_COMPRESS 2u
 
 __device__ __forceinline__ uint32_t bit_of(const uint32_t* __restrict__ w, uint64_t x) {
-    return (__ldg(w + (x >> 5)) >> (31u - (uint32_t)(x & 31u))) & 1u;
+    return (load(w + (x >> 5)) >> (31u - (uint32_t)(x & 31u))) & 1u;
 }
 
 // Bits (x, x+1) of the key_start sequence (zero past bit h).  x is even.
 __device__ __forceinline__ void key_pair(const uint32_t* __restrict__ ks, const BlockGeom& g, uint64_t x,
                                          uint32_t& b0, uint32_t& b1) {
     if (x + 1 <= g.h) {
-        uint32_t w = __ldg(ks + (x >> 5));
+        uint32_t w = load(ks + (x >> 5));
         uint32_t o = (uint32_t)(x & 31u);
         b0 = (w >> (31u - o)) & 1u;
         b1 = (w >> (30u - o)) & 1u;
@@ -47,7 +47,7 @@ __device__ __forceinline__ void key_pair(const uint32_t* __restrict__ ks, const 
 __device__ __forceinline__ void seed_pair(const uint32_t* __restrict__ sd, const BlockGeom& g, uint64_t x,
                                           uint32_t& b0, uint32_t& b1) {
     if ((1u << g.log_np) == g.n) {
-        uint32_t w = __ldg(sd + (x >> 5));
+        uint32_t w = load(sd + (x >> 5));
         uint32_t o = (uint32_t)(x & 31u);
         b0 = (w >> (31u - o)) & 1u;
         b1 = (w >> (30u - o)) & 1u;
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(NT) k_mono_key(const uint32_t* __restrict__ ke
     for (int k = threadIdx.x; k <= N / 2; k += NT) {
         if (k == 0) {
             float2 z = sm[0];
-            float pn = 2.0f * (z.x - z.y) * __ldg(&spec[0].x);
+            float pn = 2.0f * (z.x - z.y) * load(&spec[0].x);
             sm[0] = make_float2(pn, -pn);
             continue;
         }
@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(NT) k_mono_key(const uint32_t* __restrict__ ke
         float2 za = sm[pad16(k)], zb = sm[pad16(N - k)];
         float2 xa, xb, qa, qb;
         real_split(za, zb, w, xa, xb);
-        float2 pa_ = cmul(xa, __ldg(spec + k)), pb_ = cmul(xb, __ldg(spec + (N - k)));
+        float2 pa_ = cmul(xa, load(spec + k)), pb_ = cmul(xb, load(spec + (N - k)));
         real_merge(pa_, pb_, w, qa, qb);
         sm[pad16(k)] = qa;
         if (k != N - k) sm[pad16(N - k)] = qb;
@@ -222,7 +222,7 @@ __global__ void __launch_bounds__(NT) k_mono_key(const uint32_t* __restrict__ ke
         if (lane < 2) {
             uint32_t w = (uint32_t)(m - lane) / 16u + lane;  // two words per 32 samples
             if (32u * w < g.out_bits) {
-                uint32_t kr = (do_xor && 32u * w < g.v) ? __ldg(key_rest + w) : 0u;
+                uint32_t kr = (do_xor && 32u * w < g.v) ? load(key_rest + w) : 0u;
                 out_words[w] = out_word(lane ? be >> 16 : be, lane ? bo >> 16 : bo, kr);
             }
         }

@@ -11,10 +11,30 @@
 // batch of 64 uneven blocks: 6.15, 6.24, 5.94 ms).
 #pragma once
 #include <cuda_runtime.h>
+#include <stdint.h>
 
 namespace pa {
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Loads of the block's data in these kernels: in place of __ldg (or a plain load that the compiler may turn into one),
+// whose read-only data may be fetched before the wait.
+__device__ __forceinline__ uint32_t load(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.global.b32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float load(const float* p) { return __uint_as_float(load(reinterpret_cast<const uint32_t*>(p))); }
+__device__ __forceinline__ float2 load(const float2* p) {
+    float2 v;
+    asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ uint4 load(const uint4* p) {
+    uint4 v;
+    asm volatile("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
 
 template <class... P, class... A>
 inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A&&... args) {

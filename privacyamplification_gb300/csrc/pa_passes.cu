@@ -56,13 +56,13 @@ __global__ void __launch_bounds__(256) k_bit_rows(const uint32_t* __restrict__ s
     const uint64_t x0 = 2ull * n1 * m2 + 32ull * a;
     uint32_t v;
     if (!SEED) {
-        if (x0 + 31 <= g.h) v = __ldg(src + (x0 >> 5));
+        if (x0 + 31 <= g.h) v = load(src + (x0 >> 5));
         else if (x0 > g.h) v = 0u;
-        else v = __ldg(src + (x0 >> 5)) & ~(0xFFFFFFFFu >> (uint32_t)(g.h - x0 + 1));
+        else v = load(src + (x0 >> 5)) & ~(0xFFFFFFFFu >> (uint32_t)(g.h - x0 + 1));
     } else if ((1u << g.log_np) == g.n) {
-        v = __ldg(src + (x0 >> 5));
+        v = load(src + (x0 >> 5));
     } else {  // padded placement: whole words
-        v = __ldg(src + seed_word(g, x0));
+        v = load(src + seed_word(g, x0));
     }
     const uint32_t w = transpose16x2(v, lane);
     rows[(size_t)(16u * a + (uint32_t)(lane & 15)) * (n2 / 16u) + 2u * c + (uint32_t)(lane >> 4)] = w;
@@ -93,8 +93,8 @@ __global__ void __launch_bounds__(256) k_bit_rows_tiled(const uint32_t* __restri
         const int r = (t >> 4) + 16 * i, w = t & 15;
         const uint64_t word = (uint64_t)(m20 + (uint32_t)r) * win + a0 + (uint32_t)w;
         const uint64_t x0 = 32ull * word;  // first sample of the word
-        if (SEED) v[i] = __ldg(src + ((1u << g.log_np) == g.n ? word : seed_word(g, x0)));
-        else v[i] = x0 <= g.h ? __ldg(src + word) : 0u;
+        if (SEED) v[i] = load(src + ((1u << g.log_np) == g.n ? word : seed_word(g, x0)));
+        else v[i] = x0 <= g.h ? load(src + word) : 0u;
     }
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(1024) k_finish(const uint32_t* __restrict__ pl
     const uint32_t c = blockIdx.y * 8u + (uint32_t)(warp >> 2);
     if (a >= n1 / 32u || c >= wpr) return;
     const size_t off = (size_t)(32u * a + (uint32_t)lane) * wpr + c;
-    const uint32_t ve = __ldg(planes + off), vo = __ldg(planes + plane_words + off);
+    const uint32_t ve = load(planes + off), vo = load(planes + plane_words + off);
     const uint32_t lo = transpose16x2(msb_pairs(ve, vo), lane);
     const uint32_t hi = transpose16x2(msb_pairs(ve >> 16, vo >> 16), lane);
     const uint32_t L = (uint32_t)(lane & 15), h = (uint32_t)(lane >> 4);
@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(1024) k_finish(const uint32_t* __restrict__ pl
         const uint64_t ow = (m2 * n1 + 32ull * a + 16ull * h) / 16ull;
         if (ow >= nwords) continue;
         uint32_t w = k ? hi : lo;
-        if ((flags & kXor) && 32ull * ow < g.v) w ^= __ldg(key_rest + ow);
+        if ((flags & kXor) && 32ull * ow < g.v) w ^= load(key_rest + ow);
         out[ow] = __byte_perm(w, 0, 0x0123);
     }
 }
@@ -226,14 +226,14 @@ __global__ void __launch_bounds__(256) k_finish_tiled(const uint32_t* __restrict
         const int r = (t >> 3) + 32 * i, w = t & 7;
         const uint32_t c = c0 + (uint32_t)w;
         const size_t off = (size_t)(m10 + (uint32_t)r) * wpr + c;
-        pv[2 * i] = c < wpr ? __ldg(planes + off) : 0u;
-        pv[2 * i + 1] = c < wpr ? __ldg(planes + plane_words + off) : 0u;
+        pv[2 * i] = c < wpr ? load(planes + off) : 0u;
+        pv[2 * i + 1] = c < wpr ? load(planes + plane_words + off) : 0u;
     }
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
         const int ml = (t >> 4) + 16 * i, j = t & 15;
         const uint64_t ow = ((32ull * c0 + (uint64_t)ml) * n1 + m10) / 16ull + (uint64_t)j;
-        kr[i] = ((flags & kXor) && ow < nwords && 32ull * ow < g.v) ? __ldg(key_rest + ow) : 0u;
+        kr[i] = ((flags & kXor) && ow < nwords && 32ull * ow < g.v) ? load(key_rest + ow) : 0u;
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
