@@ -537,8 +537,11 @@ __device__ __forceinline__ void pass_b_tiles(const CUtensorMap* mapY, const floa
                     }
                 }
                 __syncthreads();
-                if (pp == 0) {
-                    for (int u = jj; u < L; u += LR) {
+                // Every thread takes bin pairs, not only pair 0's LR threads: with short columns those were a chain of
+                // 16 round trips to L2 for a handful of threads (12 us, more than an ordinary tile; 2^20 bits 45.2 -> 41
+                // us a block, 2^18 41 -> 37).  With columns of 2^12 pair 0 is every thread.
+                if (CPT > 2 || pp == 0) {
+                    for (int u = CPT > 2 ? t : jj; u < L; u += CPT > 2 ? NT : LR) {
                         int ca, ka, cb, kb;
                         uint32_t k;
                         if (u < L / 2) {  // column k2 = 0, rows u <-> L-u
@@ -803,9 +806,17 @@ __device__ __forceinline__ void pass_c_rows(const CUtensorMap* mapZ, const float
         } else {
             const float4* z4 = reinterpret_cast<const float4*>(Z);
             float4* s4 = reinterpret_cast<float4*>(srow);
-            for (int p = t; p < L / 2; p += NT) {
-                int tl = p / pairs_per_tile, cp = p % pairs_per_tile;
-                s4[p] = __ldcs(z4 + ((size_t)tl * n1 + r) * pairs_per_tile + cp);
+            const int ps = __ffs(pairs_per_tile) - 1;  // a power of two
+#pragma unroll 1
+            for (int i0 = 0; i0 < 16; i0 += 4) {       // L / 2 = 16 NT; four loads before the first store
+                float4 v[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int p = t + (i0 + i) * NT;
+                    v[i] = __ldcs(z4 + (((size_t)(p >> ps) * n1 + r) << ps) + (p & (pairs_per_tile - 1)));
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) s4[t + (i0 + i) * NT] = v[i];
             }
         }
     };
