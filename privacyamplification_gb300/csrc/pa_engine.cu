@@ -82,13 +82,7 @@ int ensure_maps(pa_engine* e, const BlockGeom& g) {
 
 pa::Scratch scratch(pa_engine* e) { return {e->d_work, e->d_work2, e->d_planes, e->d_err, &e->maps}; }
 
-int build_exact_seed(pa_engine* e, const BlockGeom& g, cudaStream_t s) {
-    int rc = pa::launch_exact_seed(g, e->d_seed, e->d_exact_seed, reinterpret_cast<uint32_t*>(e->d_work2), s);
-    if (rc) return cuda_fail(e, (cudaError_t)rc);
-    e->exact_geom = g;
-    e->exact_valid = true;
-    return PA_OK;
-}
+int build_exact_seed(pa_engine* e, const BlockGeom& g, cudaStream_t s);
 
 int build_spectrum(pa_engine* e, const BlockGeom& g, cudaStream_t s) {
     if (g.exact_only) return build_exact_seed(e, g, s);
@@ -112,6 +106,7 @@ int seed_common(pa_engine* e, uint32_t n, int32_t reuse, cudaStream_t s) {
     e->seed_left = reuse < 0 ? -1 : std::max<int64_t>(reuse, 1);
     e->spec_valid = false;
     e->exact_valid = false;
+    e->chunk_valid = false;
     if (is_pow2(n)) {  // placement does not depend on v: build the spectrum now
         BlockGeom g;
         int rc = make_geom(n, n / 2u, PA_FLAG_COMPRESS, e->split, &g);
@@ -140,51 +135,56 @@ int fused_block(pa_engine* e, const uint32_t* d_ks, const uint32_t* d_kr, const 
     return rc ? cuda_fail(e, (cudaError_t)rc) : PA_OK;
 }
 
-// n > 2^27: the block as 2^27-bit FP32 chunk blocks (pa_chunk.cu).  The exact seed transform's buffer
-// is the chunks' staging area and the chunk spectra go through d_spec, so both caches are invalidated.
-// Block popcounts are not formed on this path (take_stats reports 0).
-//
-// Two lanes take the diagonals in turn.  The second lane's three-pass buffers are the upper halves of
-// d_work / d_work2 (each holds Np / 2 >= 2^27 complex here, a chunk block needs 2^26); its staging, bit
-// planes and seed spectrum follow the first lane's staging in d_exact_seed (Np >= 2^28 words, the four
-// need under 2^28); its stream is `side`, free here because the block waited for key_rest's copy.
+// Scratch of the exact path: 2 P words beside the P of d_work.  Engines for n > 2^27 take the last two of the chunk
+// buffers, which hold key spectra or row products only.
+uint32_t* exact_scratch(pa_engine* e) {
+    if (!e->d_chunk) return reinterpret_cast<uint32_t*>(e->d_work2);
+    return reinterpret_cast<uint32_t*>(e->d_chunk + (pa::chunk_units(e->cap_log_np) - 2) * (size_t(1) << 26));
+}
+
+int build_exact_seed(pa_engine* e, const BlockGeom& g, cudaStream_t s) {
+    int rc = pa::launch_exact_seed(g, e->d_seed, e->d_exact_seed, exact_scratch(e), s);
+    if (rc) return cuda_fail(e, (cudaError_t)rc);
+    e->exact_geom = g;
+    e->exact_valid = true;
+    return PA_OK;
+}
+
+// n > 2^27: the block in 2^27-bit FP32 transforms (pa_chunk.cu).  Block popcounts are not formed on this path
+// (take_stats reports 0).  Lane 0 has d_work / d_work2 and the block's stream, lane 1 the first two chunk buffers and
+// `side` (free here because the block waited for key_rest's copy).  A seed that is kept has its window spectra kept
+// too, as long as they all fit (up to three rows) and the next block has the same rows and columns.
 int chunked_block(pa_engine* e, const uint32_t* d_ks, const uint32_t* d_kr, const BlockGeom& g, uint32_t flags,
                   uint32_t* d_out, cudaStream_t s) {
     BlockGeom gc;
     const uint32_t side = 1u << pa::kChunkLog;
     int rc = make_geom(2u * side, side, 0u, e->split, &gc);
     if (rc) return rc;
-    const size_t np = size_t(1) << e->cap_log_np;
-    if (pa::chunk_staging_words(g) > np) return PA_ERR_TOO_LARGE;
     rc = ensure_maps(e, gc);
     if (rc) return rc;
-    e->exact_valid = false;
-    e->spec_valid = false;
-    auto align64 = [](size_t w) { return (w + 63u) & ~size_t(63); };
-    const size_t nc = size_t(1) << gc.log_n;                               // complex per three-pass buffer
-    const size_t w0 = align64(pa::chunk_staging_words(g));                 // first lane's staging
-    const size_t w1 = align64(pa::chunk_lane_words(g));                    // second lane's staging
-    const size_t wp = align64((size_t(1) << gc.log_np) / 32u + 64u);       // bit planes: Np / 8 + 256 bytes
-    pa::ChunkLane lane{};
-    const pa::ChunkLane* lp = nullptr;
-    if (2 * nc <= np / 2 && w0 + w1 + wp + 2 * nc <= np) {
-        if (e->lane_maps_key != pa_host::maps_key(gc)) {
-            rc = pa::make_pass_maps(gc, e->d_work + nc, e->d_work2 + nc, &e->lane_maps);
-            if (rc) return cuda_fail(e, (cudaError_t)rc);
-            e->lane_maps_key = pa_host::maps_key(gc);
-        }
-        uint32_t* base = e->d_exact_seed;
-        lane.staging = base + w0;
-        lane.sc = {e->d_work + nc, e->d_work2 + nc, base + w0 + w1, e->d_err, &e->lane_maps};
-        lane.spec = reinterpret_cast<float2*>(base + w0 + w1 + wp);
-        lane.s = e->side;
-        lane.fork = e->lane_fork;
-        lane.join = e->lane_join;
-        lp = &lane;
+    const size_t nc = size_t(1) << gc.log_n;  // complex values per buffer
+    if (e->lane_maps_key != pa_host::maps_key(gc)) {
+        rc = pa::make_pass_maps(gc, e->d_chunk, e->d_chunk + nc, &e->lane_maps);
+        if (rc) return cuda_fail(e, (cudaError_t)rc);
+        e->lane_maps_key = pa_host::maps_key(gc);
     }
-    rc = pa::launch_chunked_block(g, gc, e->d_seed, d_ks, d_kr, flags, d_out, e->d_exact_seed, e->d_spec, scratch(e),
-                                  e->d_cnt, e->d_resid, e->num_sms, s, lp);
+    const size_t wwords = 2 * (side / 32u);
+    uint32_t* st = e->d_stage;
+    pa::ChunkBuffers cb{};
+    cb.lane[0] = {scratch(e), st, s};
+    cb.lane[1] = {{e->d_chunk, e->d_chunk + nc, st + 2 * wwords, e->d_err, &e->lane_maps}, st + wwords, e->side};
+    cb.fork = e->lane_fork;
+    cb.join = e->lane_join;
+    cb.units = e->d_chunk + 2 * nc;
+    cb.cnt = reinterpret_cast<unsigned long long*>(st + 3 * wwords + 64);
+    const pa::ChunkPlan p = pa::chunk_plan(g);
+    const bool ready = e->chunk_valid && e->chunk_rows == p.rows && e->chunk_cols == p.cols;
+    e->chunk_valid = false;
+    rc = pa::launch_chunked_block(g, gc, e->d_seed, d_ks, d_kr, flags, d_out, cb, ready, e->d_resid, e->num_sms, s);
     if (rc) return cuda_fail(e, (cudaError_t)rc);
+    e->chunk_valid = p.slots == p.diagonals;
+    e->chunk_rows = p.rows;
+    e->chunk_cols = p.cols;
     return PA_OK;
 }
 
@@ -196,7 +196,7 @@ int exact_block(pa_engine* e, const uint32_t* d_ks, const uint32_t* d_kr, const 
         if (rc) return rc;
     }
     int rc = pa::launch_exact_block(g, d_ks, d_kr, flags, e->d_exact_seed, reinterpret_cast<uint32_t*>(e->d_work),
-                                    reinterpret_cast<uint32_t*>(e->d_work2), d_out, s);
+                                    exact_scratch(e), d_out, s);
     if (rc) return cuda_fail(e, (cudaError_t)rc);
     // the exact path leaves no residual: report 0 and the reference popcounts are not needed
     PA_CUDA(e, cudaMemsetAsync(e->d_resid, 0, sizeof(unsigned int), s));
@@ -353,11 +353,16 @@ int pa_create(const pa_config* cfg, pa_engine** out) {
     if ((err = cudaMalloc(&e->d_key_rest, words * 4)) != cudaSuccess) return fail(err);
     if ((err = cudaMalloc(&e->d_seed, words * 4)) != cudaSuccess) return fail(err);
     if ((err = cudaMalloc(&e->d_out, words * 4)) != cudaSuccess) return fail(err);
-    if ((err = cudaMalloc(&e->d_work, (np / 2) * sizeof(float2))) != cudaSuccess) return fail(err);
-    const size_t np_fp32 = std::min<size_t>(np, size_t(1) << 27);  // the FP32 path stops at n = 2^27
+    const size_t np_fp32 = std::min<size_t>(np, size_t(1) << 27);  // one pass of the FP32 path stops at n = 2^27
+    if ((err = cudaMalloc(&e->d_work, (np_fp32 / 2) * sizeof(float2))) != cudaSuccess) return fail(err);
     if ((err = cudaMalloc(&e->d_spec, (np_fp32 / 2) * sizeof(float2))) != cudaSuccess) return fail(err);
-    if ((err = cudaMalloc(&e->d_exact_seed, np * sizeof(uint32_t))) != cudaSuccess) return fail(err);
-    if ((err = cudaMalloc(&e->d_work2, (np / 2) * sizeof(float2))) != cudaSuccess) return fail(err);
+    if ((err = cudaMalloc(&e->d_work2, (np_fp32 / 2) * sizeof(float2))) != cudaSuccess) return fail(err);
+    if ((err = cudaMalloc(&e->d_exact_seed, np / 4 * sizeof(uint32_t))) != cudaSuccess) return fail(err);
+    if (np > np_fp32) {
+        const size_t units = pa::chunk_units(e->cap_log_np);
+        if ((err = cudaMalloc(&e->d_chunk, units * (np_fp32 / 2) * sizeof(float2))) != cudaSuccess) return fail(err);
+        if ((err = cudaMalloc(&e->d_stage, pa::chunk_staging_words() * sizeof(uint32_t))) != cudaSuccess) return fail(err);
+    }
     if ((err = cudaMalloc(&e->d_words, sizeof(pa_engine::Words))) != cudaSuccess) return fail(err);
     cudaMemset(e->d_words, 0, sizeof(pa_engine::Words));
     e->d_cnt = e->d_words->cnt;
@@ -388,6 +393,8 @@ void pa_destroy(pa_engine* e) {
     cudaFree(e->d_spec);
     cudaFree(e->d_exact_seed);
     cudaFree(e->d_work2);
+    cudaFree(e->d_chunk);
+    cudaFree(e->d_stage);
     cudaFree(e->d_words);
     cudaFreeHost(e->h_words);
     cudaFree(e->d_planes);

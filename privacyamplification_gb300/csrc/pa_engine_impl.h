@@ -35,15 +35,20 @@ struct pa_engine {
     float2* d_work2 = nullptr;  // pass B output (tile-major)
     float2* d_spec = nullptr;
     int* d_err = nullptr;       // device error word of the bounded TMA waits (in d_words)
-    uint32_t* d_exact_seed = nullptr;  // the seed's transform (exact path), Np words
+    uint32_t* d_exact_seed = nullptr;  // the seed's transform (exact path), up to Np / 4 words
     bool exact_valid = false;          // d_exact_seed matches the current seed for exact_geom
     bool last_exact = false;           // the last block ran on the exact path
     bool last_chunked = false;         // the last block ran as FP32 chunk blocks (n > 2^27)
     pa::BlockGeom exact_geom{};
     pa::PassMaps maps{};        // tensor maps for the geometry maps_key
     int maps_key = -1;
-    // second lane of the chunk blocks (n > 2^27): tensor maps over the upper halves of d_work / d_work2,
-    // its stream is `side`, and the events it forks and joins on
+    // blocks of n > 2^27 (pa_chunk.cu): chunk_units() buffers of 2^26 complex (lane 1's two, seed and key spectra, a row
+    // product), the lanes' seed windows, lane 1's bit planes and the popcounts; the window spectra in place, if any
+    float2* d_chunk = nullptr;
+    uint32_t* d_stage = nullptr;
+    bool chunk_valid = false;
+    uint32_t chunk_rows = 0, chunk_cols = 0;
+    // lane 1: tensor maps over its buffers, its stream is `side`, and the events the lanes fork and join on
     pa::PassMaps lane_maps{};
     int lane_maps_key = -1;
     cudaEvent_t lane_fork = nullptr, lane_join = nullptr;

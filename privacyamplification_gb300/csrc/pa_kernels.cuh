@@ -163,7 +163,8 @@ int launch_finish(const BlockGeom& g, const uint32_t* planes, const uint32_t* ke
                   uint32_t* out, cudaStream_t s, const Group& gp = kOneBlock);
 
 // Exact path (pa_exact.cu): the product over GF(2) by an additive FFT, or for short blocks (direct_geom,
-// pa_direct.cu) word by word.  seed_hat, a, tmp: Np words each; seed_hat holds for the same n, h and out_bits.
+// pa_direct.cu) word by word.  With P <= max(2^16, 3 Np / 16) words:
+// seed_hat and a hold P, tmp 2 P (and n / 32 words each); seed_hat holds for the same n, h and out_bits.
 int launch_exact_seed(const BlockGeom& g, const uint32_t* seed, uint32_t* seed_hat, uint32_t* tmp, cudaStream_t s);
 int launch_exact_block(const BlockGeom& g, const uint32_t* key_start, const uint32_t* key_rest, uint32_t flags,
                        const uint32_t* seed_hat, uint32_t* a, uint32_t* tmp, uint32_t* out_words, cudaStream_t s);
@@ -173,31 +174,33 @@ int launch_direct(const BlockGeom& g, const uint32_t* seed, const uint32_t* key_
                   uint32_t flags, uint32_t* out_words, cudaStream_t s);
 int exact_kernel_count(const BlockGeom& g);
 
-// Blocks beyond the single-pass FP32 size (pa_chunk.cu): side x side chunk blocks (n' = 2 side) on the
-// FP32 path.  gc: geometry of a chunk block (n' = 2 side, v' = side, no flags).  staging:
-// chunk_staging_words(g) words; spec / sc / cnt: the FP32 path's buffers for gc.  resid_bits receives
-// the largest chunk residual.
+// Blocks beyond the single-pass FP32 size (pa_chunk.cu): side x side chunks as transforms of n' = 2 side bits on
+// the FP32 path, summed per row as spectra.  gc: geometry of a chunk transform (n' = 2 side, v' = side, no flags).
+// resid_bits receives the largest residual.
 constexpr int kChunkLog = 26;
 struct ChunkPlan {
-    uint32_t side, rows, cols, chunks, diagonals;
-    uint32_t absorb;  // 1: key bit h = cols * side (alone past the last full column) rides in that column
+    uint32_t side, rows, cols, diagonals;
+    uint32_t slots;  // seed spectra held at a time
 };
 ChunkPlan chunk_plan(const BlockGeom& g);
-size_t chunk_staging_words(const BlockGeom& g);
 int chunk_kernel_count(const BlockGeom& g, const BlockGeom& gc);
-// A second lane for the chunk blocks: its own staging (chunk_lane_words(g) words), seed spectrum and
-// three-pass buffers, and a stream; the diagonals alternate between the lanes, so one lane's short kernels
-// and kernel tails overlap the other's work.  fork / join: events the lanes synchronise with.
+// A lane of the chunk transforms: row-pass and column-pass buffers, bit planes, a seed window, a stream.
 struct ChunkLane {
-    uint32_t* staging;
-    float2* spec;
     Scratch sc;
+    uint32_t* window;
     cudaStream_t s;
-    cudaEvent_t fork, join;
 };
-size_t chunk_lane_words(const BlockGeom& g);
+struct ChunkBuffers {
+    ChunkLane lane[2];        // lane 0 runs on the block's stream
+    cudaEvent_t fork, join;   // the lanes synchronise with
+    float2* units;            // seed spectra, key spectra, one row product: N complex each
+    unsigned long long* cnt;  // popcounts: 128 words
+};
+// Buffers of N = 2^26 complex for blocks of cyclic length up to 2^log_np: lane 1's two and `units`.
+size_t chunk_units(int log_np);
+size_t chunk_staging_words();
+// seed_ready: the spectra of all the block's windows (at most `slots`) are already in place.
 int launch_chunked_block(const BlockGeom& g, const BlockGeom& gc, const uint32_t* seed, const uint32_t* key_start,
-                         const uint32_t* key_rest, uint32_t flags, uint32_t* out_words, uint32_t* staging,
-                         float2* spec, const Scratch& sc, unsigned long long* cnt, unsigned int* resid_bits,
-                         int num_sms, cudaStream_t s, const ChunkLane* lane2 = nullptr);
+                         const uint32_t* key_rest, uint32_t flags, uint32_t* out_words, const ChunkBuffers& cb,
+                         bool seed_ready, unsigned int* resid_bits, int num_sms, cudaStream_t s);
 }  // namespace pa
