@@ -13,7 +13,7 @@
 // larger than one chunk's, so the largest residual grows with the root of the columns: 0.021 -> 0.053 at n = 2^29,
 // 0.074 at the most (n = 2^30, sixteen columns), against the limit of 0.25.
 //
-// Forward transforms are the row pass and the seed form of the column pass (spectra scaled by 1 / (4 Np), a power
+// Forward transforms are the row pass and the seed form of the column pass (spectra scaled by 1 / (16 Np), a power
 // of two, taken back in the sum); the sum reads every spectrum once for three rows (15 x 512 MB at n = 2^29,
 // bound by HBM); the inverse column pass is the second half of pass B.  Two lanes (streams with their own row-pass
 // and column-pass buffers) take the transforms in turn, so that one's short kernels and tails overlap the other's.
@@ -285,7 +285,7 @@ int launch_chunked_block(const BlockGeom& g, const BlockGeom& gc, const uint32_t
     if (!seed_ready)
         for (int d = -(cols - 1); d <= std::min((int)p.rows, kRowGroup) - 1 && !rc; ++d) seed_window(d);
     join();
-    const float scale = (float)(4ull << gc.log_np);
+    const float scale = (float)(16ull << gc.log_np);
     for (int a0 = 0; a0 < (int)p.rows && !rc; a0 += kRowGroup) {
         const int R = std::min(kRowGroup, (int)p.rows - a0);
         if (a0) {  // the group's new windows take the slots of the oldest

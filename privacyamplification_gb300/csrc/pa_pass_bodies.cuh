@@ -97,6 +97,11 @@ __device__ __forceinline__ uint32_t transpose16x2(uint32_t w, int lane) {
     return w;
 }
 
+// A sample bit b (the top bit of w) as 1 - 2 b: the constant 1 is in the DC bin alone, which is dropped, and the
+// factor -2 of key and seed is taken out with the seed spectrum's scale.  One LOP3 (0 and 1 by shift, mask and
+// conversion were three on the same pipe), and rows without the mean of 0/1 data.
+__device__ __forceinline__ float sign_unit(uint32_t w) { return __uint_as_float((w & 0x80000000u) | 0x3F800000u); }
+
 // ============================================================================ pass A
 // Row m1: FFT over m2 of the 2N2 bits of the row, 4-step twiddle W_N^{m1 k2}, pair-order store.
 // Radices RA, RB (linear) then 16 (mirror, NS = L/16).  The CTA (L/32 threads) takes rows first,
@@ -167,12 +172,12 @@ __device__ __forceinline__ void pass_a_rows(const uint32_t* __restrict__ rows, c
 #pragma unroll
         for (int q = 0; q < E / P::RA; ++q) {
             const int j = t + q * NT;
+            const uint32_t even = 1u << (2 * (j & 15));  // brings sample 2 m2 to the top bit (L / RA is a multiple of 16)
 #pragma unroll
             for (int r = 0; r < P::RA; ++r) {
                 const int m2 = j + r * (L / P::RA);
                 const uint32_t w = bits[buf][m2 >> 4];
-                const int sh = 30 - 2 * (m2 & 15);
-                x[q * P::RA + r] = make_float2((float)((w >> (sh + 1)) & 1u), (float)((w >> sh) & 1u));
+                x[q * P::RA + r] = make_float2(sign_unit(w * even), sign_unit(w * (2u * even)));
             }
         }
         stage<P::RA, 1, -1, E>(x, nullptr);
@@ -327,7 +332,7 @@ __device__ __forceinline__ void pass_b_tiles(const CUtensorMap* mapY, const floa
     auto unit_block = [&](int u) { return GRP ? (uint32_t)(u >> tshift) : 0u; };
     const int t = threadIdx.x;
     const int pp = t / LR, jj = t % LR;
-    const float sc = 1.0f / (float)(4ull << g.log_np);  // seed spectrum scale 2X/(4Np)
+    const float sc = 1.0f / (float)(16ull << g.log_np);  // seed spectrum scale: X/(2Np) from 2 (-2 X), for a key at -2 X
     {
         float2 w[4];
         if (P::NSTAGE == 2) {
@@ -714,6 +719,16 @@ __device__ __forceinline__ void pass_b_tiles(const CUtensorMap* mapY, const floa
 }
 
 // ============================================================================ pass C
+// |v - 2 rint(v / 2)| - 1/2: positive where rint(v) is odd, and 1/2 minus its magnitude is v's distance to the nearest
+// integer.  FP32 adds and multiplies only (rint and the conversion to an integer run at an eighth of their rate):
+// v / 2 is rounded by adding 3 2^22, exact while |v| < 2^23; beyond, v is an integer, and a value whose half is not
+// rounded right has a remainder of 2, which the residual reports as 1.
+__device__ __forceinline__ float parity_half(float v) {
+    const float magic = 12582912.0f;
+    const float q = __fadd_rn(__fmaf_rn(v, 0.5f, magic), -magic);
+    return fabsf(__fmaf_rn(-2.0f, q, v)) - 0.5f;
+}
+
 // Row m1: inverse FFT over k2 (radices 16, RB, RA), + correction, round, parity bit planes.
 // Input: Z, tile-major from pass B.  Row m1 is the CPT/2 pairs of row m1 of every tile; 3D TMA boxes
 // (256 tiles x 1 row x CPT/2 pairs) gather it into shared memory in pair order (float4 p = pair p),
@@ -914,13 +929,12 @@ __device__ __forceinline__ void pass_c_rows(const CUtensorMap* mapZ, const float
             for (int r = 0; r < KR; ++r) {
                 const uint32_t m2 = (uint32_t)(j + NSL * r);
                 const float2 v = x[q * RL + r];
-                const float v0 = v.x + corr, v1 = v.y + corr;
-                const float r0 = rintf(v0), r1 = rintf(v1);
                 const bool ok0 = m2 < lim0, ok1 = m2 < lim1;
-                if (ok0) res = fmaxf(res, fabsf(v0 - r0));
-                if (ok1) res = fmaxf(res, fabsf(v1 - r1));
-                const uint32_t be = __ballot_sync(0xffffffffu, ok0 && ((int)r0 & 1));
-                const uint32_t bo = __ballot_sync(0xffffffffu, ok1 && ((int)r1 & 1));
+                const float p0 = parity_half(v.x + corr), p1 = parity_half(v.y + corr);
+                if (ok0) res = fmaxf(res, fabsf(fabsf(p0) - 0.5f));
+                if (ok1) res = fmaxf(res, fabsf(fabsf(p1) - 0.5f));
+                const uint32_t be = __ballot_sync(0xffffffffu, ok0 && p0 > 0.f);
+                const uint32_t bo = __ballot_sync(0xffffffffu, ok1 && p1 > 0.f);
                 if (lane == 0) {
                     pstage[pb][0][m2 >> 5] = be;
                     pstage[pb][1][m2 >> 5] = bo;
