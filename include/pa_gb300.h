@@ -19,7 +19,8 @@
  *   - Result: out[i] = (sum_{j=0..h} key_start[j] * seed[(i-j) mod n] mod 2) XOR key_rest[i].
  *   - Precision: the FP32 FFT path measures every block's largest distance of an output value to the
  *     nearest integer; above residual_limit pa_process recomputes the block on the exact path, which
- *     forms the product over GF(2) itself (additive FFT).  Blocks with n > 2^27 (up to 2^30) run as 2^27-bit FP32 chunk blocks
+ *     forms the product over GF(2) itself (additive FFT).  Single short blocks (up to 1.07e10 bit
+ *     products, n = 2^17) are multiplied word by word, which is exact.  Blocks with n > 2^27 (up to 2^30) run as 2^27-bit FP32 chunk blocks
  *     (large-block decomposition) under the same guard.
  *
  * All functions return 0 (PA_OK) or a negative PA_ERR_* code; nothing exits the process.
@@ -65,12 +66,13 @@ typedef struct pa_config {
 } pa_config;
 
 typedef struct pa_stats {
-    float max_residual;       /* largest distance of an output value to the nearest integer */
+    float max_residual;       /* largest distance of an output value to the nearest integer (0 for a short block) */
     uint64_t popcount_key;    /* Hamming weight of key_start (count_one_of_global_key) */
     uint64_t popcount_seed;   /* Hamming weight of the seed (count_one_of_global_seed) */
-    float gpu_ms;             /* device time of the block (CUDA events) */
+    float gpu_ms;             /* device time of the block: its first kernel's start to its last one's end on the GPU's
+                                 global timer (CUDA events around a block above 2^27 bits and around a batch) */
     int32_t seed_uses_left;   /* remaining blocks for the cached seed, -1 = unlimited */
-    int32_t exact;            /* 0: FP32 path, one pass; 2: FP32 path as 2^27-bit chunk blocks (n > 2^27);
+    int32_t exact;            /* 0: FP32 path, one pass, or a short block, word by word; 2: FP32 path as 2^27-bit chunk blocks (n > 2^27);
                                  1: exact path (guard fallback or PA_FLAG_EXACT).  Popcounts are 0 for 1, 2 */
 } pa_stats;
 
@@ -116,7 +118,7 @@ PA_API int pa_kernels_per_block(uint32_t n, uint32_t v, uint32_t flags);
  * (PrivacyAmplification.cu:146-166, 2053-2074).  When enabled, every block records CUDA events on its
  * stream before the first and after each kernel (no host synchronisation).  pa_stage_times() waits
  * for the recorded blocks and writes the mean device time per kernel in ms (up to max_stages values,
- * order: pass A, pass B, pass C, finish; one value for single-CTA blocks), the stage count and the
+ * order: pass A, pass B, pass C, finish; one value for short and single-CTA blocks), the stage count and the
  * number of blocks averaged, then clears the record. */
 PA_API int pa_set_timing(pa_engine* e, int enable);
 PA_API int pa_stage_times(pa_engine* e, float* ms, int max_stages, int* nstages, int* nblocks);

@@ -355,7 +355,7 @@ int exact_in_slot(pa_engine* e, Slot* sl, const BlockGeom& g, const uint32_t* d_
     uint32_t* a = reinterpret_cast<uint32_t*>(sl->work);
     uint32_t* tmp = reinterpret_cast<uint32_t*>(sl->work2);
     int rc = pa::launch_exact_seed(g, d_seed, hat, tmp, s);
-    if (!rc) rc = pa::launch_exact_block(g, ks, kr, flags, hat, a, tmp, out, s);
+    if (!rc) rc = pa::launch_exact_block(g, d_seed, ks, kr, flags, hat, a, tmp, out, s);
     return rc ? cuda_fail(e, (cudaError_t)rc) : PA_OK;
 }
 

@@ -107,11 +107,13 @@ int seed_common(pa_engine* e, uint32_t n, int32_t reuse, cudaStream_t s) {
     e->spec_valid = false;
     e->exact_valid = false;
     e->chunk_valid = false;
+    e->count_valid = false;
     if (is_pow2(n)) {  // placement does not depend on v: build the spectrum now
         BlockGeom g;
         int rc = make_geom(n, n / 2u, PA_FLAG_COMPRESS, e->split, &g);
         if (rc) return rc;
         if (g.exact_only) return PA_OK;  // chunk spectra are built per block, the exact transform on demand
+        if (pa::short_geom(g)) return PA_OK;  // the block needs no spectrum, or builds it (g has the longest output)
         if (fuse_seed(e, g)) return PA_OK;  // transformed inside the block's column pass
         return build_spectrum(e, g, s);
     }
@@ -131,7 +133,7 @@ int fused_block(pa_engine* e, const uint32_t* d_ks, const uint32_t* d_kr, const 
     }
     e->spec_valid = false;
     rc = pa::launch_fused_block(g, e->d_seed, d_ks, d_kr, flags, e->d_spec, e->seed_maps, e->d_park, e->park_ctas,
-                                scratch(e), e->d_cnt, e->d_resid, d_out, e->num_sms, s, sev, kr_ready);
+                                scratch(e), e->d_cnt, e->d_resid, d_out, e->num_sms, s, sev, kr_ready, e->d_words->clock);
     return rc ? cuda_fail(e, (cudaError_t)rc) : PA_OK;
 }
 
@@ -143,7 +145,7 @@ uint32_t* exact_scratch(pa_engine* e) {
 }
 
 int build_exact_seed(pa_engine* e, const BlockGeom& g, cudaStream_t s) {
-    int rc = pa::launch_exact_seed(g, e->d_seed, e->d_exact_seed, exact_scratch(e), s);
+    int rc = pa::launch_exact_seed(g, e->d_seed, e->d_exact_seed, exact_scratch(e), s, e->d_words->clock);
     if (rc) return cuda_fail(e, (cudaError_t)rc);
     e->exact_geom = g;
     e->exact_valid = true;
@@ -188,15 +190,47 @@ int chunked_block(pa_engine* e, const uint32_t* d_ks, const uint32_t* d_kr, cons
     return PA_OK;
 }
 
+// The stage events of one block while timing is on (null otherwise).
+cudaEvent_t* stage_events(pa_engine* e, const BlockGeom& g) {
+    if (!e->timing || e->tev.empty()) return nullptr;
+    const size_t slot = e->tev_next;
+    e->tev_stages[slot] = pa::stage_count_key_block(g);
+    e->tev_next = (slot + 1) % e->tev.size();
+    e->tev_count = std::min(e->tev_count + 1, e->tev.size());
+    return e->tev[slot].data();
+}
+
+// A short block word by word (pa_direct.cu): exact, so that its residual is zero.  The seed's popcount is formed with
+// the first block of a seed and placement.
+int direct_block(pa_engine* e, const uint32_t* d_ks, const uint32_t* d_kr, const BlockGeom& g, uint32_t flags,
+                 uint32_t* d_out, cudaStream_t s) {
+    if (pa::direct_overlap(g, d_ks, d_out)) {  // every result word reads the whole key
+        PA_CUDA(e, cudaMemcpyAsync(e->d_key_start, d_ks, (size_t)(g.h / 32u + 1u) * 4u, cudaMemcpyDeviceToDevice, s));
+        d_ks = e->d_key_start;
+    }
+    const bool counted = e->count_valid && same_seed_geom(e->count_geom, g);
+    cudaEvent_t* ev = stage_events(e, g);
+    if (ev) cudaEventRecord(ev[0], s);
+    int rc = pa::launch_direct(g, e->d_seed, d_ks, d_kr, flags, d_out, s, {e->d_words->short_cnt, e->d_resid, counted ? 0 : 1, e->d_words->clock});
+    if (rc) return cuda_fail(e, (cudaError_t)rc);
+    if (ev) cudaEventRecord(ev[1], s);
+    e->count_geom = g;
+    e->count_valid = true;
+    return PA_OK;
+}
+
 // Exact path for one block (the seed's transform is built on first use and cached with the seed).
 int exact_block(pa_engine* e, const uint32_t* d_ks, const uint32_t* d_kr, const BlockGeom& g, uint32_t flags,
                 uint32_t* d_out, cudaStream_t s) {
-    if (!e->exact_valid || !same_exact_geom(e->exact_geom, g)) {
+    unsigned long long* const clock = e->d_words->clock;
+    unsigned long long* start = clock;  // of the seed's transform if that runs first
+    if (!pa::direct_geom(g) && (!e->exact_valid || !same_exact_geom(e->exact_geom, g))) {
         int rc = build_exact_seed(e, g, s);
         if (rc) return rc;
+        start = nullptr;
     }
-    int rc = pa::launch_exact_block(g, d_ks, d_kr, flags, e->d_exact_seed, reinterpret_cast<uint32_t*>(e->d_work),
-                                    exact_scratch(e), d_out, s);
+    int rc = pa::launch_exact_block(g, e->d_seed, d_ks, d_kr, flags, e->d_exact_seed, reinterpret_cast<uint32_t*>(e->d_work),
+                                    exact_scratch(e), d_out, s, start, clock);
     if (rc) return cuda_fail(e, (cudaError_t)rc);
     // the exact path leaves no residual: report 0 and the reference popcounts are not needed
     PA_CUDA(e, cudaMemsetAsync(e->d_resid, 0, sizeof(unsigned int), s));
@@ -207,14 +241,12 @@ int block_common(pa_engine* e, const uint32_t* d_ks, const uint32_t* d_kr, const
                  uint32_t* d_out, cudaStream_t s, cudaEvent_t kr_ready = nullptr) {
     if (!e->seed_valid || e->seed_left == 0) return PA_ERR_NO_SEED;
     if (g.n != e->seed_n) return PA_ERR_INVALID_ARG;
-    e->last_chunked = false;
+    e->last_chunked = e->last_direct = false;
     if (kr_ready && ((flags & PA_FLAG_EXACT) || g.exact_only))  // these paths read key_rest early
         PA_CUDA(e, cudaStreamWaitEvent(s, kr_ready, 0));
     if (flags & PA_FLAG_EXACT) {
-        PA_CUDA(e, cudaEventRecord(e->ev0, s));
         int rc = exact_block(e, d_ks, d_kr, g, flags, d_out, s);
         if (rc) return rc;
-        PA_CUDA(e, cudaEventRecord(e->ev1, s));
         e->last_exact = true;
         if (e->seed_left > 0) --e->seed_left;
         return PA_OK;
@@ -229,6 +261,14 @@ int block_common(pa_engine* e, const uint32_t* d_ks, const uint32_t* d_kr, const
         if (e->seed_left > 0) --e->seed_left;
         return PA_OK;
     }
+    if (pa::short_geom(g)) {
+        if (kr_ready) PA_CUDA(e, cudaStreamWaitEvent(s, kr_ready, 0));
+        int rc = direct_block(e, d_ks, d_kr, g, flags, d_out, s);
+        if (rc) return rc;
+        e->last_direct = true;
+        if (e->seed_left > 0) --e->seed_left;
+        return PA_OK;
+    }
     const bool fused = (!e->spec_valid || !same_seed_geom(e->spec_geom, g)) && fuse_seed(e, g);
     if (!fused && (!e->spec_valid || !same_seed_geom(e->spec_geom, g))) {
         int rc = build_spectrum(e, g, s);
@@ -236,24 +276,15 @@ int block_common(pa_engine* e, const uint32_t* d_ks, const uint32_t* d_kr, const
     }
     int mrc = ensure_maps(e, g);
     if (mrc) return mrc;
-    PA_CUDA(e, cudaEventRecord(e->ev0, s));
-    cudaEvent_t* sev = nullptr;
-    if (e->timing && !e->tev.empty()) {
-        size_t slot = e->tev_next;
-        sev = e->tev[slot].data();
-        e->tev_stages[slot] = pa::stage_count_key_block(g);
-        e->tev_next = (slot + 1) % e->tev.size();
-        e->tev_count = std::min(e->tev_count + 1, e->tev.size());
-    }
+    cudaEvent_t* sev = stage_events(e, g);
     if (fused) {
         int rc = fused_block(e, d_ks, d_kr, g, flags, d_out, s, sev, kr_ready);
         if (rc) return rc;
     } else {
         int rc = pa::launch_key_block(g, d_ks, d_kr, flags, e->d_spec, scratch(e), e->d_cnt, e->d_resid, d_out,
-                                      e->num_sms, s, sev, kr_ready);
+                                      e->num_sms, s, sev, kr_ready, e->d_words->clock);
         if (rc) return cuda_fail(e, (cudaError_t)rc);
     }
-    PA_CUDA(e, cudaEventRecord(e->ev1, s));
     if (e->seed_left > 0) --e->seed_left;
     return PA_OK;
 }
@@ -271,11 +302,12 @@ int take_stats(pa_engine* e, pa_stats* st, float* resid_out) {
     *resid_out = resid;
     if (st) {
         st->max_residual = resid;
-        const bool counted = !e->last_exact && !e->last_chunked;  // popcounts exist on the one-pass FP32 path
-        st->popcount_key = counted ? w.cnt[0] : 0;
-        st->popcount_seed = counted ? w.cnt[1] : 0;
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, e->ev0, e->ev1);
+        const bool counted = !e->last_exact && !e->last_chunked;  // short blocks and the one-pass FP32 path
+        const unsigned long long* cnt = e->last_direct ? w.short_cnt : w.cnt;
+        st->popcount_key = counted ? cnt[0] : 0;
+        st->popcount_seed = counted ? cnt[1] : 0;
+        float ms = w.clock[1] > w.clock[0] ? (float)((double)(w.clock[1] - w.clock[0]) * 1e-6) : 0.f;
+        if (e->last_chunked) cudaEventElapsedTime(&ms, e->ev0, e->ev1);
         st->gpu_ms = ms;
         st->seed_uses_left = e->seed_left < 0 ? -1 : (int32_t)e->seed_left;
         st->exact = e->last_exact ? 1 : (e->last_chunked ? 2 : 0);

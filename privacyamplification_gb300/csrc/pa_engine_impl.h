@@ -38,6 +38,7 @@ struct pa_engine {
     uint32_t* d_exact_seed = nullptr;  // the seed's transform (exact path), up to Np / 4 words
     bool exact_valid = false;          // d_exact_seed matches the current seed for exact_geom
     bool last_exact = false;           // the last block ran on the exact path
+    bool last_direct = false;          // the last block was a short one (pa_direct.cu)
     bool last_chunked = false;         // the last block ran as FP32 chunk blocks (n > 2^27)
     pa::BlockGeom exact_geom{};
     pa::PassMaps maps{};        // tensor maps for the geometry maps_key
@@ -61,9 +62,11 @@ struct pa_engine {
     uint32_t* d_planes = nullptr;
     // a block's words, in one allocation (d_words) that one copy brings to the host
     struct Words {
-        unsigned long long cnt[2];  // key popcount, seed popcount
-        unsigned int resid;         // largest residual (float bits)
-        int err;                    // bounded device waits that expired
+        unsigned long long cnt[2];        // key popcount, seed popcount (pass C reads them beside the spectrum)
+        unsigned long long short_cnt[2];  // the same of a short block, whose seed's count outlives the block
+        unsigned long long clock[2];      // the block's start and end on the global timer, ns
+        unsigned int resid;               // largest residual (float bits)
+        int err;                          // bounded device waits that expired
     };
     Words* d_words = nullptr;
     unsigned long long* d_cnt = nullptr;  // d_words->cnt
@@ -79,6 +82,8 @@ struct pa_engine {
     int64_t seed_left = 0;  // -1 = unlimited
     bool spec_valid = false;
     pa::BlockGeom spec_geom{};
+    bool count_valid = false;  // short_cnt[1] is the seed's popcount for count_geom
+    pa::BlockGeom count_geom{};
     int last_cuda = 0;
     bool pending = false;  // device-form work queued and not yet synchronised
     // per-kernel timing ring (pa_set_timing / pa_stage_times)

@@ -86,10 +86,11 @@ __device__ __forceinline__ void transpose16(uint32_t (&w)[16]) {
 // p's word s at V[p * pw + s] holds the elements 32 s .. 32 s + 31.
 template <bool SEED>
 __global__ void __launch_bounds__(128) k_exact_planes(const uint32_t* __restrict__ src, BlockGeom g, uint32_t pw,
-                                                      uint32_t* __restrict__ V) {
+                                                      uint32_t* __restrict__ V, unsigned long long* clock) {
     const uint32_t s = blockIdx.x * 128u + threadIdx.x;
     if (s >= pw) return;
     pdl_wait();
+    if (clock && s == 0) clock_start(clock);
     const uint32_t H = g.h / 32u, nw = g.n / 32u;
     const uint64_t tbits = (uint64_t)g.h + g.out_bits;
     auto word = [&](uint64_t q) -> uint32_t {
@@ -123,7 +124,8 @@ __global__ void __launch_bounds__(128) k_exact_planes(const uint32_t* __restrict
 // Planes of the result -> output words, XOR key_rest, reference byte order.
 __global__ void __launch_bounds__(128) k_exact_words(const uint32_t* __restrict__ V, BlockGeom g, uint32_t pw,
                                                      const uint32_t* __restrict__ key_rest, uint32_t flags,
-                                                     uint32_t* __restrict__ out, uint32_t nwords) {
+                                                     uint32_t* __restrict__ out, uint32_t nwords,
+                                                     unsigned long long* clock) {
     const uint32_t s = blockIdx.x * 128u + threadIdx.x;
     if (s >= pw || 16u * s >= nwords) return;
     pdl_wait();
@@ -142,6 +144,7 @@ __global__ void __launch_bounds__(128) k_exact_words(const uint32_t* __restrict_
         if ((flags & 1u) && 32ull * q < g.v) w ^= load(key_rest + q);
         out[q] = __byte_perm(w, 0, 0x0123);
     }
+    if (clock && threadIdx.x == 0) clock_end(clock);
 }
 
 // ============================================================================ basis conversion
@@ -1043,13 +1046,13 @@ int exact_kernel_count(const BlockGeom& g) {
 }
 
 // Buffers: P = 2^l field elements are at most Np / 8 words, 32 planes as much.
-int launch_exact_seed(const BlockGeom& g, const uint32_t* seed, uint32_t* seed_hat, uint32_t* tmp, cudaStream_t s) {
-    if (direct_geom(g))  // the block kernel reads the seed itself
-        return (int)cudaMemcpyAsync(seed_hat, seed, (size_t)(g.n / 32u) * 4u, cudaMemcpyDeviceToDevice, s);
+int launch_exact_seed(const BlockGeom& g, const uint32_t* seed, uint32_t* seed_hat, uint32_t* tmp, cudaStream_t s,
+                      unsigned long long* clock) {
+    if (direct_geom(g)) return 0;
     const Shape sh = shape_of(g);
     Chain ch{s};
     const size_t P = size_t(32) * sh.pw;
-    ch.run(k_exact_planes<true>, (sh.pw + 127u) / 128u, 128, 0, seed, g, sh.pw, tmp);
+    ch.run(k_exact_planes<true>, (sh.pw + 127u) / 128u, 128, 0, seed, g, sh.pw, tmp, clock);
     const uint32_t* V = convert_basis<kIT>(sh, tmp, tmp + P, 32, ch);
     ch.run(k_exact_to_field<true>, sh.pw / kConvThreads, kConvThreads, 0, V, sh.pw, seed_hat);
     top_levels<kIT>(sh, seed_hat, ch);
@@ -1057,20 +1060,21 @@ int launch_exact_seed(const BlockGeom& g, const uint32_t* seed, uint32_t* seed_h
     return (int)ch.err;
 }
 
-int launch_exact_block(const BlockGeom& g, const uint32_t* key_start, const uint32_t* key_rest, uint32_t flags,
-                       const uint32_t* seed_hat, uint32_t* a, uint32_t* tmp, uint32_t* out_words, cudaStream_t s) {
+int launch_exact_block(const BlockGeom& g, const uint32_t* seed, const uint32_t* key_start, const uint32_t* key_rest,
+                       uint32_t flags, const uint32_t* seed_hat, uint32_t* a, uint32_t* tmp, uint32_t* out_words,
+                       cudaStream_t s, unsigned long long* start, unsigned long long* end) {
     if (direct_geom(g)) {
         if (direct_overlap(g, key_start, out_words)) {  // every result word reads the whole key
             cudaError_t err = cudaMemcpyAsync(a, key_start, 4u * (size_t)(g.h / 32u + 1u), cudaMemcpyDeviceToDevice, s);
             if (err != cudaSuccess) return (int)err;
             key_start = a;
         }
-        return launch_direct(g, seed_hat, key_start, key_rest, flags, out_words, s);
+        return launch_direct(g, seed, key_start, key_rest, flags, out_words, s, {nullptr, nullptr, 0, start});
     }
     const Shape sh = shape_of(g);
     Chain ch{s};
     const size_t half = size_t(16) * sh.pw;
-    ch.run(k_exact_planes<false>, (sh.pw + 127u) / 128u, 128, 0, key_start, g, sh.pw, tmp);
+    ch.run(k_exact_planes<false>, (sh.pw + 127u) / 128u, 128, 0, key_start, g, sh.pw, tmp, start);
     const uint32_t* V = convert_basis<kF>(sh, tmp, tmp + half, 16, ch);
     ch.run(k_exact_to_field<false>, sh.pw / kConvThreads, kConvThreads, 0, V, sh.pw, a);
     top_levels<kF>(sh, a, ch);
@@ -1080,7 +1084,7 @@ int launch_exact_block(const BlockGeom& g, const uint32_t* key_start, const uint
     V = convert_basis<kT>(sh, tmp, tmp + half, 16, ch);
     const uint32_t nwords = (g.out_bits + 31u) / 32u;
     ch.run(k_exact_words, ((nwords + 15u) / 16u + 127u) / 128u, 128, 0, V, g, sh.pw, key_rest, flags, out_words,
-           nwords);
+           nwords, end);
     return (int)ch.err;
 }
 

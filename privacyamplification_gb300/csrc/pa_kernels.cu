@@ -285,7 +285,8 @@ int launch_seed_spectrum(const BlockGeom& g, const uint32_t* seed, float2* spec,
 
 int launch_key_block(const BlockGeom& g, const uint32_t* key_start, const uint32_t* key_rest, uint32_t flags,
                      const float2* spec, const Scratch& sc, unsigned long long* cnt, unsigned int* resid_bits,
-                     uint32_t* out_words, int num_sms, cudaStream_t s, cudaEvent_t* ev, cudaEvent_t key_rest_ready) {
+                     uint32_t* out_words, int num_sms, cudaStream_t s, cudaEvent_t* ev, cudaEvent_t key_rest_ready,
+                     unsigned long long* clock) {
     auto mark = [&](int i) {
         if (ev) cudaEventRecord(ev[i], s);
     };
@@ -300,7 +301,8 @@ int launch_key_block(const BlockGeom& g, const uint32_t* key_start, const uint32
         return rc;
     }
     mark(0);
-    int rc = launch_bit_rows(g, key_start, false, sc.planes, s, kOneBlock, cnt, resid_bits);  // cnt[1] is the seed's
+    int rc = launch_bit_rows(g, key_start, false, sc.planes, s, kOneBlock, cnt, resid_bits,
+                             clock);  // cnt[1] is the seed's
     if (!rc) rc = launch_pass_a(g, sc.planes, false, sc.work, cnt, num_sms, s);
     mark(1);
     if (!rc) rc = launch_pass_b(g, false, *sc.maps, sc.work, sc.work2, const_cast<float2*>(spec), sc.err, num_sms, s);
@@ -308,7 +310,7 @@ int launch_key_block(const BlockGeom& g, const uint32_t* key_start, const uint32
     if (!rc) rc = launch_pass_c(g, *sc.maps, sc.work2, cnt, sc.planes, resid_bits, sc.err, num_sms, s);
     mark(3);
     if (!rc && key_rest_ready) rc = (int)cudaStreamWaitEvent(s, key_rest_ready, 0);  // key_rest copied meanwhile
-    if (!rc) rc = launch_finish(g, sc.planes, key_rest, flags, out_words, s);
+    if (!rc) rc = launch_finish(g, sc.planes, key_rest, flags, out_words, s, kOneBlock, clock);
     mark(4);
     return rc;
 }
@@ -316,13 +318,14 @@ int launch_key_block(const BlockGeom& g, const uint32_t* key_start, const uint32
 int launch_fused_block(const BlockGeom& g, const uint32_t* seed, const uint32_t* key_start, const uint32_t* key_rest,
                        uint32_t flags, float2* seed_y, const PassMaps& seed_maps, float2* park, uint32_t park_ctas,
                        const Scratch& sc, unsigned long long* cnt, unsigned int* resid_bits, uint32_t* out_words,
-                       int num_sms, cudaStream_t s, cudaEvent_t* ev, cudaEvent_t key_rest_ready) {
+                       int num_sms, cudaStream_t s, cudaEvent_t* ev, cudaEvent_t key_rest_ready,
+                       unsigned long long* clock) {
     if (!fused_geom(g)) return (int)cudaErrorInvalidValue;
     auto mark = [&](int i) {
         if (ev) cudaEventRecord(ev[i], s);
     };
     mark(0);
-    int rc = launch_bit_rows(g, seed, true, sc.planes, s, kOneBlock, cnt + 1);
+    int rc = launch_bit_rows(g, seed, true, sc.planes, s, kOneBlock, cnt + 1, nullptr, clock);
     if (!rc) rc = launch_pass_a(g, sc.planes, true, seed_y, cnt + 1, num_sms, s);
     if (!rc) rc = launch_bit_rows(g, key_start, false, sc.planes, s, kOneBlock, cnt, resid_bits);
     if (!rc) rc = launch_pass_a(g, sc.planes, false, sc.work, cnt, num_sms, s);
@@ -332,7 +335,7 @@ int launch_fused_block(const BlockGeom& g, const uint32_t* seed, const uint32_t*
     if (!rc) rc = launch_pass_c(g, *sc.maps, sc.work2, cnt, sc.planes, resid_bits, sc.err, num_sms, s);
     mark(3);
     if (!rc && key_rest_ready) rc = (int)cudaStreamWaitEvent(s, key_rest_ready, 0);  // key_rest copied meanwhile
-    if (!rc) rc = launch_finish(g, sc.planes, key_rest, flags, out_words, s);
+    if (!rc) rc = launch_finish(g, sc.planes, key_rest, flags, out_words, s, kOneBlock, clock);
     mark(4);
     return rc;
 }
@@ -352,7 +355,7 @@ int launch_group_mono_key(const BlockGeom& g, const Group& gp, uint32_t flags, c
 #undef C
 }
 
-int kernel_count_key_block(const BlockGeom& g) { return g.log_n1 == 0 ? 1 : 5; }
-int stage_count_key_block(const BlockGeom& g) { return g.log_n1 == 0 ? 1 : 4; }
+int kernel_count_key_block(const BlockGeom& g) { return g.log_n1 == 0 || short_geom(g) ? 1 : 5; }
+int stage_count_key_block(const BlockGeom& g) { return g.log_n1 == 0 || short_geom(g) ? 1 : 4; }
 
 }  // namespace pa

@@ -72,10 +72,12 @@ int launch_seed_spectrum(const BlockGeom& g, const uint32_t* seed, float2* spec,
 // stage_ev (optional, kernel_count_key_block()+1 events) is recorded before the first kernel and
 // after each stage.  key_rest_ready (optional): the stream waits on it before the first kernel that
 // reads key_rest (k_finish, or the single-CTA kernel), so key_rest may still be arriving meanwhile.
+// clock (optional; three-pass blocks, short blocks and the exact path): two words that receive the start of the
+// block's first kernel and the end of its last one (pa_launch.cuh).
 int launch_key_block(const BlockGeom& g, const uint32_t* key_start, const uint32_t* key_rest, uint32_t flags,
                      const float2* spec, const Scratch& sc, unsigned long long* cnt, unsigned int* resid_bits,
                      uint32_t* out_words, int num_sms, cudaStream_t s, cudaEvent_t* stage_ev,
-                     cudaEvent_t key_rest_ready = nullptr);
+                     cudaEvent_t key_rest_ready = nullptr, unsigned long long* clock = nullptr);
 // A key block whose seed serves it alone, the seed's column transform fused into the key's column pass
 // (fused_geom(g) only): seed_y (N complex values, where the spectrum would go) receives the seed's row
 // pass, seed_maps are over seed_y, park holds park_ctas * kParkBytes; cnt[0] / cnt[1] receive the key and
@@ -83,7 +85,8 @@ int launch_key_block(const BlockGeom& g, const uint32_t* key_start, const uint32
 int launch_fused_block(const BlockGeom& g, const uint32_t* seed, const uint32_t* key_start, const uint32_t* key_rest,
                        uint32_t flags, float2* seed_y, const PassMaps& seed_maps, float2* park, uint32_t park_ctas,
                        const Scratch& sc, unsigned long long* cnt, unsigned int* resid_bits, uint32_t* out_words,
-                       int num_sms, cudaStream_t s, cudaEvent_t* stage_ev, cudaEvent_t key_rest_ready = nullptr);
+                       int num_sms, cudaStream_t s, cudaEvent_t* stage_ev, cudaEvent_t key_rest_ready = nullptr,
+                       unsigned long long* clock = nullptr);
 int kernel_count_key_block(const BlockGeom& g);   // kernels one key block launches
 int stage_count_key_block(const BlockGeom& g);    // timed stages (events - 1) of a key block
 
@@ -126,7 +129,7 @@ int launch_group_mono_key(const BlockGeom& g, const Group& gp, uint32_t flags, c
 // zero_cnt, zero_resid (may be null): words of the block that this first kernel clears.
 int launch_bit_rows(const BlockGeom& g, const uint32_t* bits, bool seed, uint32_t* rows, cudaStream_t s,
                     const Group& gp = kOneBlock, unsigned long long* zero_cnt = nullptr,
-                    unsigned int* zero_resid = nullptr);
+                    unsigned int* zero_resid = nullptr, unsigned long long* clock = nullptr);
 int launch_pass_a(const BlockGeom& g, const uint32_t* rows, bool seed, float2* Y, unsigned long long* cnt,
                   int num_sms, cudaStream_t s, const Group& gp = kOneBlock);
 struct PassMaps {
@@ -160,18 +163,33 @@ int launch_pass_c(const BlockGeom& g, const PassMaps& maps, const float2* Z, con
                   uint32_t* planes, unsigned int* resid, int* err, int num_sms, cudaStream_t s,
                   const Group& gp = kOneBlock);
 int launch_finish(const BlockGeom& g, const uint32_t* planes, const uint32_t* key_rest, uint32_t flags,
-                  uint32_t* out, cudaStream_t s, const Group& gp = kOneBlock);
+                  uint32_t* out, cudaStream_t s, const Group& gp = kOneBlock, unsigned long long* clock = nullptr);
 
 // Exact path (pa_exact.cu): the product over GF(2) by an additive FFT, or for short blocks (direct_geom,
 // pa_direct.cu) word by word.  With P <= max(2^16, 3 Np / 16) words:
-// seed_hat and a hold P, tmp 2 P (and n / 32 words each); seed_hat holds for the same n, h and out_bits.
-int launch_exact_seed(const BlockGeom& g, const uint32_t* seed, uint32_t* seed_hat, uint32_t* tmp, cudaStream_t s);
-int launch_exact_block(const BlockGeom& g, const uint32_t* key_start, const uint32_t* key_rest, uint32_t flags,
-                       const uint32_t* seed_hat, uint32_t* a, uint32_t* tmp, uint32_t* out_words, cudaStream_t s);
+// seed_hat and a hold P (a also n / 32 words), tmp 2 P; seed_hat holds for the same n, h and out_bits.
+// Short blocks have no transform of the seed: launch_exact_seed does nothing and the block reads the seed itself.
+int launch_exact_seed(const BlockGeom& g, const uint32_t* seed, uint32_t* seed_hat, uint32_t* tmp, cudaStream_t s,
+                      unsigned long long* clock = nullptr);
+int launch_exact_block(const BlockGeom& g, const uint32_t* seed, const uint32_t* key_start, const uint32_t* key_rest,
+                       uint32_t flags, const uint32_t* seed_hat, uint32_t* a, uint32_t* tmp, uint32_t* out_words,
+                       cudaStream_t s, unsigned long long* start = nullptr, unsigned long long* end = nullptr);
 bool direct_geom(const BlockGeom& g);
+// Single blocks that run word by word without being asked to (the pool and its groups keep to the transforms, whose
+// rate is higher with several blocks in flight).
+bool short_geom(const BlockGeom& g);
 bool direct_overlap(const BlockGeom& g, const uint32_t* key_start, const uint32_t* out_words);
+// cnt (may be null): receives the key's popcount and, with count_seed, the placed seed's in cnt[1]; *resid then
+// becomes zero.
+struct DirectCounts {
+    unsigned long long* cnt;
+    unsigned int* resid;
+    int count_seed;
+    unsigned long long* clock;
+};
+constexpr DirectCounts kNoCounts{nullptr, nullptr, 0, nullptr};
 int launch_direct(const BlockGeom& g, const uint32_t* seed, const uint32_t* key_start, const uint32_t* key_rest,
-                  uint32_t flags, uint32_t* out_words, cudaStream_t s);
+                  uint32_t flags, uint32_t* out_words, cudaStream_t s, const DirectCounts& dc = kNoCounts);
 int exact_kernel_count(const BlockGeom& g);
 
 // Blocks beyond the single-pass FP32 size (pa_chunk.cu): side x side chunks as transforms of n' = 2 side bits on

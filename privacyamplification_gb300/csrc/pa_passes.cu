@@ -21,14 +21,16 @@
 
 namespace pa {
 
-// A block's popcount and residual words, cleared by its first kernel (later kernels add to them).
+// A block's popcount and residual words, cleared by its first kernel (later kernels add to them), and its clock.
 struct Zeroed {
     unsigned long long* cnt;
     unsigned int* resid;
+    unsigned long long* clock;
     __device__ __forceinline__ void clear() const {
         if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) {
             if (cnt) *cnt = 0ull;
             if (resid) *resid = 0u;
+            if (clock) clock_start(clock);
         }
     }
 };
@@ -170,7 +172,8 @@ __global__ void __launch_bounds__((1 << LOGL) / 32, 1)
 // XORed with key_rest word ow.
 __global__ void __launch_bounds__(1024) k_finish(const uint32_t* __restrict__ planes, BlockGeom g,
                                                  const uint32_t* __restrict__ key_rest, uint32_t flags,
-                                                 uint32_t* __restrict__ out, uint32_t nwords, Group gp) {
+                                                 uint32_t* __restrict__ out, uint32_t nwords, Group gp,
+                                                 unsigned long long* clock) {
     pdl_wait();
     if (gp.e) {  // block blockIdx.z of a group
         planes += (size_t)blockIdx.z * gp.planes;
@@ -197,6 +200,7 @@ __global__ void __launch_bounds__(1024) k_finish(const uint32_t* __restrict__ pl
         if ((flags & kXor) && 32ull * ow < g.v) w ^= load(key_rest + ow);
         out[ow] = __byte_perm(w, 0, 0x0123);
     }
+    if (clock && lane == 0) clock_end(clock);
 }
 
 // Tiled form for N1 >= 256: a CTA takes plane rows m1 = m10 .. m10+255 and plane word columns
@@ -205,7 +209,8 @@ __global__ void __launch_bounds__(1024) k_finish(const uint32_t* __restrict__ pl
 // (64 bytes), with key_rest read the same way.
 __global__ void __launch_bounds__(256) k_finish_tiled(const uint32_t* __restrict__ planes, BlockGeom g,
                                                       const uint32_t* __restrict__ key_rest, uint32_t flags,
-                                                      uint32_t* __restrict__ out, uint32_t nwords, Group gp) {
+                                                      uint32_t* __restrict__ out, uint32_t nwords, Group gp,
+                                                      unsigned long long* clock) {
     __shared__ uint32_t se[256][9], so[256][9];  // [m1 - m10][c - c0], even / odd samples
     __shared__ uint32_t sw[256][17];             // [m2 - 32 c0][(m1 - m10) / 16]
     pdl_wait();
@@ -259,6 +264,7 @@ __global__ void __launch_bounds__(256) k_finish_tiled(const uint32_t* __restrict
         const uint64_t ow = ((32ull * c0 + (uint64_t)ml) * n1 + m10) / 16ull + (uint64_t)j;
         if (ow < nwords) out[ow] = __byte_perm(sw[ml][j] ^ kr[i], 0, 0x0123);
     }
+    if (clock && t == 0) clock_end(clock);
 }
 
 // ============================================================================ launchers
@@ -291,8 +297,9 @@ static int group_ctas(uint32_t units, int per_wave, const Group& gp) {
 }
 
 int launch_bit_rows(const BlockGeom& g, const uint32_t* bits, bool seed, uint32_t* rows, cudaStream_t s,
-                    const Group& gp, unsigned long long* zero_cnt, unsigned int* zero_resid) {
-    const Zeroed z{zero_cnt, zero_resid};
+                    const Group& gp, unsigned long long* zero_cnt, unsigned int* zero_resid,
+                    unsigned long long* clock) {
+    const Zeroed z{zero_cnt, zero_resid, clock};
     const uint32_t n1 = 1u << g.log_n1, n2 = 1u << g.log_n2;
     if (n1 >= 256u && n2 >= 256u) {
         dim3 grid(n1 / 256u, n2 / 256u, gp.count);
@@ -559,7 +566,7 @@ int make_group_maps(const BlockGeom& g, const float2* Y, const float2* Z, uint32
 }
 
 int launch_finish(const BlockGeom& g, const uint32_t* planes, const uint32_t* key_rest, uint32_t flags,
-                  uint32_t* out, cudaStream_t s, const Group& gp) {
+                  uint32_t* out, cudaStream_t s, const Group& gp, unsigned long long* clock) {
     const uint32_t n1 = 1u << g.log_n1, wpr = (1u << g.log_n2) / 32u;
     const uint32_t nwords = (g.out_bits + 31u) / 32u;
     // only plane columns that hold output samples: m2 < ceil(out_bits / (2 N1))
@@ -567,10 +574,10 @@ int launch_finish(const BlockGeom& g, const uint32_t* planes, const uint32_t* ke
     const uint32_t cols = std::min<uint32_t>(wpr, (m2max + 31u) / 32u);
     if (n1 >= 256u) {
         dim3 grid(n1 / 256u, (cols + 7u) / 8u, gp.count);
-        return (int)launch_pdl(k_finish_tiled, grid, 256, 0, s, planes, g, key_rest, flags, out, nwords, gp);
+        return (int)launch_pdl(k_finish_tiled, grid, 256, 0, s, planes, g, key_rest, flags, out, nwords, gp, clock);
     }
     dim3 grid((n1 / 32u + 3u) / 4u, (cols + 7u) / 8u, gp.count);
-    return (int)launch_pdl(k_finish, grid, 1024, 0, s, planes, g, key_rest, flags, out, nwords, gp);
+    return (int)launch_pdl(k_finish, grid, 1024, 0, s, planes, g, key_rest, flags, out, nwords, gp, clock);
 }
 
 }  // namespace pa

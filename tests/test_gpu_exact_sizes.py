@@ -59,3 +59,35 @@ def test_noalloc_output_over_an_input(n, v, where):
     torch.cuda.synchronize()
     got = bufs[where].cpu().numpy().view(np.uint8)[: v // 8]
     assert np.array_equal(got, O.direct(seed, ks, kr, n, v))
+
+
+@pytest.mark.parametrize("n,v", [(1024, 32), (1056, 480), (4096, 1536), (10240, 10208), (10304, 10272), (20480, 7680),
+                                 (32768, 12288), (65536, 24576), (65568, 40032), (131072, 49152), (196608, 73728),
+                                 (262144, 4096)])
+def test_short_blocks_by_default(gpu_engine, n, v):
+    """Short blocks of pa_process: whole output, zero residual, popcounts of the key and of the placed seed, the second
+    block against the kept seed's count."""
+    seed, recv = O.random_block(n, v, n + 3 * v)
+    ks, kr = O.key_split(recv, n, v)
+    gpu_engine.set_seed(seed, n, -1)
+    for _ in range(2):
+        out = gpu_engine.process(ks, kr, n, v)
+        st = gpu_engine.last_stats
+        assert np.array_equal(out, O.direct(seed, ks, kr, n, v))
+        assert st.exact == 0 and st.max_residual == 0
+        assert st.popcount_key == O.popcount(ks, n - v + 1)
+        if n & (n - 1) == 0:
+            assert st.popcount_seed == O.popcount(seed, n)
+
+
+def test_short_and_transformed_blocks_share_a_seed(gpu_engine):
+    """One seed, blocks on either side of the boundary in turn: the transformed block's spectrum and popcount are not
+    disturbed by the short block's, and the other way round."""
+    n = 294912
+    seed, recv = O.random_block(n, 32, 5)
+    gpu_engine.set_seed(seed, n, -1)
+    for v in (147456, 4096, 147456, 196608, 4096, 147456):
+        ks, kr = O.key_split(recv, n, v)
+        out = gpu_engine.process(ks, kr, n, v)
+        assert np.array_equal(out, O.ntt(seed, ks, kr, n, v)), v
+        assert gpu_engine.last_stats.popcount_key == O.popcount(ks, n - v + 1)
