@@ -262,7 +262,8 @@ int launch_chunked_block(const BlockGeom& g, const BlockGeom& gc, const uint32_t
     auto next_lane = [&]() -> const ChunkLane& { return cb.lane[turn++ & 1]; };
     auto column_pass = [&](const ChunkLane& L, bool is_seed, unsigned long long* cnt, float2* spec) {
         if (!rc) rc = launch_pass_a(gc, L.sc.planes, is_seed, L.sc.work, cnt, num_sms, L.s);
-        if (!rc) rc = launch_pass_b(gc, true, *L.sc.maps, L.sc.work, L.sc.work2, spec, L.sc.err, num_sms, L.s);
+        if (!rc) rc = launch_pass_b(gc, true, *L.sc.maps, L.sc.work, L.sc.work2, spec, L.sc.err, num_sms, L.s,
+                                   kOneBlock, true);
     };
     auto seed_window = [&](int d) {
         const ChunkLane& L = next_lane();

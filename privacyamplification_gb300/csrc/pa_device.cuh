@@ -231,4 +231,26 @@ __device__ __forceinline__ void real_merge(float2 pa, float2 pb, float2 w, float
     qb = cadd(cadd(pb, pac), mul_i(cmul(make_float2(-w.x, -w.y), csub(pb, pac))));
 }
 
+// The product of two packed real spectra without forming them.  With Z = E + i O (E, O: transforms of the even and odd
+// samples) and w = W_2N^k, X = E + w O and the packed transform of the product of X and S = Es + w Os is
+//   Y[k] = Z[k] U + conj(Z[N-k]) V,   U = Es + A - w^2 A,  V = A + w^2 A,  A = i Os / 2,
+// and with the same Es, A for the bin N - k: Y[N-k] = Z[N-k] conj(Es - A + w^2 A) - conj(Z[k] V).  The seed keeps Es and
+// A, which need no twiddle (Es = (Z + conj Z')/2, A = (Z - conj Z')/4), in place of S[k] and S[N-k]: about half the FP32
+// operations of splitting both spectra, multiplying and merging (n = 2^27, kept
+// seed 884 -> 858 us a block, own seed 1355 -> 1325).
+__device__ __forceinline__ void spectrum_pair(float2 za, float2 zb, float sc, float2& es, float2& a) {
+    const float2 zbc = cconj(zb);
+    es = cscale(cadd(za, zbc), 0.5f * sc);
+    a = cscale(csub(za, zbc), 0.25f * sc);
+}
+// t = w^2 A.
+__device__ __forceinline__ void product_pair(float2 za, float2 zb, float2 es, float2 a, float2 t, float2& qa, float2& qb) {
+    const float2 d = csub(a, t), v = cadd(a, t);
+    const float2 u = cadd(es, d), m = csub(es, d);
+    qa.x = fmaf(zb.y, v.y, fmaf(zb.x, v.x, fmaf(-za.y, u.y, za.x * u.x)));
+    qa.y = fmaf(-zb.y, v.x, fmaf(zb.x, v.y, fmaf(za.y, u.x, za.x * u.y)));
+    qb.x = fmaf(za.y, v.y, fmaf(-za.x, v.x, fmaf(zb.y, m.y, zb.x * m.x)));
+    qb.y = fmaf(za.y, v.x, fmaf(za.x, v.y, fmaf(-zb.x, m.y, zb.y * m.x)));
+}
+
 }  // namespace pa

@@ -143,8 +143,9 @@ int make_group_maps(const BlockGeom& g, const float2* Y, const float2* Z, uint32
 // columns, over `blocks` consecutive blocks.
 int encode_pass_maps(int log_n1, int log_n2, uint32_t cpt, const float2* Y, const float2* Z, CUtensorMap* out,
                      uint32_t blocks = 1);
+// xspec: a seed pass that stores real spectra (columns of 2^12; see pass_b_tiles).
 int launch_pass_b(const BlockGeom& g, bool seed, const PassMaps& maps, float2* Y, float2* Z, float2* spec, int* err,
-                  int num_sms, cudaStream_t s, const Group& gp = kOneBlock);
+                  int num_sms, cudaStream_t s, const Group& gp = kOneBlock, bool xspec = false);
 // A group's pass B with columns of 2^LOGL (pa_group.cu), grid and shared memory as launch_pass_b chose.
 template <int LOGL>
 int launch_pass_b_group(bool seed, dim3 grid, size_t smem, const CUtensorMap& mapY, float2* Y, float2* Z,

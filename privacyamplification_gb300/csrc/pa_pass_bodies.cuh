@@ -281,7 +281,8 @@ struct PassBBases {
 // FUSED: a seed used by this block only.  Every tile is taken twice, first from the seed's row pass output
 // (mapYs) as a seed pass, its spectrum tile parked in this CTA's CPT * L values of `spec` (written and read
 // back by the same CTA a tile later, so it stays in L2), then from the key's (mapY) as a key pass against it.
-template <int LOGL, bool SEED, int NT, bool GRP = false, bool FUSED = false>
+// XSPEC (a seed pass): spectra as X = real spectrum instead of the (E, A) form, for sums of products (pa_chunk.cu).
+template <int LOGL, bool SEED, int NT, bool GRP = false, bool FUSED = false, bool XSPEC = false>
 __device__ __forceinline__ void pass_b_tiles(const CUtensorMap* mapY, const float2* __restrict__ Y,
                                              float2* __restrict__ Z, const BlockGeom& g, float2* __restrict__ spec,
                                              int* err, int early, uint32_t first, uint32_t stride,
@@ -290,6 +291,7 @@ __device__ __forceinline__ void pass_b_tiles(const CUtensorMap* mapY, const floa
     constexpr int L = 1 << LOGL, E = 32, CPT = 32 * NT / L, LR = L / 16, SP = TileStride<L>::value;
     constexpr bool TMA = CPT <= 128;              // box inner extent 2*CPT floats <= 256
     static_assert(!FUSED || (TMA && !GRP && !SEED), "the fused pass is a one-block key pass with TMA tiles");
+    static_assert(!XSPEC || SEED, "only a seed pass stores real spectra");
     constexpr int BOXR = L < 256 ? L : 256;       // rows per box
     using P = Plan<LOGL>;
     using Lin = MapLinear<NT>;
@@ -332,7 +334,9 @@ __device__ __forceinline__ void pass_b_tiles(const CUtensorMap* mapY, const floa
     auto unit_block = [&](int u) { return GRP ? (uint32_t)(u >> tshift) : 0u; };
     const int t = threadIdx.x;
     const int pp = t / LR, jj = t % LR;
-    const float sc = 1.0f / (float)(16ull << g.log_np);  // seed spectrum scale: X/(2Np) from 2 (-2 X), for a key at -2 X
+    // Spectrum scale, for transforms of samples at -2 x (pass A): X form 2 (-2 X) sc = -X / (4 Np), (E, A) form
+    // E sc and A sc with 1 / (4 N) = 1 / (2 Np).
+    const float sc = XSPEC ? 1.0f / (float)(16ull << g.log_np) : 1.0f / (float)(2ull << g.log_np);
     {
         float2 w[4];
         if (P::NSTAGE == 2) {
@@ -562,27 +566,38 @@ __device__ __forceinline__ void pass_b_tiles(const CUtensorMap* mapY, const floa
                         }
                         if (u == 0) {  // DC (dropped) and Nyquist in slot (0, 0); then the self pair N/2
                             float2 z = sm[padk<4>(0)];
-                            float nyq = 2.0f * (z.x - z.y);
+                            const float nyq = XSPEC ? 2.0f * (z.x - z.y) : z.x - z.y;
                             if (sd) {
-                                tspec[spec_index<LR>(0, 0)] = make_float2(nyq * sc, 0.f);
+                                tspec[spec_index<LR>(0, 0)] = make_float2(XSPEC ? nyq * sc : 0.5f * nyq * sc, 0.f);
                             } else {
                                 float pn = nyq * tspec[spec_index<LR>(0, 0)].x;
                                 sm[padk<4>(0)] = make_float2(pn, -pn);
                             }
                             ka = kb = L / 2;
                             k = n2 * (uint32_t)(L / 2);
+                            if (!XSPEC) {  // w^2 = -1, V = 0: Y = Z Zs, in the pair's one slot
+                                float2* self = &sm[padk<4>(L / 2)];
+                                float2* slot = &tspec[spec_index<LR>(0, L / 2)];
+                                if (sd) *slot = cscale(*self, sc);
+                                else *self = cmul(*self, *slot);
+                                continue;
+                            }
                         }
-                        float2 w = expmi_pi(k, g.log_n);
-                        float2 za = sm[ca * SP + padk<4>(ka)], zb = sm[cb * SP + padk<4>(kb)];
-                        float2 xa, xb;
-                        real_split(za, zb, w, xa, xb);
+                        float2 za = sm[ca * SP + padk<4>(ka)], zb = sm[ca * SP + padk<4>(kb)];
                         int ia = spec_index<LR>(ca, ka), ib = spec_index<LR>(cb, kb);
                         if (sd) {
-                            tspec[ia] = cscale(xa, sc);
-                            tspec[ib] = cscale(xb, sc);
+                            if (XSPEC) {
+                                float2 xa, xb;
+                                real_split(za, zb, expmi_pi(k, g.log_n), xa, xb);
+                                tspec[ia] = cscale(xa, sc);
+                                tspec[ib] = cscale(xb, sc);
+                            } else {
+                                spectrum_pair(za, zb, sc, tspec[ia], tspec[ib]);
+                            }
                         } else {
                             float2 qa, qb;
-                            real_merge(cmul(xa, tspec[ia]), cmul(xb, tspec[ib]), w, qa, qb);
+                            const float2 fb = tspec[ib];
+                            product_pair(za, zb, tspec[ia], fb, cmul(fb, expmi_pi(2u * k, g.log_n)), qa, qb);
                             sm[ca * SP + padk<4>(ka)] = qa;
                             sm[cb * SP + padk<4>(kb)] = qb;
                         }
@@ -601,48 +616,60 @@ __device__ __forceinline__ void pass_b_tiles(const CUtensorMap* mapY, const floa
                 }
             }
             if (!special || pp != 0) {
-                // bins (k1 = jj + LR r, k2 = p) and (L-1-k1, N2-p): x[r] and x[16 + 15 - r];
-                // W_2N^{p + N2 (jj + LR r)} = W_2N^{p + N2 jj} * W_32^r
+                // bins (k1 = jj + LR r, k2 = p) and (L-1-k1, N2-p): x[r] and x[16 + 15 - r]
                 const uint32_t p = (uint32_t)tile * (CPT / 2) + (uint32_t)pp;
-                const float2 base = expmi_pi(p + n2 * (uint32_t)jj, g.log_n);
                 const float2* sbase = spec_smem ? sm : tspec;  // key pass: the copy in shared memory
                 const float2* sa = sbase + (2 * pp) * 16 * LR + jj;
                 const float2* sb = sbase + (2 * pp + 1) * 16 * LR + jj;
                 float2* da = tspec + (2 * pp) * 16 * LR + jj;
                 float2* db = tspec + (2 * pp + 1) * 16 * LR + jj;
-                if (sd) {
+                if (XSPEC) {
+                    // W_2N^{p + N2 (jj + LR r)} = W_2N^{p + N2 jj} * W_32^r
+                    const float2 base = expmi_pi(p + n2 * (uint32_t)jj, g.log_n);
 #pragma unroll
                     for (int r = 0; r < 16; ++r) {
-                        // W_32^r = e^{-i pi r/16} = (cos, -sin)(2 pi r/32), r < 16
                         const float2 w = r ? cmul(base, make_float2(w32(r).x, -w32(r).y)) : base;
                         float2 xa, xb;
                         real_split(x[r], x[16 + 15 - r], w, xa, xb);
+                        __stcs(da + r * LR, cscale(xa, sc));
+                        __stcs(db + (15 - r) * LR, cscale(xb, sc));
+                    }
+                } else if (sd) {
+#pragma unroll
+                    for (int r = 0; r < 16; ++r) {
+                        float2 ea, eb;
+                        spectrum_pair(x[r], x[16 + 15 - r], sc, ea, eb);
                         if (FUSED) {  // parked for this CTA's key pass: keep it in L2
-                            da[r * LR] = cscale(xa, sc);
-                            db[(15 - r) * LR] = cscale(xb, sc);
+                            da[r * LR] = ea;
+                            db[(15 - r) * LR] = eb;
                         } else {
-                            __stcs(da + r * LR, cscale(xa, sc));
-                            __stcs(db + (15 - r) * LR, cscale(xb, sc));
+                            __stcs(da + r * LR, ea);
+                            __stcs(db + (15 - r) * LR, eb);
                         }
                     }
                 } else {
+                    // W_N^{p + N2 (jj + LR r)} = W_N^{p + N2 jj} * W_16^r, and W_16^(r + 8) = -W_16^r
+                    const float2 base = expmi_pi(2u * (p + n2 * (uint32_t)jj), g.log_n);
 #pragma unroll
-                    for (int r = 0; r < 16; ++r) {
-                        const float2 w = r ? cmul(base, make_float2(w32(r).x, -w32(r).y)) : base;
-                        float2 xa, xb;
-                        real_split(x[r], x[16 + 15 - r], w, xa, xb);
-                        float2 qa, qb;
-                        float2 fa, fb;
-                        if (spec_smem) {
-                            fa = sa[r * LR];
-                            fb = sb[(15 - r) * LR];
-                        } else {
-                            fa = __ldcs(sa + r * LR);
-                            fb = __ldcs(sb + (15 - r) * LR);
+                    for (int r = 0; r < 8; ++r) {
+                        const float2 w = r ? cmul(base, make_float2(w32(2 * r).x, -w32(2 * r).y)) : base;
+#pragma unroll
+                        for (int hi = 0; hi < 2; ++hi) {
+                            const int i = r + 8 * hi;
+                            float2 fa, fb;
+                            if (spec_smem) {
+                                fa = sa[i * LR];
+                                fb = sb[(15 - i) * LR];
+                            } else {
+                                fa = __ldcs(sa + i * LR);
+                                fb = __ldcs(sb + (15 - i) * LR);
+                            }
+                            const float2 t = cmul(fb, hi ? make_float2(-w.x, -w.y) : w);
+                            float2 qa, qb;
+                            product_pair(x[i], x[16 + 15 - i], fa, fb, t, qa, qb);
+                            x[i] = qa;
+                            x[16 + 15 - i] = qb;
                         }
-                        real_merge(cmul(xa, fa), cmul(xb, fb), w, qa, qb);
-                        x[r] = qa;
-                        x[16 + 15 - r] = qb;
                     }
                 }
             }
