@@ -481,6 +481,16 @@ int pa_set_seed_device(pa_engine* e, const uint32_t* d_seed_words, uint32_t n, i
     return seed_common(e, n, reuse_seed_amount, s);
 }
 
+// Device address of pinned (or registered) host memory that kernels can read in 32-bit words, else null.
+static const uint32_t* pinned_view(const uint32_t* p) {
+    cudaPointerAttributes at{};
+    if ((reinterpret_cast<uintptr_t>(p) & 3u) || cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return at.type == cudaMemoryTypeHost ? static_cast<const uint32_t*>(at.devicePointer) : nullptr;
+}
+
 int pa_process(pa_engine* e, const uint32_t* key_start, const uint32_t* key_rest, uint32_t n, uint32_t v,
                uint32_t flags, uint8_t* out, pa_stats* stats) {
     if (!e || !key_start || !out) return PA_ERR_INVALID_ARG;
@@ -492,13 +502,24 @@ int pa_process(pa_engine* e, const uint32_t* key_start, const uint32_t* key_rest
     if (n != e->seed_n) return PA_ERR_INVALID_ARG;
     PA_CUDA(e, cudaSetDevice(e->device));
     cudaStream_t s = e->stream;
-    PA_CUDA(e, cudaMemcpyAsync(e->d_key_start, key_start, (size_t)(g.h / 32u + 1u) * 4u, cudaMemcpyHostToDevice, s));
-    // key_rest is first read by the block's last kernel: a long one is copied on the side stream (after
-    // whatever the engine stream had queued) while the passes run; a short one costs less than the events
+    // Pinned inputs of up to 256 KB are read where they lie: a copy of any size holds the stream for 11 us (2^16 bits
+    // host to host 40 -> 29.5 us a call; longer keys come faster by a copy).  key_rest is first read by the block's last
+    // kernel: a long one is copied on the side stream (after whatever the engine stream had queued) while the passes run.
+    const size_t ks_bytes = (size_t)(g.h / 32u + 1u) * 4u;
+    const uint32_t* d_ks = ks_bytes <= pa_engine::kStageBytes ? pinned_view(key_start) : nullptr;
+    if (!d_ks) {
+        PA_CUDA(e, cudaMemcpyAsync(e->d_key_start, key_start, ks_bytes, cudaMemcpyHostToDevice, s));
+        d_ks = e->d_key_start;
+    }
     cudaEvent_t kr_ready = nullptr;
+    const uint32_t* d_kr = e->d_key_rest;
     const size_t kr_bytes = (size_t)(v / 32u) * 4u;
     if ((flags & PA_FLAG_XOR_KEY_REST) && kr_bytes <= pa_engine::kStageBytes) {
-        PA_CUDA(e, cudaMemcpyAsync(e->d_key_rest, key_rest, kr_bytes, cudaMemcpyHostToDevice, s));
+        d_kr = pinned_view(key_rest);
+        if (!d_kr) {
+            PA_CUDA(e, cudaMemcpyAsync(e->d_key_rest, key_rest, kr_bytes, cudaMemcpyHostToDevice, s));
+            d_kr = e->d_key_rest;
+        }
     } else if (flags & PA_FLAG_XOR_KEY_REST) {
         PA_CUDA(e, cudaEventRecord(e->main_ready, s));
         PA_CUDA(e, cudaStreamWaitEvent(e->side, e->main_ready, 0));
@@ -506,19 +527,20 @@ int pa_process(pa_engine* e, const uint32_t* key_start, const uint32_t* key_rest
         PA_CUDA(e, cudaEventRecord(e->kr_ready, e->side));
         kr_ready = e->kr_ready;
     }
-    rc = block_common(e, e->d_key_start, e->d_key_rest, g, flags, e->d_out, s, kr_ready);
-    if (rc) {
-        cudaStreamSynchronize(kr_ready ? e->side : s);  // the caller's key_rest is not read after we return
-        return rc;
-    }
-    // The words, and a short result, come back behind the kernels and are waited for once; the caller's buffer is
-    // written when the words say that the result holds (a 2^16-bit call: 111 -> 88 us; it was a wait, three copies of
-    // a word and one of the result, each a round trip).
+    // A short result goes to pinned staging, and the block's words follow it by a kernel; both are waited for once, and
+    // the caller's buffer is written when the words say that the result holds.
     const size_t ob = pa_output_bytes(n, v, flags);
     const bool staged = ob <= pa_engine::kStageBytes;
+    uint32_t* const d_out = staged ? reinterpret_cast<uint32_t*>(e->h_stage) : e->d_out;
+    rc = block_common(e, d_ks, d_kr, g, flags, d_out, s, kr_ready);
+    if (rc) {
+        if (kr_ready) cudaStreamSynchronize(e->side);
+        cudaStreamSynchronize(s);  // the caller's buffers are not read after we return
+        return rc;
+    }
     auto collect = [&](pa_stats* st, float* resid) -> int {
-        PA_CUDA(e, cudaMemcpyAsync(e->h_words, e->d_words, sizeof(pa_engine::Words), cudaMemcpyDeviceToHost, s));
-        if (staged) PA_CUDA(e, cudaMemcpyAsync(e->h_stage, e->d_out, ob, cudaMemcpyDeviceToHost, s));
+        int prc = pa::launch_publish(e->d_words, e->h_words, sizeof(pa_engine::Words), s);
+        if (prc) return cuda_fail(e, (cudaError_t)prc);
         PA_CUDA(e, cudaStreamSynchronize(s));
         return take_stats(e, st, resid);
     };
@@ -528,7 +550,7 @@ int pa_process(pa_engine* e, const uint32_t* key_start, const uint32_t* key_rest
     if (!(resid <= e->residual_limit)) {
         // FP32 rounding budget exceeded: recompute this block exactly (same inputs, same seed use)
         if (e->seed_left >= 0) ++e->seed_left;
-        rc = block_common(e, e->d_key_start, e->d_key_rest, g, flags | PA_FLAG_EXACT, e->d_out, s);
+        rc = block_common(e, d_ks, d_kr, g, flags | PA_FLAG_EXACT, d_out, s);
         if (rc) return rc;
         float r2 = 0.f;
         rc = collect(stats, &r2);

@@ -84,60 +84,83 @@ __device__ __forceinline__ void transpose16(uint32_t (&w)[16]) {
 
 // Planes of the key sequence K (16 planes) or, SEED, of the windows T[16 e .. 16 e + 31] (32 planes): plane
 // p's word s at V[p * pw + s] holds the elements 32 s .. 32 s + 31.
+// The words of a CTA's 128 slices pass through shared memory, 17 words per slice, so that they are read in order.
+constexpr int kSlices = 128;  // per CTA, one per thread
 template <bool SEED>
-__global__ void __launch_bounds__(128) k_exact_planes(const uint32_t* __restrict__ src, BlockGeom g, uint32_t pw,
-                                                      uint32_t* __restrict__ V, unsigned long long* clock) {
-    const uint32_t s = blockIdx.x * 128u + threadIdx.x;
-    if (s >= pw) return;
+__global__ void __launch_bounds__(kSlices) k_exact_planes(const uint32_t* __restrict__ src, BlockGeom g, uint32_t pw,
+                                                          uint32_t* __restrict__ V, unsigned long long* clock) {
+    __shared__ uint32_t sm[(kSlices + 1) * 17];
     pdl_wait();
+    const uint32_t s = blockIdx.x * kSlices + threadIdx.x;
     if (clock && s == 0) clock_start(clock);
     const uint32_t H = g.h / 32u, nw = g.n / 32u;
     const uint64_t tbits = (uint64_t)g.h + g.out_bits;
-    auto word = [&](uint64_t q) -> uint32_t {
+    // word first + i of the sequence: of T, or for the key word H - q of key_start, whose top bit and the next one's
+    // other bits are word q of K
+    const uint64_t first = 16ull * kSlices * blockIdx.x;
+    auto fetch = [&](uint32_t i) -> uint32_t {
+        const uint64_t q = first + i;
         if (SEED) {
-            if (32ull * q >= tbits) return 0u;
-            const uint32_t i = q < H ? (uint32_t)q + nw - H : (uint32_t)q - H;  // (32 q - h) mod n, in words
-            const uint32_t v = __brev(load(src + i));
-            const uint64_t left = tbits - 32ull * q;
-            return left >= 32u ? v : v & ((1u << left) - 1u);
+            const bool in = 32ull * q < tbits;
+            const uint32_t at = q < H ? (uint32_t)q + nw - H : (uint32_t)q - H;  // (32 q - h) mod n, in words
+            return in ? load(src + at) : 0u;
         }
-        if (q > H) return 0u;
-        return (load(src + (H - q)) >> 31) | (q < H ? load(src + (H - q - 1u)) << 1 : 0u);
+        return q <= H ? load(src + (H - q)) : 0u;
     };
-    uint32_t w[17], a[16];
+    uint32_t a[16];
 #pragma unroll
-    for (int k = 0; k < (SEED ? 17 : 16); ++k) w[k] = word(16ull * s + k);
+    for (int k = 0; k < 16; ++k) a[k] = fetch(k * kSlices + threadIdx.x);
+    uint32_t past = 0;  // the last slice's windows end in the word after the CTA's
+    if (threadIdx.x == 0) past = fetch(16u * kSlices);
+    auto put = [&](uint32_t i, uint32_t v) {
+        if (SEED) {
+            v = __brev(v);
+            const uint64_t bit = 32ull * (first + i);
+            if (bit < tbits && tbits - bit < 32u) v &= (1u << (tbits - bit)) - 1u;
+        }
+        sm[(i >> 4) * 17 + (i & 15)] = v;
+    };
 #pragma unroll
-    for (int k = 0; k < 16; ++k) a[k] = w[k];
+    for (int k = 0; k < 16; ++k) put(k * kSlices + threadIdx.x, a[k]);
+    if (threadIdx.x == 0) put(16u * kSlices, past);
+    __syncthreads();
+    const uint32_t* w = sm + threadIdx.x * 17;  // w[17] is the next slice's first word
+#pragma unroll
+    for (int k = 0; k < 16; ++k)
+        a[k] = SEED ? w[k] : (w[k] >> 31) | ((k < 15 ? w[k + 1] : w[17]) << 1);
     transpose16(a);
 #pragma unroll
     for (int p = 0; p < 16; ++p) V[(size_t)p * pw + s] = spread2(a[p]);
     if (SEED) {
 #pragma unroll
-        for (int k = 0; k < 16; ++k) a[k] = __funnelshift_r(w[k], w[k + 1], 16);
+        for (int k = 0; k < 16; ++k) a[k] = __funnelshift_r(w[k], k < 15 ? w[k + 1] : w[17], 16);
         transpose16(a);
 #pragma unroll
         for (int p = 0; p < 16; ++p) V[(size_t)(16 + p) * pw + s] = spread2(a[p]);
     }
 }
 
-// Planes of the result -> output words, XOR key_rest, reference byte order.
-__global__ void __launch_bounds__(128) k_exact_words(const uint32_t* __restrict__ V, BlockGeom g, uint32_t pw,
-                                                     const uint32_t* __restrict__ key_rest, uint32_t flags,
-                                                     uint32_t* __restrict__ out, uint32_t nwords,
-                                                     unsigned long long* clock) {
-    const uint32_t s = blockIdx.x * 128u + threadIdx.x;
-    if (s >= pw || 16u * s >= nwords) return;
+// Planes of the result -> output words, XOR key_rest, reference byte order; written in order, as above.
+__global__ void __launch_bounds__(kSlices) k_exact_words(const uint32_t* __restrict__ V, BlockGeom g, uint32_t pw,
+                                                         const uint32_t* __restrict__ key_rest, uint32_t flags,
+                                                         uint32_t* __restrict__ out, uint32_t nwords,
+                                                         unsigned long long* clock) {
+    __shared__ uint32_t sm[kSlices * 17];
     pdl_wait();
+    const uint32_t s = blockIdx.x * kSlices + threadIdx.x;
     uint32_t a[16];
 #pragma unroll
     for (int p = 0; p < 16; ++p) a[p] = gather2(load(V + (size_t)p * pw + s));
     transpose16(a);
 #pragma unroll
+    for (int k = 0; k < 16; ++k) sm[threadIdx.x * 17 + k] = a[k];
+    __syncthreads();
+    const uint32_t first = 16u * kSlices * blockIdx.x;
+#pragma unroll
     for (int k = 0; k < 16; ++k) {
-        const uint32_t q = 16u * s + k;
+        const uint32_t i = k * kSlices + threadIdx.x, q = first + i;
         if (q >= nwords) break;
-        uint32_t w = a[k];
+        uint32_t w = sm[(i >> 4) * 17 + (i & 15)];
         const uint32_t left = g.out_bits - 32u * q;
         if (left < 32u) w &= (1u << left) - 1u;
         w = __brev(w);
@@ -1052,7 +1075,7 @@ int launch_exact_seed(const BlockGeom& g, const uint32_t* seed, uint32_t* seed_h
     const Shape sh = shape_of(g);
     Chain ch{s};
     const size_t P = size_t(32) * sh.pw;
-    ch.run(k_exact_planes<true>, (sh.pw + 127u) / 128u, 128, 0, seed, g, sh.pw, tmp, clock);
+    ch.run(k_exact_planes<true>, sh.pw / kSlices, kSlices, 0, seed, g, sh.pw, tmp, clock);
     const uint32_t* V = convert_basis<kIT>(sh, tmp, tmp + P, 32, ch);
     ch.run(k_exact_to_field<true>, sh.pw / kConvThreads, kConvThreads, 0, V, sh.pw, seed_hat);
     top_levels<kIT>(sh, seed_hat, ch);
@@ -1074,7 +1097,7 @@ int launch_exact_block(const BlockGeom& g, const uint32_t* seed, const uint32_t*
     const Shape sh = shape_of(g);
     Chain ch{s};
     const size_t half = size_t(16) * sh.pw;
-    ch.run(k_exact_planes<false>, (sh.pw + 127u) / 128u, 128, 0, key_start, g, sh.pw, tmp, start);
+    ch.run(k_exact_planes<false>, sh.pw / kSlices, kSlices, 0, key_start, g, sh.pw, tmp, start);
     const uint32_t* V = convert_basis<kF>(sh, tmp, tmp + half, 16, ch);
     ch.run(k_exact_to_field<false>, sh.pw / kConvThreads, kConvThreads, 0, V, sh.pw, a);
     top_levels<kF>(sh, a, ch);
@@ -1083,7 +1106,7 @@ int launch_exact_block(const BlockGeom& g, const uint32_t* seed, const uint32_t*
     ch.run(k_exact_to_traces, sh.pw / kConvThreads, kConvThreads, 0, a, sh.pw, tmp);
     V = convert_basis<kT>(sh, tmp, tmp + half, 16, ch);
     const uint32_t nwords = (g.out_bits + 31u) / 32u;
-    ch.run(k_exact_words, ((nwords + 15u) / 16u + 127u) / 128u, 128, 0, V, g, sh.pw, key_rest, flags, out_words,
+    ch.run(k_exact_words, ((nwords + 15u) / 16u + kSlices - 1u) / kSlices, kSlices, 0, V, g, sh.pw, key_rest, flags, out_words,
            nwords, end);
     return (int)ch.err;
 }

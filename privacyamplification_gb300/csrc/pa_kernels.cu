@@ -355,6 +355,19 @@ int launch_group_mono_key(const BlockGeom& g, const Group& gp, uint32_t flags, c
 #undef C
 }
 
+// One CTA copies `words` 32-bit words to pinned host memory behind a block's last kernel: a copy-engine transfer of any
+// small size holds the stream for 11 us, this launch for about 2.
+__global__ void __launch_bounds__(64) k_publish(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst, int words) {
+    pdl_wait();
+    if ((int)threadIdx.x < words) dst[threadIdx.x] = load(src + threadIdx.x);
+}
+
+int launch_publish(const void* src, void* dst, size_t bytes, cudaStream_t s) {
+    if (bytes > 64 * sizeof(uint32_t) || bytes % sizeof(uint32_t)) return (int)cudaErrorInvalidValue;
+    return (int)launch_pdl(k_publish, 1, 64, 0, s, static_cast<const uint32_t*>(src), static_cast<uint32_t*>(dst),
+                           (int)(bytes / sizeof(uint32_t)));
+}
+
 int kernel_count_key_block(const BlockGeom& g) { return g.log_n1 == 0 || short_geom(g) ? 1 : 5; }
 int stage_count_key_block(const BlockGeom& g) { return g.log_n1 == 0 || short_geom(g) ? 1 : 4; }
 

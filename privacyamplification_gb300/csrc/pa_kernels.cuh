@@ -87,6 +87,8 @@ int launch_fused_block(const BlockGeom& g, const uint32_t* seed, const uint32_t*
                        const Scratch& sc, unsigned long long* cnt, unsigned int* resid_bits, uint32_t* out_words,
                        int num_sms, cudaStream_t s, cudaEvent_t* stage_ev, cudaEvent_t key_rest_ready = nullptr,
                        unsigned long long* clock = nullptr);
+// Copies up to 256 bytes (a multiple of 4) from device to pinned host memory by a kernel.
+int launch_publish(const void* src, void* dst, size_t bytes, cudaStream_t s);
 int kernel_count_key_block(const BlockGeom& g);   // kernels one key block launches
 int stage_count_key_block(const BlockGeom& g);    // timed stages (events - 1) of a key block
 
