@@ -285,21 +285,27 @@ __device__ __forceinline__ void smem_round(uint32_t* x) {
         }
         __syncthreads();
     };
-    auto shift = [&] {
-        for (int i = threadIdx.x; i < 1024; i += kBcThreads) {
-            uint32_t *lo = x + (i / RW) * 2 * RW, *hi = lo + RW;
+    auto shift = [&] {  // the loads of a thread's four pairs before the first store
+        constexpr int Q = 1024 / kBcThreads;
+        uint32_t v[Q];
+#pragma unroll
+        for (int k = 0; k < Q; ++k) {
+            const int i = k * kBcThreads + (int)threadIdx.x;
+            const uint32_t *lo = x + (i / RW) * 2 * RW, *hi = lo + RW;
             const int j = i % RW;
             if constexpr (OP == kF) {
-                if constexpr (DW > 0) {
-                    if (j >= DW) lo[j] ^= hi[j - DW];
-                } else {
-                    lo[j] ^= (hi[j] << S) | (j ? hi[j - 1] >> (32 - S) : 0u);
-                }
+                if constexpr (DW > 0) v[k] = lo[j] ^ (j >= DW ? hi[j - DW] : 0u);
+                else v[k] = lo[j] ^ ((hi[j] << S) | (j ? hi[j - 1] >> (32 - S) : 0u));
             } else if constexpr (DW > 0) {
-                if (j + DW < RW) hi[j] ^= lo[j + DW];
+                v[k] = hi[j] ^ (j + DW < RW ? lo[j + DW] : 0u);
             } else {
-                hi[j] ^= (lo[j] >> S) | (j + 1 < RW ? lo[j + 1] << (32 - S) : 0u);
+                v[k] = hi[j] ^ ((lo[j] >> S) | (j + 1 < RW ? lo[j + 1] << (32 - S) : 0u));
             }
+        }
+#pragma unroll
+        for (int k = 0; k < Q; ++k) {
+            const int i = k * kBcThreads + (int)threadIdx.x;
+            x[(i / RW) * 2 * RW + i % RW + (OP == kF ? 0 : RW)] = v[k];
         }
         __syncthreads();
     };
@@ -510,9 +516,20 @@ __global__ void __launch_bounds__(kUpThreads) k_exact_upper(const uint32_t* __re
     // edge tile: kF columns 2048 - H .. 2047 and H words past the end; otherwise columns 0 .. 2 H.
     uint32_t* xa = xu;
     uint32_t* xe = xu + R * kUpRow;
-    for (int i = t; i < R * kUpRow; i += kUpThreads) {
-        const int col = w0 + (i & (kUpRow - 1)) - (OP == kF ? H : 0);
-        xa[i] = col >= 0 && col < 2048 ? load(in + (size_t)(i / kUpRow) * 2048u + col) : 0u;
+    {  // a thread's words are one column of every fourth row: four loads before the first store
+        const int col = w0 + (t & (kUpRow - 1)) - (OP == kF ? H : 0);
+        const bool inside = col >= 0 && col < 2048;
+        for (int i0 = t; i0 < R * kUpRow; i0 += 4 * kUpThreads) {
+            uint32_t v[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int i = i0 + k * kUpThreads;
+                v[k] = inside && i < R * kUpRow ? load(in + (size_t)(i / kUpRow) * 2048u + col) : 0u;
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (i0 + k * kUpThreads < R * kUpRow) xa[i0 + k * kUpThreads] = v[k];
+        }
     }
     if (edge)
         for (int i = t; i < R * kUpEdge; i += kUpThreads) {
@@ -739,16 +756,31 @@ __device__ __forceinline__ void store_words(uint32_t* p, const uint32_t (&v)[N])
         reinterpret_cast<uint4*>(p)[k] = make_uint4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
 }
 
+// Masks of t's low K bits: b[m] all ones where bit m is set.  PRMT spreads the top bit of a byte over a word, so eight
+// shifts of t serve every byte (two shifts a mask otherwise).
+template <int K>
+__device__ __forceinline__ void bit_masks(uint32_t t, uint32_t (&b)[K]) {
+#pragma unroll
+    for (int s = 0; s < 8 && s < K; ++s) {
+        const int low = K < 8 ? K - 1 - s : 7 - s;  // the bit of a byte that is brought to its top
+        const uint32_t v = t << (7 - low);
+#pragma unroll
+        for (int k = 0; 8 * k + low < K; ++k)
+            asm("prmt.b32 %0, %1, 0, %2;" : "=r"(b[8 * k + low]) : "r"(v), "r"(0x8888u | 0x1111u * (uint32_t)k));
+    }
+}
+
 // One butterfly on N words of x and y (shared memory) by a twiddle of GF(2^K), K <= N: its words are the masks
 // of t's low K bits, XOR pat (the lane-dependent part) where PAT.
 template <int K, int N, Op OP, bool PAT>
 __device__ __forceinline__ void butterfly(uint32_t* px, uint32_t* py, uint32_t t, const uint32_t* pat) {
     uint32_t b[K], a[N], p[N];
-    if (PAT) load_words<K>(pat, b);
+    bit_masks<K>(t, b);
+    if constexpr (PAT) {
+        uint32_t lanes[K];
+        load_words<K>(pat, lanes);
 #pragma unroll
-    for (int m = 0; m < K; ++m) {
-        const uint32_t s = (uint32_t)((int32_t)(t << (31 - m)) >> 31);
-        b[m] = PAT ? b[m] ^ s : s;
+        for (int m = 0; m < K; ++m) b[m] ^= lanes[m];
     }
     load_words<N>(OP == kF ? py : px, a);
     if (OP == kT) {  // x += y first: the product's argument
@@ -801,9 +833,19 @@ __global__ void __launch_bounds__(512) k_exact_top(uint32_t* __restrict__ W, int
     const uint32_t cols = 1u << (lo - 5);
     uint32_t* base = W + ((size_t)blockIdx.y * rows * cols + col) * 32u + 16u * half;
     pdl_wait();
-    for (uint32_t i = threadIdx.x; i < rows * 4u; i += blockDim.x)
-        *reinterpret_cast<uint4*>(xt + (i >> 2) * kTopRow + 4u * (i & 3u)) =
-            *reinterpret_cast<const uint4*>(base + (size_t)(i >> 2) * cols * 32u + 4u * (i & 3u));
+    {  // up to eight loads per thread (blockDim.x = rows / 2), all before the first store
+        uint4 v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const uint32_t i = k * blockDim.x + threadIdx.x;
+            if (i < rows * 4u) v[k] = load(reinterpret_cast<const uint4*>(base + (size_t)(i >> 2) * cols * 32u + 4u * (i & 3u)));
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const uint32_t i = k * blockDim.x + threadIdx.x;
+            if (i < rows * 4u) *reinterpret_cast<uint4*>(xt + (i >> 2) * kTopRow + 4u * (i & 3u)) = v[k];
+        }
+    }
     __syncthreads();
     for (int k = 0; k < T; ++k) {
         const int q = OP == kT ? k : T - 1 - k;  // row bit
@@ -874,13 +916,15 @@ __global__ void __launch_bounds__(1 << (LOWB - 5), LOWB >= 13 ? 2 : 1)
         // index bits above i that the slice number gives, from bit i + 1 on
         const uint32_t e = transposed ? ((s >> 5) << (9 - i)) | ((s & 31u) >> (i + 1)) : (s >> q) >> 1;
         const uint32_t tw = tt.at(e) ^ tc[i];
-        const uint32_t* pp = pat[transposed ? i : 5];
+        const uint32_t* pp = pat[transposed ? i : 5];  // only long transforms multiply in full before the transposes
         uint32_t* px = xl + s * kRow;
         uint32_t* py = px + (kRow << q);
         if (full) {
             if (half == 0) butterfly<32, 32, OP, true>(px, py, tw, pp);
-        } else {
+        } else if (transposed) {
             butterfly<16, 16, OP, true>(px + 16 * half, py + 16 * half, tw, pp);
+        } else {
+            butterfly<16, 16, OP, false>(px + 16 * half, py + 16 * half, tw, nullptr);
         }
         __syncthreads();
     };
@@ -963,7 +1007,7 @@ Shape shape_of(const BlockGeom& g) {
     const uint64_t need = (uint64_t)g.h + g.out_bits;
     s.l = 16;
     while ((16ull << s.l) < need) ++s.l;
-    s.lowb = s.l <= 18 ? 11 : (s.l <= 20 ? 12 : 13);
+    s.lowb = s.l <= 18 ? 11 : (s.l == 19 ? 12 : 13);
     const int top = s.l - s.lowb;
     s.passes = top > 10 ? 2 : 1;
     s.T[0] = s.passes == 2 ? (top + 1) / 2 : top;  // the upper pass first
