@@ -8,10 +8,10 @@
 // The chunks of a row are summed as spectra: every seed window and every key column is transformed forward once, a
 // row's product spectrum is sum_b K_b S_(a-b), and one inverse transform per row gives the integer sums, which are
 // rounded and packed straight into the result.  n = 2^29 (v = 3n/8): 7 + 5 forward and 3 inverse transforms, where
-// chunk by chunk took 7 + 15 forward and 15 inverse ones: 16.7 -> 8.2 ms a
-// block with its own seed (4.9 ms with a kept one, whose window spectra stay); n = 2^30 60 -> 18.5 ms.  The sums are
-// larger than one chunk's, so the largest residual grows with the root of the columns: 0.021 -> 0.053 at n = 2^29,
-// 0.074 at the most (n = 2^30, sixteen columns), against the limit of 0.25.
+// chunk by chunk took 7 + 15 forward and 15 inverse ones: 16.7 -> 8.2 ms a block with its own seed (4.9 ms with a kept
+// one, whose window spectra stay); n = 2^30 60 -> 18.5 ms.  The sums are larger than one chunk's, so the largest
+// residual grows with the root of the columns: 0.021 -> 0.053 at n = 2^29, 0.074 at the most (n = 2^30, sixteen
+// columns), against the limit of 0.25.
 //
 // Forward transforms are the row pass and the seed form of the column pass (spectra scaled by 1 / (16 Np), a power
 // of two, taken back in the sum); the sum reads every spectrum once for three rows (15 x 512 MB at n = 2^29,

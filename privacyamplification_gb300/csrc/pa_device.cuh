@@ -236,8 +236,8 @@ __device__ __forceinline__ void real_merge(float2 pa, float2 pb, float2 w, float
 //   Y[k] = Z[k] U + conj(Z[N-k]) V,   U = Es + A - w^2 A,  V = A + w^2 A,  A = i Os / 2,
 // and with the same Es, A for the bin N - k: Y[N-k] = Z[N-k] conj(Es - A + w^2 A) - conj(Z[k] V).  The seed keeps Es and
 // A, which need no twiddle (Es = (Z + conj Z')/2, A = (Z - conj Z')/4), in place of S[k] and S[N-k]: about half the FP32
-// operations of splitting both spectra, multiplying and merging (n = 2^27, kept
-// seed 884 -> 858 us a block, own seed 1355 -> 1325).
+// operations of splitting both spectra, multiplying and merging (n = 2^27: kept seed 884 -> 858 us a block, own seed
+// 1355 -> 1325).
 __device__ __forceinline__ void spectrum_pair(float2 za, float2 zb, float sc, float2& es, float2& a) {
     const float2 zbc = cconj(zb);
     es = cscale(cadd(za, zbc), 0.5f * sc);

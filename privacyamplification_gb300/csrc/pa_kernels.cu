@@ -10,8 +10,8 @@
 //   * three-pass four-step path, N = N1 * N2 (N2 <= 2^14, N1 <= 2^12), kernels in pa_passes.cu:
 //       bit rows  key bits -> per-row bit planes
 //       pass A    row FFTs over m2 (length N2), 4-step twiddle, write Y
-//       pass B    column FFTs over m1 (length N1), real split, spectral product with the cached seed
-//                 spectrum (DC removed), real merge, inverse column FFTs, inverse twiddle, write Y
+//       pass B    column FFTs over m1 (length N1), product of the packed spectrum with the cached seed's
+//                 (DC removed), inverse column FFTs, inverse twiddle, write Y
 //       pass C    inverse row FFTs, + correction, round, parity -> bit planes
 //       finish    bit planes -> reference byte order, XOR key_rest
 #include "pa_device.cuh"

@@ -2,13 +2,13 @@
 // the per-pass kernels (pa_passes.cu: one launch per pass, the grid walks rows or tiles) and the persistent
 // lane kernel (pa_lanes.cu: a few CTAs of one lane walk a block's rows and tiles between lane barriers).
 //
-//
 // Data layout in HBM for one block (n = 2^27: N1 = 2^12, N2 = 2^14):
 //   rows     bit planes, row m1 holds the 2*N2 sample bits x = 2(m1 + N1*m2) + t, 16 m2 per word,
 //            MSB first (n/8 bytes)                                  -- k_bit_rows
 //   Y        N complex64, row m1 = N2 values in "pair" order: float4 p holds columns p and N2-p
 //            (p = 0 holds 0 and N2/2)                               -- pass A writes, pass B rewrites
-//   spec     N complex64, the seed's real spectrum / (2 Np) in the thread order of pass B
+//   spec     N complex64, the seed's packed spectrum (E, A) / (2 Np) in the thread order of pass B, see
+//            spectrum_pair (sums over chunks keep the real spectrum instead)
 //   planes   parity bits, [t][m1][N2/32 words], bit m2 of row m1 -- pass C writes
 //   out      v/8 bytes in the reference byte order                  -- k_finish
 // Each pass is one persistent CTA per SM walking rows (A, C) or column tiles (B); the FFT data stay
@@ -532,7 +532,7 @@ __device__ __forceinline__ void pass_b_tiles(const CUtensorMap* mapY, const floa
                 parity_spec ^= 1u;
             }
 
-            // ---- spectral step: real split, product with the seed spectrum, real merge
+            // ---- spectral step: the seed's (E, A) from its packed spectrum, or the key's product with them
             if (special) {
                 __syncthreads();
                 if (pp == 0) {

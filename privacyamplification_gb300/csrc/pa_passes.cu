@@ -6,7 +6,8 @@
 //            MSB first (n/8 bytes)                                  -- k_bit_rows
 //   Y        N complex64, row m1 = N2 values in "pair" order: float4 p holds columns p and N2-p
 //            (p = 0 holds 0 and N2/2)                               -- pass A writes, pass B rewrites
-//   spec     N complex64, the seed's real spectrum / (2 Np) in the thread order of pass B
+//   spec     N complex64, the seed's packed spectrum (E, A) / (2 Np) in the thread order of pass B, see
+//            spectrum_pair (sums over chunks keep the real spectrum instead)
 //   planes   parity bits, [t][m1][N2/32 words], bit m2 of row m1 -- pass C writes
 //   out      v/8 bytes in the reference byte order                  -- k_finish
 // Each pass is one persistent CTA per SM walking rows (A, C) or column tiles (B); the FFT data stay
