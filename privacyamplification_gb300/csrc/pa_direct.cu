@@ -15,6 +15,8 @@
 
 #include <cooperative_groups.h>
 
+#include <algorithm>
+
 namespace pa {
 
 namespace {
@@ -23,6 +25,7 @@ namespace cg = cooperative_groups;
 
 constexpr int kWarps = 8;
 constexpr uint32_t kOneWords = 1024;
+constexpr uint32_t kCounters = 64;
 
 // ONE: a single CTA takes every result word and writes them when the last is formed, for an output that
 // overlaps the inputs (up to kOneWords words).
@@ -152,11 +155,15 @@ __global__ void __launch_bounds__(32 * kWarps, 4) k_direct(const uint32_t* __res
     if (ONE)
         for (uint32_t q = threadIdx.x; q < nwords; q += 32 * kWarps) out[q] = held[q];
     if (dc.clock && threadIdx.x == 0) clock_end(dc.clock);
-    if (dc.count_seed && blockIdx.x == gridDim.x - 1) {  // the placed seed's popcount, once per seed and placement
+    // The placed seed's popcount, once per seed and placement, by up to kCounters CTAs: the last of them to add its share
+    // to cnt[2] (arrivals above bit 48) takes the sum and leaves zero.  One CTA took 20 us at 2^20 bits, 270 at 2^24.
+    const uint32_t counters = min(gridDim.x, kCounters);
+    if (dc.count_seed && blockIdx.x < counters) {
         const uint32_t words = 1u << (g.log_np - 5);
         uint32_t c = 0;
 #pragma unroll 4
-        for (uint32_t w = threadIdx.x; w < words; w += 32 * kWarps) c += __popc(load(seed + seed_word(g, 32ull * w)));
+        for (uint32_t w = 32 * kWarps * blockIdx.x + threadIdx.x; w < words; w += 32 * kWarps * counters)
+            c += __popc(load(seed + seed_word(g, 32ull * w)));
 #pragma unroll
         for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
         __syncthreads();
@@ -165,7 +172,11 @@ __global__ void __launch_bounds__(32 * kWarps, 4) k_direct(const uint32_t* __res
         if (threadIdx.x == 0) {
             unsigned long long t = 0;
             for (int i = 0; i < kWarps; ++i) t += red[i][0][0];
-            dc.cnt[1] = t;
+            const unsigned long long before = atomicAdd(dc.cnt + 2, t + (1ull << 48));
+            if ((before >> 48) == counters - 1) {
+                dc.cnt[1] = (before & ((1ull << 48) - 1ull)) + t;
+                dc.cnt[2] = 0ull;
+            }
         }
     }
 }
@@ -182,10 +193,16 @@ bool overlap(const void* a, size_t na, const void* b, size_t nb) {
 
 }  // namespace
 
-// The ordinary path's bound is where the FP32 transforms (31 us from 2^17 to 2^19 bits) catch up: 9.1e9 bit products take
-// 22 us, 9.7e9 26, 12.3e9 36, 16.1e9 41.  The exact path's transform takes 50 us from there on.
-bool short_geom(const BlockGeom& g) { return ((uint64_t)g.h + 1u) * g.out_bits <= (5ull << 31); }
-bool direct_geom(const BlockGeom& g) { return ((uint64_t)g.h + 1u) * g.out_bits <= (1ull << 34); }
+// The ordinary path's bounds are where the FP32 transforms (31 us from 2^17 to 2^19 bits) catch up: 9.1e9 bit products
+// take 22 us, 9.7e9 26, 12.3e9 36, 16.1e9 41.  The exact path's transform takes 50 us from there on.  A long key with
+// few results has few clusters and a long result with a short key few warps per CTA: the time then grows with the longer
+// of the two (2^21 bits 23 .. 34 us against 34.5, 2^22 43 .. 62 against 46.5, 2^24 158 .. 172 against 98 .. 119), the
+// exact path's transform being 58, 62 and 93.
+static bool word_by_word(const BlockGeom& g, uint64_t products, uint64_t longest) {
+    return ((uint64_t)g.h + 1u) * g.out_bits <= products && std::max(g.h, g.out_bits) <= longest;
+}
+bool short_geom(const BlockGeom& g) { return word_by_word(g, 5ull << 31, 1ull << 21); }
+bool direct_geom(const BlockGeom& g) { return word_by_word(g, 1ull << 34, 1ull << 22); }
 
 bool direct_overlap(const BlockGeom& g, const uint32_t* key_start, const uint32_t* out_words) {
     return overlap(out_words, 4u * (size_t)((g.out_bits + 31u) / 32u), key_start, 4u * (size_t)(g.h / 32u + 1u));

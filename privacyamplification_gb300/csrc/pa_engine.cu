@@ -201,21 +201,27 @@ cudaEvent_t* stage_events(pa_engine* e, const BlockGeom& g) {
 }
 
 // A short block word by word (pa_direct.cu): exact, so that its residual is zero.  The seed's popcount is formed with
-// the first block of a seed and placement.
+// the first block of a seed and placement, and with every block that is captured, which may be replayed on later seeds.
 int direct_block(pa_engine* e, const uint32_t* d_ks, const uint32_t* d_kr, const BlockGeom& g, uint32_t flags,
                  uint32_t* d_out, cudaStream_t s) {
     if (pa::direct_overlap(g, d_ks, d_out)) {  // every result word reads the whole key
         PA_CUDA(e, cudaMemcpyAsync(e->d_key_start, d_ks, (size_t)(g.h / 32u + 1u) * 4u, cudaMemcpyDeviceToDevice, s));
         d_ks = e->d_key_start;
     }
-    const bool counted = e->count_valid && same_seed_geom(e->count_geom, g);
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    PA_CUDA(e, cudaStreamIsCapturing(s, &capture));
+    const bool captured = capture != cudaStreamCaptureStatusNone;
+    const bool counted = !captured && e->count_valid && same_seed_geom(e->count_geom, g);
     cudaEvent_t* ev = stage_events(e, g);
     if (ev) cudaEventRecord(ev[0], s);
-    int rc = pa::launch_direct(g, e->d_seed, d_ks, d_kr, flags, d_out, s, {e->d_words->short_cnt, e->d_resid, counted ? 0 : 1, e->d_words->clock});
+    int rc = pa::launch_direct(g, e->d_seed, d_ks, d_kr, flags, d_out, s,
+                               {e->d_words->short_cnt, e->d_resid, counted ? 0 : 1, e->d_words->clock});
     if (rc) return cuda_fail(e, (cudaError_t)rc);
     if (ev) cudaEventRecord(ev[1], s);
-    e->count_geom = g;
-    e->count_valid = true;
+    if (!captured) {
+        e->count_geom = g;
+        e->count_valid = true;
+    }
     return PA_OK;
 }
 

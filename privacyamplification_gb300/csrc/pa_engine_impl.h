@@ -63,11 +63,13 @@ struct pa_engine {
     // a block's words, in one allocation (d_words) that one copy brings to the host
     struct Words {
         unsigned long long cnt[2];        // key popcount, seed popcount (pass C reads them beside the spectrum)
-        unsigned long long short_cnt[2];  // the same of a short block, whose seed's count outlives the block
+        unsigned long long short_cnt[3];  // the same of a short block, whose seed's count outlives the block; the
+                                          // third gathers that count and is zero between blocks
         unsigned long long clock[2];      // the block's start and end on the global timer, ns
         unsigned int resid;               // largest residual (float bits)
         int err;                          // bounded device waits that expired
     };
+    static_assert(sizeof(Words) == 64, "the pinned copy's room before the staged results");
     Words* d_words = nullptr;
     unsigned long long* d_cnt = nullptr;  // d_words->cnt
     unsigned int* d_resid = nullptr;      // &d_words->resid

@@ -182,8 +182,8 @@ bool direct_geom(const BlockGeom& g);
 // rate is higher with several blocks in flight).
 bool short_geom(const BlockGeom& g);
 bool direct_overlap(const BlockGeom& g, const uint32_t* key_start, const uint32_t* out_words);
-// cnt (may be null): receives the key's popcount and, with count_seed, the placed seed's in cnt[1]; *resid then
-// becomes zero.
+// cnt (may be null): receives the key's popcount and, with count_seed, the placed seed's in cnt[1], which cnt[2] gathers
+// (zero before and after); *resid then becomes zero.
 struct DirectCounts {
     unsigned long long* cnt;
     unsigned int* resid;

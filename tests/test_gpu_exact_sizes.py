@@ -91,3 +91,22 @@ def test_short_and_transformed_blocks_share_a_seed(gpu_engine):
         out = gpu_engine.process(ks, kr, n, v)
         assert np.array_equal(out, O.ntt(seed, ks, kr, n, v)), v
         assert gpu_engine.last_stats.popcount_key == O.popcount(ks, n - v + 1)
+
+
+@pytest.mark.parametrize("n,v,exact", [(2097152, 32, 0), (2097152, 2097120, 0), (2097216, 32, 0), (2097248, 2097216, 0),
+                                       (1048576, 4096, 0), (4194304, 32, 1), (4194336, 32, 1), (4194368, 4194336, 1)])
+def test_long_keys_and_long_results(gpu_engine, n, v, exact):
+    """Skewed blocks on either side of the word-by-word product's longest key and result (2^21 bits, exact path 2^22):
+    whole output, popcounts of the key and of the seed, which several CTAs count."""
+    seed, recv = O.random_block(n, v, n + 5 * v)
+    ks, kr = O.key_split(recv, n, v)
+    gpu_engine.set_seed(seed, n, 2)
+    for _ in range(2):
+        out = gpu_engine.process(ks, kr, n, v, DEFAULT | (pa.FLAG_EXACT if exact else 0))
+        st = gpu_engine.last_stats
+        assert np.array_equal(out, O.ntt(seed, ks, kr, n, v))
+        assert st.exact == exact
+        if not exact:
+            assert st.popcount_key == O.popcount(ks, n - v + 1)
+            if n & (n - 1) == 0:
+                assert st.popcount_seed == O.popcount(seed, n)
