@@ -110,9 +110,9 @@ PA_API int pa_key_split(const uint32_t* recv_key, uint32_t n, uint32_t v, uint32
 /* Output length in bytes (PrivacyAmplification.cu:1197). */
 PA_API size_t pa_output_bytes(uint32_t n, uint32_t v, uint32_t flags);
 
-/* Number of kernels one pa_process_device launches for (n, v) with a cached seed spectrum (a one-use
- * seed of 2^21 bits and more adds its two row-pass kernels: bit rows and row FFTs); 1 for the short
- * blocks that one kernel computes without a spectrum. */
+/* Number of kernels one pa_process_device launches for (n, v) with a cached seed spectrum (or a
+ * one-use seed of 2^21 bits and more, which shares them); 1 for the short blocks that one kernel computes
+ * without a spectrum. */
 PA_API int pa_kernels_per_block(uint32_t n, uint32_t v, uint32_t flags);
 
 /* Per-kernel timing, the counterpart of the reference's STOPWATCH stage deltas

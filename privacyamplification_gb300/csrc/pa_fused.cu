@@ -1,8 +1,8 @@
 // pa_fused.cu -- a block whose seed serves that block only: one column pass for the seed and the key.
 //
 // A fresh seed's spectrum is otherwise written to HBM by a column pass of its own and read back by the
-// key's (N complex values each way: 1 GiB of traffic at n = 2^27).  Here both row passes run first, the
-// seed's into the buffer its spectrum would take, and one column pass takes every tile twice: the seed's
+// key's (N complex values each way: 1 GiB of traffic at n = 2^27).  Here both row passes run first, in
+// one launch (k_pass_a_both), the seed's into the buffer its spectrum would take, and one column pass takes every tile twice: the seed's
 // tile, transformed and split into its spectrum tile, which is parked in the CTA's own 64 KiB of a small
 // buffer (2 CTAs per SM: about 20 MB, rewritten by the same CTA a tile later, so it stays in L2), then
 // the key's tile against it (pass_b_tiles, FUSED).

@@ -325,10 +325,9 @@ int launch_fused_block(const BlockGeom& g, const uint32_t* seed, const uint32_t*
         if (ev) cudaEventRecord(ev[i], s);
     };
     mark(0);
-    int rc = launch_bit_rows(g, seed, true, sc.planes, s, kOneBlock, cnt + 1, nullptr, clock);
-    if (!rc) rc = launch_pass_a(g, sc.planes, true, seed_y, cnt + 1, num_sms, s);
-    if (!rc) rc = launch_bit_rows(g, key_start, false, sc.planes, s, kOneBlock, cnt, resid_bits);
-    if (!rc) rc = launch_pass_a(g, sc.planes, false, sc.work, cnt, num_sms, s);
+    // the seed's bit rows in work2, which is pass B's to write
+    int rc = launch_rows_both(g, key_start, seed, sc.planes, reinterpret_cast<uint32_t*>(sc.work2), sc.work, seed_y, cnt,
+                              resid_bits, clock, num_sms, s);
     mark(1);
     if (!rc) rc = launch_pass_b_fused(g, seed_maps, *sc.maps, sc.work2, park, park_ctas, sc.err, num_sms, s);
     mark(2);

@@ -132,6 +132,9 @@ int launch_group_mono_key(const BlockGeom& g, const Group& gp, uint32_t flags, c
 int launch_bit_rows(const BlockGeom& g, const uint32_t* bits, bool seed, uint32_t* rows, cudaStream_t s,
                     const Group& gp = kOneBlock, unsigned long long* zero_cnt = nullptr,
                     unsigned int* zero_resid = nullptr, unsigned long long* clock = nullptr);
+int launch_rows_both(const BlockGeom& g, const uint32_t* key, const uint32_t* seed, uint32_t* key_rows,
+                     uint32_t* seed_rows, float2* Y, float2* Ys, unsigned long long* cnt, unsigned int* resid,
+                     unsigned long long* clock, int num_sms, cudaStream_t s);
 int launch_pass_a(const BlockGeom& g, const uint32_t* rows, bool seed, float2* Y, unsigned long long* cnt,
                   int num_sms, cudaStream_t s, const Group& gp = kOneBlock);
 struct PassMaps {

@@ -77,15 +77,8 @@ __global__ void __launch_bounds__(256) k_bit_rows(const uint32_t* __restrict__ s
 // is a 64-byte run instead of one word per row.  Rows padded to 17 words keep the column reads of the
 // transpose on distinct banks.  SEED with a padded Np: each word comes from its placed source word.
 template <bool SEED>
-__global__ void __launch_bounds__(256) k_bit_rows_tiled(const uint32_t* __restrict__ src, BlockGeom g,
-                                                        uint32_t* __restrict__ rows, Zeroed z, Group gp) {
-    __shared__ uint32_t tile[256][17];  // [m2 - m20][a - a0], then [m1 - 16 a0][(m2 - m20) / 16]
-    pdl_wait();
-    z.clear();
-    if (gp.e) {
-        src = SEED ? gp.e[blockIdx.z].seed : gp.e[blockIdx.z].key_start;
-        rows += (size_t)blockIdx.z * gp.planes;
-    }
+__device__ __forceinline__ void bit_rows_tile(const uint32_t* __restrict__ src, const BlockGeom& g,
+                                              uint32_t* __restrict__ rows, uint32_t (*tile)[17]) {
     const int t = threadIdx.x, lane = t & 31;
     const uint32_t win = (1u << g.log_n1) / 16u, wout = (1u << g.log_n2) / 16u;  // words per input / output row
     const uint32_t a0 = blockIdx.x * 16u, m20 = blockIdx.y * 256u;
@@ -129,6 +122,34 @@ __global__ void __launch_bounds__(256) k_bit_rows_tiled(const uint32_t* __restri
     }
 }
 
+template <bool SEED>
+__global__ void __launch_bounds__(256) k_bit_rows_tiled(const uint32_t* __restrict__ src, BlockGeom g,
+                                                        uint32_t* __restrict__ rows, Zeroed z, Group gp) {
+    __shared__ uint32_t tile[256][17];  // [m2 - m20][a - a0], then [m1 - 16 a0][(m2 - m20) / 16]
+    pdl_wait();
+    z.clear();
+    if (gp.e) {
+        src = SEED ? gp.e[blockIdx.z].seed : gp.e[blockIdx.z].key_start;
+        rows += (size_t)blockIdx.z * gp.planes;
+    }
+    bit_rows_tile<SEED>(src, g, rows, tile);
+}
+
+// Key (blockIdx.z = 0) and seed (1) of a block with its own seed.
+__global__ void __launch_bounds__(256)
+    k_bit_rows_both(const uint32_t* __restrict__ key, const uint32_t* __restrict__ seed, BlockGeom g,
+                    uint32_t* __restrict__ key_rows, uint32_t* __restrict__ seed_rows, Zeroed z) {
+    __shared__ uint32_t tile[256][17];
+    pdl_wait();
+    z.clear();
+    if (blockIdx.z == 0) {
+        bit_rows_tile<false>(key, g, key_rows, tile);
+    } else {
+        if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0) z.cnt[1] = 0ull;
+        bit_rows_tile<true>(seed, g, seed_rows, tile);
+    }
+}
+
 // The pass kernels take block blockIdx.y of a group: its slices of the working set and its entry.
 template <int LOGL, bool SEED>
 __global__ void __launch_bounds__((1 << LOGL) / 32, 1)
@@ -140,6 +161,19 @@ __global__ void __launch_bounds__((1 << LOGL) / 32, 1)
         cnt = gp.e[blockIdx.y].cnt + (SEED ? 1 : 0);
     }
     pass_a_rows<LOGL>(rows, g, Y, cnt, blockIdx.x, gridDim.x);
+}
+
+// Key (blockIdx.y = 0) and seed (1) of a block with its own seed.
+template <int LOGL>
+__global__ void __launch_bounds__((1 << LOGL) / 32, 1)
+    k_pass_a_both(const uint32_t* __restrict__ key_rows, const uint32_t* __restrict__ seed_rows, BlockGeom g,
+                  float2* __restrict__ Y, float2* __restrict__ Ys, unsigned long long* cnt) {
+    if (blockIdx.y) {
+        key_rows = seed_rows;
+        Y = Ys;
+        ++cnt;
+    }
+    pass_a_rows<LOGL>(key_rows, g, Y, cnt, blockIdx.x, gridDim.x);
 }
 
 // One block (a group's pass B is k_pass_b_group in pa_group.cu: pass B runs at the 128-register limit
@@ -327,6 +361,17 @@ static int pass_a_l(const BlockGeom& g, const uint32_t* rows, bool seed, float2*
     return seed ? go(k_pass_a<LOGL, true>) : go(k_pass_a<LOGL, false>);
 }
 
+template <int LOGL>
+static int pass_a_both_l(const BlockGeom& g, const uint32_t* key_rows, const uint32_t* seed_rows, float2* Y, float2* Ys,
+                         unsigned long long* cnt, int num_sms, cudaStream_t s) {
+    constexpr int NT = (1 << LOGL) / 32;
+    const size_t smem = (size_t)TileStride<(1 << LOGL)>::value * sizeof(float2);
+    smem_attr(k_pass_a_both<LOGL>, smem);
+    static const int per_sm = resident_ctas(k_pass_a_both<LOGL>, NT, smem);
+    const dim3 grid(grid_units(1u << g.log_n1, std::max(1, num_sms * per_sm / 2)), 2);
+    return (int)launch_pdl(k_pass_a_both<LOGL>, grid, NT, smem, s, key_rows, seed_rows, g, Y, Ys, cnt);
+}
+
 // Pass B's shared memory without the early boxes: tile / exchange buffer, column tables, stage bases, and
 // the alignment of the TMA destination.
 template <int LOGL>
@@ -473,6 +518,22 @@ static int pass_c_l(const BlockGeom& g, const PassMaps& maps, const float2* Z, c
 int launch_pass_a(const BlockGeom& g, const uint32_t* rows, bool seed, float2* Y, unsigned long long* cnt,
                   int num_sms, cudaStream_t s, const Group& gp) {
 #define C(LG) pass_a_l<LG>(g, rows, seed, Y, cnt, num_sms, s, gp)
+    PA_ROWS_DISPATCH(g.log_n2, C)
+#undef C
+}
+
+// The row passes of a block with its own seed, key and seed in one launch each: two launches less in the chain, and one
+// transform's last CTAs run beside the other's first.  2^21 bits 54.4 -> 47.8 us a block, 2^22 72.2 -> 65.1, 2^24 181 ->
+// 171, 2^27 1324 -> 1319.
+int launch_rows_both(const BlockGeom& g, const uint32_t* key, const uint32_t* seed, uint32_t* key_rows,
+                     uint32_t* seed_rows, float2* Y, float2* Ys, unsigned long long* cnt, unsigned int* resid,
+                     unsigned long long* clock, int num_sms, cudaStream_t s) {
+    const uint32_t n1 = 1u << g.log_n1, n2 = 1u << g.log_n2;
+    if (n1 < 256u || n2 < 256u) return (int)cudaErrorInvalidValue;
+    const int rc = (int)launch_pdl(k_bit_rows_both, dim3(n1 / 256u, n2 / 256u, 2), 256, 0, s, key, seed, g, key_rows,
+                                   seed_rows, Zeroed{cnt, resid, clock});
+    if (rc) return rc;
+#define C(LG) pass_a_both_l<LG>(g, key_rows, seed_rows, Y, Ys, cnt, num_sms, s)
     PA_ROWS_DISPATCH(g.log_n2, C)
 #undef C
 }

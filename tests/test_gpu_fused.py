@@ -91,3 +91,23 @@ def test_seed_sequence_switches_paths(gpu_engine):
         out = gpu_engine.process(ks, kr, n, v, DEFAULT)
         assert gpu_engine.last_stats.exact == 0
         assert np.array_equal(out, O.ntt(seed, ks, kr, n, v, DEFAULT)), step
+
+
+@pytest.mark.parametrize("n,rows", [(1 << 21, 10), (1 << 23, 10), (1 << 23, 11), (1 << 23, 12), (1 << 24, 13),
+                                    (1 << 25, 12), (1 << 25, 13), (1 << 25, 14), ((1 << 23) - 96, 11)])
+def test_one_use_seed_with_every_row_length(n, rows):
+    """Key and seed take their bit rows and row FFTs in the same launches: every row length, against the kept seed's."""
+    v = n // 4 // 32 * 32
+    seed, recv = O.random_block(n, v, n % 1009 + rows)
+    ks, kr = pa.key_split(recv, n, v)
+    with pa.Engine(1 << 25) as eng:
+        eng.set_split((n - 1).bit_length() - 1, rows)
+        assert eng.get_split((n - 1).bit_length() - 1) == rows
+        eng.set_seed(seed, n, -1)
+        kept = eng.process(ks, kr, n, v, DEFAULT)
+        popcounts = (eng.last_stats.popcount_key, eng.last_stats.popcount_seed)
+        for _ in range(2):
+            eng.set_seed(seed, n, 1)
+            assert np.array_equal(eng.process(ks, kr, n, v, DEFAULT), kept)
+            assert (eng.last_stats.popcount_key, eng.last_stats.popcount_seed) == popcounts
+    assert np.array_equal(kept, O.ntt(seed, ks, kr, n, v, DEFAULT))
