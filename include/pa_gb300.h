@@ -111,8 +111,8 @@ PA_API int pa_key_split(const uint32_t* recv_key, uint32_t n, uint32_t v, uint32
 PA_API size_t pa_output_bytes(uint32_t n, uint32_t v, uint32_t flags);
 
 /* Number of kernels one pa_process_device launches for (n, v) with a cached seed spectrum (or a
- * one-use seed of 2^21 bits and more, which shares them); 1 for the short blocks that one kernel computes
- * without a spectrum. */
+ * one-use seed, which shares them; below 2^21 bits that adds its column pass); 1 for the short blocks that
+ * one kernel computes without a spectrum. */
 PA_API int pa_kernels_per_block(uint32_t n, uint32_t v, uint32_t flags);
 
 /* Per-kernel timing, the counterpart of the reference's STOPWATCH stage deltas

@@ -95,9 +95,9 @@ int build_spectrum(pa_engine* e, const BlockGeom& g, cudaStream_t s) {
     return PA_OK;
 }
 
-// The seed serves the next block only and that block's column pass can transform it (the fused pass).
-bool fuse_seed(const pa_engine* e, const BlockGeom& g) {
-    return e->seed_left == 1 && e->d_park && pa::fused_geom(g);
+// The seed serves the next block only: its transform runs beside that block's.
+bool one_use(const pa_engine* e, const BlockGeom& g) {
+    return e->seed_left == 1 && g.log_n1 != 0 && (e->d_park || !pa::fused_geom(g));
 }
 
 int seed_common(pa_engine* e, uint32_t n, int32_t reuse, cudaStream_t s) {
@@ -114,26 +114,25 @@ int seed_common(pa_engine* e, uint32_t n, int32_t reuse, cudaStream_t s) {
         if (rc) return rc;
         if (g.exact_only) return PA_OK;  // chunk spectra are built per block, the exact transform on demand
         if (pa::short_geom(g)) return PA_OK;  // the block needs no spectrum, or builds it (g has the longest output)
-        if (fuse_seed(e, g)) return PA_OK;  // transformed inside the block's column pass
+        if (one_use(e, g)) return PA_OK;  // transformed with the block
         return build_spectrum(e, g, s);
     }
     return PA_OK;
 }
 
-// A block whose seed serves it alone: the seed's row pass into d_spec, then the fused column pass.
-// d_spec then holds no spectrum.
-int fused_block(pa_engine* e, const uint32_t* d_ks, const uint32_t* d_kr, const BlockGeom& g, uint32_t flags,
+// A block whose seed serves it alone (launch_own_block).  d_spec holds no spectrum that a later block could use.
+int own_block(pa_engine* e, const uint32_t* d_ks, const uint32_t* d_kr, const BlockGeom& g, uint32_t flags,
                 uint32_t* d_out, cudaStream_t s, cudaEvent_t* sev, cudaEvent_t kr_ready) {
     int rc = ensure_maps(e, g);
     if (rc) return rc;
     if (e->seed_maps_key != pa_host::maps_key(g)) {
-        rc = pa::make_pass_maps(g, e->d_spec, e->d_work2, &e->seed_maps);
+        rc = pa::make_pass_maps(g, pa::fused_geom(g) ? e->d_spec : e->d_work2, e->d_work2, &e->seed_maps);
         if (rc) return cuda_fail(e, (cudaError_t)rc);
         e->seed_maps_key = pa_host::maps_key(g);
     }
     e->spec_valid = false;
-    rc = pa::launch_fused_block(g, e->d_seed, d_ks, d_kr, flags, e->d_spec, e->seed_maps, e->d_park, e->park_ctas,
-                                scratch(e), e->d_cnt, e->d_resid, d_out, e->num_sms, s, sev, kr_ready, e->d_words->clock);
+    rc = pa::launch_own_block(g, e->d_seed, d_ks, d_kr, flags, e->d_spec, e->seed_maps, e->d_park, e->park_ctas,
+                              scratch(e), e->d_cnt, e->d_resid, d_out, e->num_sms, s, sev, kr_ready, e->d_words->clock);
     return rc ? cuda_fail(e, (cudaError_t)rc) : PA_OK;
 }
 
@@ -275,16 +274,16 @@ int block_common(pa_engine* e, const uint32_t* d_ks, const uint32_t* d_kr, const
         if (e->seed_left > 0) --e->seed_left;
         return PA_OK;
     }
-    const bool fused = (!e->spec_valid || !same_seed_geom(e->spec_geom, g)) && fuse_seed(e, g);
-    if (!fused && (!e->spec_valid || !same_seed_geom(e->spec_geom, g))) {
+    const bool build = !e->spec_valid || !same_seed_geom(e->spec_geom, g), own = build && one_use(e, g);
+    if (build && !own) {
         int rc = build_spectrum(e, g, s);
         if (rc) return rc;
     }
     int mrc = ensure_maps(e, g);
     if (mrc) return mrc;
     cudaEvent_t* sev = stage_events(e, g);
-    if (fused) {
-        int rc = fused_block(e, d_ks, d_kr, g, flags, d_out, s, sev, kr_ready);
+    if (own) {
+        int rc = own_block(e, d_ks, d_kr, g, flags, d_out, s, sev, kr_ready);
         if (rc) return rc;
     } else {
         int rc = pa::launch_key_block(g, d_ks, d_kr, flags, e->d_spec, scratch(e), e->d_cnt, e->d_resid, d_out,

@@ -315,21 +315,25 @@ int launch_key_block(const BlockGeom& g, const uint32_t* key_start, const uint32
     return rc;
 }
 
-int launch_fused_block(const BlockGeom& g, const uint32_t* seed, const uint32_t* key_start, const uint32_t* key_rest,
-                       uint32_t flags, float2* seed_y, const PassMaps& seed_maps, float2* park, uint32_t park_ctas,
-                       const Scratch& sc, unsigned long long* cnt, unsigned int* resid_bits, uint32_t* out_words,
-                       int num_sms, cudaStream_t s, cudaEvent_t* ev, cudaEvent_t key_rest_ready,
-                       unsigned long long* clock) {
-    if (!fused_geom(g)) return (int)cudaErrorInvalidValue;
+int launch_own_block(const BlockGeom& g, const uint32_t* seed, const uint32_t* key_start, const uint32_t* key_rest,
+                     uint32_t flags, float2* spec, const PassMaps& seed_maps, float2* park, uint32_t park_ctas,
+                     const Scratch& sc, unsigned long long* cnt, unsigned int* resid_bits, uint32_t* out_words,
+                     int num_sms, cudaStream_t s, cudaEvent_t* ev, cudaEvent_t key_rest_ready,
+                     unsigned long long* clock) {
     auto mark = [&](int i) {
         if (ev) cudaEventRecord(ev[i], s);
     };
     mark(0);
-    // the seed's bit rows in work2, which is pass B's to write
-    int rc = launch_rows_both(g, key_start, seed, sc.planes, reinterpret_cast<uint32_t*>(sc.work2), sc.work, seed_y, cnt,
+    // work2 is the key's column pass's to write: until then it has the seed's bit rows, or what its row pass makes of them
+    const bool fused = fused_geom(g);
+    float2 *seed_y = spec, *seed_rows = sc.work2;
+    if (!fused) std::swap(seed_y, seed_rows);
+    int rc = launch_rows_both(g, key_start, seed, sc.planes, reinterpret_cast<uint32_t*>(seed_rows), sc.work, seed_y, cnt,
                               resid_bits, clock, num_sms, s);
+    if (!rc && !fused) rc = launch_pass_b(g, true, seed_maps, seed_y, sc.work2, spec, sc.err, num_sms, s);
     mark(1);
-    if (!rc) rc = launch_pass_b_fused(g, seed_maps, *sc.maps, sc.work2, park, park_ctas, sc.err, num_sms, s);
+    if (!rc && fused) rc = launch_pass_b_fused(g, seed_maps, *sc.maps, sc.work2, park, park_ctas, sc.err, num_sms, s);
+    if (!rc && !fused) rc = launch_pass_b(g, false, *sc.maps, sc.work, sc.work2, spec, sc.err, num_sms, s);
     mark(2);
     if (!rc) rc = launch_pass_c(g, *sc.maps, sc.work2, cnt, sc.planes, resid_bits, sc.err, num_sms, s);
     mark(3);

@@ -78,15 +78,16 @@ int launch_key_block(const BlockGeom& g, const uint32_t* key_start, const uint32
                      const float2* spec, const Scratch& sc, unsigned long long* cnt, unsigned int* resid_bits,
                      uint32_t* out_words, int num_sms, cudaStream_t s, cudaEvent_t* stage_ev,
                      cudaEvent_t key_rest_ready = nullptr, unsigned long long* clock = nullptr);
-// A key block whose seed serves it alone, the seed's column transform fused into the key's column pass
-// (fused_geom(g) only): seed_y (N complex values, where the spectrum would go) receives the seed's row
-// pass, seed_maps are over seed_y, park holds park_ctas * kParkBytes; cnt[0] / cnt[1] receive the key and
-// seed popcounts.  Otherwise as launch_key_block (the seed's bit rows and row pass time as stage 0).
-int launch_fused_block(const BlockGeom& g, const uint32_t* seed, const uint32_t* key_start, const uint32_t* key_rest,
-                       uint32_t flags, float2* seed_y, const PassMaps& seed_maps, float2* park, uint32_t park_ctas,
-                       const Scratch& sc, unsigned long long* cnt, unsigned int* resid_bits, uint32_t* out_words,
-                       int num_sms, cudaStream_t s, cudaEvent_t* stage_ev, cudaEvent_t key_rest_ready = nullptr,
-                       unsigned long long* clock = nullptr);
+// A key block whose seed serves it alone: both row passes in one launch, then with fused_geom(g) one column pass for
+// both (park holds park_ctas * kParkBytes), else the seed's and the key's.  The seed's row pass goes to spec (N complex
+// values) when fused, else to work2, and its spectrum to spec; seed_maps are over the former.  cnt[0] / cnt[1] receive
+// the key and seed popcounts.  Otherwise as launch_key_block (what the seed takes before the key's column pass times as
+// stage 0).
+int launch_own_block(const BlockGeom& g, const uint32_t* seed, const uint32_t* key_start, const uint32_t* key_rest,
+                     uint32_t flags, float2* spec, const PassMaps& seed_maps, float2* park, uint32_t park_ctas,
+                     const Scratch& sc, unsigned long long* cnt, unsigned int* resid_bits, uint32_t* out_words,
+                     int num_sms, cudaStream_t s, cudaEvent_t* stage_ev, cudaEvent_t key_rest_ready = nullptr,
+                     unsigned long long* clock = nullptr);
 // Copies up to 256 bytes (a multiple of 4) from device to pinned host memory by a kernel.
 int launch_publish(const void* src, void* dst, size_t bytes, cudaStream_t s);
 int kernel_count_key_block(const BlockGeom& g);   // kernels one key block launches

@@ -42,14 +42,8 @@ struct Zeroed {
 // 16a..16a+15; after the half-warp transpose, lane L of half h holds row 16a + L, columns
 // 32c + 16h .. 32c + 16h + 15 -- one word of the row plane.
 template <bool SEED>
-__global__ void __launch_bounds__(256) k_bit_rows(const uint32_t* __restrict__ src, BlockGeom g,
-                                                  uint32_t* __restrict__ rows, Zeroed z, Group gp) {
-    pdl_wait();
-    z.clear();
-    if (gp.e) {  // block blockIdx.z of a group
-        src = SEED ? gp.e[blockIdx.z].seed : gp.e[blockIdx.z].key_start;
-        rows += (size_t)blockIdx.z * gp.planes;
-    }
+__device__ __forceinline__ void bit_rows_warp(const uint32_t* __restrict__ src, const BlockGeom& g,
+                                              uint32_t* __restrict__ rows) {
     const int lane = threadIdx.x & 31;
     const uint32_t n1 = 1u << g.log_n1, n2 = 1u << g.log_n2;
     const uint32_t a = blockIdx.x * 8u + (threadIdx.x >> 5);  // 16-row group
@@ -69,6 +63,18 @@ __global__ void __launch_bounds__(256) k_bit_rows(const uint32_t* __restrict__ s
     }
     const uint32_t w = transpose16x2(v, lane);
     rows[(size_t)(16u * a + (uint32_t)(lane & 15)) * (n2 / 16u) + 2u * c + (uint32_t)(lane >> 4)] = w;
+}
+
+template <bool SEED>
+__global__ void __launch_bounds__(256) k_bit_rows(const uint32_t* __restrict__ src, BlockGeom g,
+                                                  uint32_t* __restrict__ rows, Zeroed z, Group gp) {
+    pdl_wait();
+    z.clear();
+    if (gp.e) {  // block blockIdx.z of a group
+        src = SEED ? gp.e[blockIdx.z].seed : gp.e[blockIdx.z].key_start;
+        rows += (size_t)blockIdx.z * gp.planes;
+    }
+    bit_rows_warp<SEED>(src, g, rows);
 }
 
 // Tiled form for N1, N2 >= 256 (the large blocks): a CTA moves a 256 x 256 block of 2-bit elements,
@@ -136,17 +142,20 @@ __global__ void __launch_bounds__(256) k_bit_rows_tiled(const uint32_t* __restri
 }
 
 // Key (blockIdx.z = 0) and seed (1) of a block with its own seed.
+template <bool TILED>
 __global__ void __launch_bounds__(256)
     k_bit_rows_both(const uint32_t* __restrict__ key, const uint32_t* __restrict__ seed, BlockGeom g,
                     uint32_t* __restrict__ key_rows, uint32_t* __restrict__ seed_rows, Zeroed z) {
-    __shared__ uint32_t tile[256][17];
+    __shared__ uint32_t tile[TILED ? 256 : 1][17];
     pdl_wait();
     z.clear();
     if (blockIdx.z == 0) {
-        bit_rows_tile<false>(key, g, key_rows, tile);
+        if (TILED) bit_rows_tile<false>(key, g, key_rows, tile);
+        else bit_rows_warp<false>(key, g, key_rows);
     } else {
         if (threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0) z.cnt[1] = 0ull;
-        bit_rows_tile<true>(seed, g, seed_rows, tile);
+        if (TILED) bit_rows_tile<true>(seed, g, seed_rows, tile);
+        else bit_rows_warp<true>(seed, g, seed_rows);
     }
 }
 
@@ -524,14 +533,15 @@ int launch_pass_a(const BlockGeom& g, const uint32_t* rows, bool seed, float2* Y
 
 // The row passes of a block with its own seed, key and seed in one launch each: two launches less in the chain, and one
 // transform's last CTAs run beside the other's first.  2^21 bits 54.4 -> 47.8 us a block, 2^22 72.2 -> 65.1, 2^24 181 ->
-// 171, 2^27 1324 -> 1319.
+// 171, 2^27 1324 -> 1319; 2^18 47.1 -> 41.4, 2^20 49.3 -> 42.7.
 int launch_rows_both(const BlockGeom& g, const uint32_t* key, const uint32_t* seed, uint32_t* key_rows,
                      uint32_t* seed_rows, float2* Y, float2* Ys, unsigned long long* cnt, unsigned int* resid,
                      unsigned long long* clock, int num_sms, cudaStream_t s) {
     const uint32_t n1 = 1u << g.log_n1, n2 = 1u << g.log_n2;
-    if (n1 < 256u || n2 < 256u) return (int)cudaErrorInvalidValue;
-    const int rc = (int)launch_pdl(k_bit_rows_both, dim3(n1 / 256u, n2 / 256u, 2), 256, 0, s, key, seed, g, key_rows,
-                                   seed_rows, Zeroed{cnt, resid, clock});
+    const bool tiled = n1 >= 256u && n2 >= 256u;
+    const dim3 grid = tiled ? dim3(n1 / 256u, n2 / 256u, 2) : dim3((n1 / 16u + 7u) / 8u, n2 / 32u, 2);
+    const int rc = (int)launch_pdl(tiled ? k_bit_rows_both<true> : k_bit_rows_both<false>, grid, 256, 0, s, key, seed, g,
+                                   key_rows, seed_rows, Zeroed{cnt, resid, clock});
     if (rc) return rc;
 #define C(LG) pass_a_both_l<LG>(g, key_rows, seed_rows, Y, Ys, cnt, num_sms, s)
     PA_ROWS_DISPATCH(g.log_n2, C)

@@ -94,7 +94,10 @@ def test_seed_sequence_switches_paths(gpu_engine):
 
 
 @pytest.mark.parametrize("n,rows", [(1 << 21, 10), (1 << 23, 10), (1 << 23, 11), (1 << 23, 12), (1 << 24, 13),
-                                    (1 << 25, 12), (1 << 25, 13), (1 << 25, 14), ((1 << 23) - 96, 11)])
+                                    (1 << 25, 12), (1 << 25, 13), (1 << 25, 14), ((1 << 23) - 96, 11),
+                                    # columns below 2^10: a column pass each
+                                    (1 << 18, 10), (1 << 18, 11), (1 << 18, 12), (1 << 19, 10), (1 << 20, 10), (1 << 20, 14),
+                                    ((1 << 19) - 96, 13), ((1 << 20) + 32, 12), (1 << 22, 13), (1 << 24, 14)])
 def test_one_use_seed_with_every_row_length(n, rows):
     """Key and seed take their bit rows and row FFTs in the same launches: every row length, against the kept seed's."""
     v = n // 4 // 32 * 32
