@@ -82,14 +82,17 @@ struct Slot {
     float2* work = nullptr;   // pass A output / exact-path elements
     float2* work2 = nullptr;  // pass B output / exact-path scratch
     float2* spec = nullptr;   // dynamic seed spectrum / exact seed transform
+    // One allocation: bit planes, result, then (still needed when a served block is computed again) seed and keys.  A
+    // column pass parks spectrum tiles in it while it holds nothing: in planes and result, in all of it for a batch.
     uint32_t* planes = nullptr;
+    uint32_t park_serve = 0, park_batch = 0;  // tiles
     int* err = nullptr;
     unsigned long long* cnt = nullptr;  // served block: [0] key, [1] seed popcount
     unsigned int* resid = nullptr;
     uint32_t *seed = nullptr, *ks = nullptr, *kr = nullptr, *out = nullptr;  // served-block staging
     Mirror* host = nullptr;
-    pa::PassMaps maps{};
-    int maps_key = -1;
+    pa::PassMaps maps{}, seed_maps{};
+    int maps_key = -1, seed_maps_key = -1;
     cudaEvent_t done = nullptr, join = nullptr;
     // served block in flight
     bool busy = false;
@@ -203,10 +206,6 @@ void free_slot(Pool* p, Slot* sl) {
     cudaFree(sl->err);
     cudaFree(sl->cnt);
     cudaFree(sl->resid);
-    cudaFree(sl->seed);
-    cudaFree(sl->ks);
-    cudaFree(sl->kr);
-    cudaFree(sl->out);
     cudaFreeHost(sl->host);
     if (sl->done) cudaEventDestroy(sl->done);
     if (sl->join) cudaEventDestroy(sl->join);
@@ -235,14 +234,16 @@ int new_slot(pa_engine* e, Pool* p, int cap, Slot** out) {
     A((void**)&sl->work, (np / 2) * sizeof(float2));
     A((void**)&sl->work2, (np / 2) * sizeof(float2));
     A((void**)&sl->spec, (np32 / 2) * sizeof(float2));
-    A((void**)&sl->planes, np32 / 8 + 256);
+    A((void**)&sl->planes, np32 / 8 + 256 + 4 * words * 4);
     A((void**)&sl->err, sizeof(int));
     A((void**)&sl->cnt, 2 * sizeof(unsigned long long));
     A((void**)&sl->resid, sizeof(unsigned int));
-    A((void**)&sl->seed, words * 4);
-    A((void**)&sl->ks, words * 4);
-    A((void**)&sl->kr, words * 4);
-    A((void**)&sl->out, words * 4);
+    sl->out = sl->planes + (np32 / 8 + 256) / 4;
+    sl->seed = sl->out + words;
+    sl->ks = sl->seed + words;
+    sl->kr = sl->ks + words;
+    sl->park_serve = (uint32_t)((size_t)(sl->seed - sl->planes) * 4 / pa::kParkBytes);
+    sl->park_batch = (uint32_t)((size_t)(sl->kr + words - sl->planes) * 4 / pa::kParkBytes);
     if (err == cudaSuccess) err = cudaMallocHost((void**)&sl->host, sizeof(Mirror));
     if (err == cudaSuccess) err = cudaStreamCreateWithFlags(&sl->s, cudaStreamNonBlocking);
     if (err == cudaSuccess) err = cudaEventCreateWithFlags(&sl->done, cudaEventDisableTiming);
@@ -348,6 +349,36 @@ int key_in_slot(pa_engine* e, Slot* sl, const BlockGeom& g, const uint32_t* ks, 
     return rc ? cuda_fail(e, (cudaError_t)rc) : PA_OK;
 }
 
+// One column pass for key and seed, where a slot's idle buffers park enough tiles for it: a CTA per SM in a batch, whose
+// slots fill the rest, and two for a served block, which may run beside few others (2^25 bits in 128 CTAs instead of 304:
+// six requests 8 % slower).
+bool fused_in_slot(const BlockGeom& g, uint32_t park_ctas, uint32_t enough) {
+    return pa::fused_geom(g) && park_ctas >= std::min(enough, 1u << (g.log_n - 13));
+}
+
+// A block with its own seed in a slot, its row passes in one launch each as those of a single block: 64 uneven blocks
+// 5.72 -> 5.62 ms, 13 of up to 2^24 bits 1.28 -> 1.17.
+int own_in_slot(pa_engine* e, Slot* sl, const BlockGeom& g, const uint32_t* d_seed, const uint32_t* ks, const uint32_t* kr,
+                uint32_t flags, uint32_t park_ctas, bool fused, unsigned long long* cnt, unsigned int* resid, uint32_t* out,
+                cudaStream_t s) {
+    if (g.log_n1 == 0) {
+        int rc = seed_in_slot(e, sl, g, d_seed, sl->spec, cnt + 1, s);
+        return rc ? rc : key_in_slot(e, sl, g, ks, kr, flags, sl->spec, cnt, resid, out, s);
+    }
+    int rc = ensure_slot_maps(e, sl, g);
+    if (rc) return rc;
+    const int key = 2 * maps_key(g) + (fused ? 1 : 0);
+    if (sl->seed_maps_key != key) {
+        rc = pa::make_pass_maps(g, fused ? sl->spec : sl->work2, sl->work2, &sl->seed_maps);
+        if (rc) return cuda_fail(e, (cudaError_t)rc);
+        sl->seed_maps_key = key;
+    }
+    rc = pa::launch_own_block(g, d_seed, ks, kr, flags, sl->spec, sl->seed_maps,
+                              fused ? reinterpret_cast<float2*>(sl->planes) : nullptr, park_ctas, slot_scratch(sl), cnt,
+                              resid, out, e->num_sms, s, nullptr);
+    return rc ? cuda_fail(e, (cudaError_t)rc) : PA_OK;
+}
+
 // Exact recompute of one block in a slot (its spectrum buffer holds the seed transform).
 int exact_in_slot(pa_engine* e, Slot* sl, const BlockGeom& g, const uint32_t* d_seed, const uint32_t* ks,
                   const uint32_t* kr, uint32_t flags, uint32_t* out, cudaStream_t s) {
@@ -449,20 +480,18 @@ int batch_enqueue(pa_engine* e, Pool* p, const std::vector<std::vector<int>>& or
             const BlockGeom& g = p->geoms[j];
             unsigned long long* cnt = p->job_cnt + 2 * (size_t)j;
             unsigned int* resid = p->job_resid + j;
-            const float2* spec;
+            uint32_t* const out = reinterpret_cast<uint32_t*>(jb.out);
+            const bool fused = fused_in_slot(g, sl->park_batch, (uint32_t)e->num_sms);
             int rc;
             if (jb.seed_id >= 0) {
                 const SeedEntry& se = p->seeds[jb.seed_id];
                 PA_CUDA(e, cudaMemcpyAsync(cnt + 1, se.cnt, sizeof(unsigned long long), cudaMemcpyDeviceToDevice,
                                            sl->s));
-                spec = se.spec;
+                rc = key_in_slot(e, sl, g, jb.key_start, jb.key_rest, jb.flags, se.spec, cnt, resid, out, sl->s);
             } else {
-                rc = seed_in_slot(e, sl, g, jb.seed_words, sl->spec, cnt + 1, sl->s);
-                if (rc) return rc;
-                spec = sl->spec;
+                rc = own_in_slot(e, sl, g, jb.seed_words, jb.key_start, jb.key_rest, jb.flags, sl->park_batch, fused,
+                                 cnt, resid, out, sl->s);
             }
-            rc = key_in_slot(e, sl, g, jb.key_start, jb.key_rest, jb.flags, spec, cnt, resid,
-                             reinterpret_cast<uint32_t*>(jb.out), sl->s);
             if (rc) return rc;
         }
         PA_CUDA(e, cudaEventRecord(sl->join, sl->s));
@@ -1365,21 +1394,27 @@ int pa_submit(pa_engine* e, const pa_job* job, uint64_t* ticket) {
     }
     const uint32_t n = job->n, v = job->v;
     cudaStream_t s = sl->s;
-    const float2* spec;
-    if (job->seed_id >= 0) {
-        const SeedEntry& se = p->seeds[job->seed_id];
-        PA_CUDA(e, cudaMemcpyAsync(sl->cnt + 1, se.cnt, sizeof(unsigned long long), cudaMemcpyDeviceToDevice, s));
-        spec = se.spec;
-    } else {
+    // A long seed's transform hides behind the key's copies (2^26 bits: four requests 3 % faster); a short one, and one
+    // whose column pass is the key's, runs with the key's.
+    const bool fused = fused_in_slot(g, sl->park_serve, 2u * (uint32_t)e->num_sms), apart = !fused && g.log_np > 24;
+    if (job->seed_id < 0) {
         PA_CUDA(e, cudaMemcpyAsync(sl->seed, job->seed_words, (size_t)(n / 32u) * 4u, cudaMemcpyHostToDevice, s));
-        rc = seed_in_slot(e, sl, g, sl->seed, sl->spec, sl->cnt + 1, s);
+        if (apart) rc = seed_in_slot(e, sl, g, sl->seed, sl->spec, sl->cnt + 1, s);
         if (rc) return rc;
-        spec = sl->spec;
     }
     PA_CUDA(e, cudaMemcpyAsync(sl->ks, job->key_start, (size_t)(g.h / 32u + 1u) * 4u, cudaMemcpyHostToDevice, s));
     if (job->flags & PA_FLAG_XOR_KEY_REST)
         PA_CUDA(e, cudaMemcpyAsync(sl->kr, job->key_rest, (size_t)(v / 32u) * 4u, cudaMemcpyHostToDevice, s));
-    rc = key_in_slot(e, sl, g, sl->ks, sl->kr, job->flags, spec, sl->cnt, sl->resid, sl->out, s);
+    if (job->seed_id >= 0) {
+        const SeedEntry& se = p->seeds[job->seed_id];
+        PA_CUDA(e, cudaMemcpyAsync(sl->cnt + 1, se.cnt, sizeof(unsigned long long), cudaMemcpyDeviceToDevice, s));
+        rc = key_in_slot(e, sl, g, sl->ks, sl->kr, job->flags, se.spec, sl->cnt, sl->resid, sl->out, s);
+    } else if (apart) {
+        rc = key_in_slot(e, sl, g, sl->ks, sl->kr, job->flags, sl->spec, sl->cnt, sl->resid, sl->out, s);
+    } else {
+        rc = own_in_slot(e, sl, g, sl->seed, sl->ks, sl->kr, job->flags, sl->park_serve, fused, sl->cnt, sl->resid, sl->out,
+                         s);
+    }
     if (rc) return rc;
     PA_CUDA(e, cudaMemcpyAsync(job->out, sl->out, pa_output_bytes(n, v, job->flags), cudaMemcpyDeviceToHost, s));
     PA_CUDA(e, cudaMemcpyAsync(sl->host->cnt, sl->cnt, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));

@@ -325,7 +325,7 @@ int launch_own_block(const BlockGeom& g, const uint32_t* seed, const uint32_t* k
     };
     mark(0);
     // work2 is the key's column pass's to write: until then it has the seed's bit rows, or what its row pass makes of them
-    const bool fused = fused_geom(g);
+    const bool fused = park && fused_geom(g);
     float2 *seed_y = spec, *seed_rows = sc.work2;
     if (!fused) std::swap(seed_y, seed_rows);
     int rc = launch_rows_both(g, key_start, seed, sc.planes, reinterpret_cast<uint32_t*>(seed_rows), sc.work, seed_y, cnt,

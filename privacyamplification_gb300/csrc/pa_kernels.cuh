@@ -78,8 +78,8 @@ int launch_key_block(const BlockGeom& g, const uint32_t* key_start, const uint32
                      const float2* spec, const Scratch& sc, unsigned long long* cnt, unsigned int* resid_bits,
                      uint32_t* out_words, int num_sms, cudaStream_t s, cudaEvent_t* stage_ev,
                      cudaEvent_t key_rest_ready = nullptr, unsigned long long* clock = nullptr);
-// A key block whose seed serves it alone: both row passes in one launch, then with fused_geom(g) one column pass for
-// both (park holds park_ctas * kParkBytes), else the seed's and the key's.  The seed's row pass goes to spec (N complex
+// A key block whose seed serves it alone: both row passes in one launch, then with fused_geom(g) and a park one column
+// pass for both (park holds park_ctas * kParkBytes), else the seed's and the key's.  The seed's row pass goes to spec (N complex
 // values) when fused, else to work2, and its spectrum to spec; seed_maps are over the former.  cnt[0] / cnt[1] receive
 // the key and seed popcounts.  Otherwise as launch_key_block (what the seed takes before the key's column pass times as
 // stage 0).

@@ -232,3 +232,33 @@ def test_two_slots_concurrently_many_times(torch_cuda, engine):
         assert st[0].exact == 0 and st[1].exact == 0
         assert np.array_equal(out_a.cpu().numpy(), want_a), it
         assert np.array_equal(out_b.cpu().numpy(), want_b), it
+
+
+@pytest.mark.parametrize("lo,hi", [(17, 21), (21, 23), (23, 25)])
+def test_own_seed_blocks_in_slots_match_alone(torch_cuda, engine, lo, hi):
+    """Blocks with their own seed, batched and served, on either side of the sizes whose column passes are one in a slot
+    of this capacity: bit for bit the kept seed's result."""
+    reqs = W.poisson_requests(rate=20000, count=10, lo=lo, hi=hi, rng_seed=100 + hi)
+    words = max(r.n // 32 + max(r.seed_word0, r.key_word0) for r in reqs) + 64
+    banks = W.HostBanks(words)
+    want = [alone(engine, banks.seed_words(r), banks.key_start(r), banks.key_rest(r), r.n, r.v, r.flags) for r in reqs]
+    small = min(reqs, key=lambda r: r.n)
+    assert np.array_equal(want[reqs.index(small)],
+                          O.ntt(banks.seed_words(small), banks.key_start(small), banks.key_rest(small), small.n, small.v,
+                                small.flags))
+    t = lambda a: torch_cuda.from_numpy(np.ascontiguousarray(a).view(np.int32).copy()).cuda()
+    bufs = [(t(banks.seed_words(r)), t(banks.key_start(r)), t(banks.key_rest(r))) for r in reqs]
+    outs = [torch_cuda.zeros(len(w), dtype=torch_cuda.uint8, device="cuda") for w in want]
+    jobs = [pa.PAJob(s.data_ptr(), -1, k.data_ptr(), x.data_ptr(), r.n, r.v, r.flags, o.data_ptr())
+            for r, (s, k, x), o in zip(reqs, bufs, outs)]
+    torch_cuda.cuda.synchronize()
+    for mode in (pa.BATCH_SERIAL, 0, pa.BATCH_GRAPH, pa.BATCH_GRAPH):
+        for o in outs:
+            o.zero_()
+        torch_cuda.cuda.synchronize()
+        engine.batch_run(jobs, mode)
+        stats = engine.batch_sync(len(jobs))
+        assert all(np.array_equal(o.cpu().numpy(), w) for o, w in zip(outs, want)), mode
+        assert all(st.exact == 0 and st.popcount_seed > 0 and st.popcount_key > 0 for st in stats)
+    res = W.serve(engine, reqs, banks, out_slots=8, keep=lambda r: True)
+    assert all(np.array_equal(res.outputs[r.rid], w) for r, w in zip(reqs, want))
