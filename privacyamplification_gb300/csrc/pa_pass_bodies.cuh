@@ -18,6 +18,7 @@
 #include "pa_fft.cuh"
 #include "pa_kernels.cuh"
 #include "pa_launch.cuh"
+#include "pa_parity.cuh"
 #include "pa_tma.cuh"
 
 namespace pa {
@@ -746,16 +747,6 @@ __device__ __forceinline__ void pass_b_tiles(const CUtensorMap* mapY, const floa
 }
 
 // ============================================================================ pass C
-// |v - 2 rint(v / 2)| - 1/2: positive where rint(v) is odd, and 1/2 minus its magnitude is v's distance to the nearest
-// integer.  FP32 adds and multiplies only (rint and the conversion to an integer run at an eighth of their rate):
-// v / 2 is rounded by adding 3 2^22, exact while |v| < 2^23; beyond, v is an integer, and a value whose half is not
-// rounded right has a remainder of 2, which the residual reports as 1.
-__device__ __forceinline__ float parity_half(float v) {
-    const float magic = 12582912.0f;
-    const float q = __fadd_rn(__fmaf_rn(v, 0.5f, magic), -magic);
-    return fabsf(__fmaf_rn(-2.0f, q, v)) - 0.5f;
-}
-
 // Row m1: inverse FFT over k2 (radices 16, RB, RA), + correction, round, parity bit planes.
 // Input: Z, tile-major from pass B.  Row m1 is the CPT/2 pairs of row m1 of every tile; 3D TMA boxes
 // (256 tiles x 1 row x CPT/2 pairs) gather it into shared memory in pair order (float4 p = pair p),
