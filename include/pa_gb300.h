@@ -96,7 +96,10 @@ PA_API int pa_process(pa_engine* e, const uint32_t* key_start, const uint32_t* k
 
 /* Device-resident forms: pointers are device memory, work is queued on `stream` (a cudaStream_t;
  * NULL = the engine's stream) and the call returns without synchronising.  d_out receives
- * pa_output_bytes() bytes rounded up to a multiple of 4.  pa_sync() waits and fills stats. */
+ * pa_output_bytes() bytes rounded up to a multiple of 4.  pa_sync() waits and fills stats.
+ * Both may be captured into a CUDA graph.  A replayed block reads the engine's seed as it is then (a later
+ * pa_set_seed* is followed) and transforms it each time; from the first captured call on, blocks that are not
+ * captured do so too, since replays rewrite what the engine keeps of a seed.  Reuse is counted per call. */
 PA_API int pa_set_seed_device(pa_engine* e, const uint32_t* d_seed_words, uint32_t n, int32_t reuse_seed_amount,
                        void* stream);
 PA_API int pa_process_device(pa_engine* e, const uint32_t* d_key_start, const uint32_t* d_key_rest, uint32_t n,

@@ -95,20 +95,31 @@ int build_spectrum(pa_engine* e, const BlockGeom& g, cudaStream_t s) {
     return PA_OK;
 }
 
-// The seed serves the next block only: its transform runs beside that block's.
+// The seed's transform runs beside the block's: the seed serves that block only, or nothing kept can be relied on.
 bool one_use(const pa_engine* e, const BlockGeom& g) {
-    return e->seed_left == 1 && g.log_n1 != 0 && (e->d_park || !pa::fused_geom(g));
+    return (e->seed_left == 1 || e->captured) && g.log_n1 != 0 && (e->d_park || !pa::fused_geom(g));
+}
+
+// What is kept of the current seed no longer holds.
+void drop_seed_data(pa_engine* e) { e->spec_valid = e->exact_valid = e->chunk_valid = e->count_valid = false; }
+
+// A captured block may be replayed after other seeds have been set and other blocks have run.  So it transforms the seed
+// that lies in d_seed then, into the buffers of the kept transforms; and since the host does not see replays, every
+// block of the engine does so from then on.
+int note_capture(pa_engine* e, cudaStream_t s) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    PA_CUDA(e, cudaStreamIsCapturing(s, &capture));
+    if (capture != cudaStreamCaptureStatusNone) e->captured = true;
+    if (e->captured) drop_seed_data(e);
+    return PA_OK;
 }
 
 int seed_common(pa_engine* e, uint32_t n, int32_t reuse, cudaStream_t s) {
     e->seed_valid = true;
     e->seed_n = n;
     e->seed_left = reuse < 0 ? -1 : std::max<int64_t>(reuse, 1);
-    e->spec_valid = false;
-    e->exact_valid = false;
-    e->chunk_valid = false;
-    e->count_valid = false;
-    if (is_pow2(n)) {  // placement does not depend on v: build the spectrum now
+    drop_seed_data(e);
+    if (is_pow2(n) && !e->captured) {  // placement does not depend on v: build the spectrum now
         BlockGeom g;
         int rc = make_geom(n, n / 2u, PA_FLAG_COMPRESS, e->split, &g);
         if (rc) return rc;
@@ -200,27 +211,22 @@ cudaEvent_t* stage_events(pa_engine* e, const BlockGeom& g) {
 }
 
 // A short block word by word (pa_direct.cu): exact, so that its residual is zero.  The seed's popcount is formed with
-// the first block of a seed and placement, and with every block that is captured, which may be replayed on later seeds.
+// the first block of a seed and placement.
 int direct_block(pa_engine* e, const uint32_t* d_ks, const uint32_t* d_kr, const BlockGeom& g, uint32_t flags,
                  uint32_t* d_out, cudaStream_t s) {
     if (pa::direct_overlap(g, d_ks, d_out)) {  // every result word reads the whole key
         PA_CUDA(e, cudaMemcpyAsync(e->d_key_start, d_ks, (size_t)(g.h / 32u + 1u) * 4u, cudaMemcpyDeviceToDevice, s));
         d_ks = e->d_key_start;
     }
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    PA_CUDA(e, cudaStreamIsCapturing(s, &capture));
-    const bool captured = capture != cudaStreamCaptureStatusNone;
-    const bool counted = !captured && e->count_valid && same_seed_geom(e->count_geom, g);
+    const bool counted = e->count_valid && same_seed_geom(e->count_geom, g);
     cudaEvent_t* ev = stage_events(e, g);
     if (ev) cudaEventRecord(ev[0], s);
     int rc = pa::launch_direct(g, e->d_seed, d_ks, d_kr, flags, d_out, s,
                                {e->d_words->short_cnt, e->d_resid, counted ? 0 : 1, e->d_words->clock});
     if (rc) return cuda_fail(e, (cudaError_t)rc);
     if (ev) cudaEventRecord(ev[1], s);
-    if (!captured) {
-        e->count_geom = g;
-        e->count_valid = true;
-    }
+    e->count_geom = g;
+    e->count_valid = true;
     return PA_OK;
 }
 
@@ -246,6 +252,8 @@ int block_common(pa_engine* e, const uint32_t* d_ks, const uint32_t* d_kr, const
                  uint32_t* d_out, cudaStream_t s, cudaEvent_t kr_ready = nullptr) {
     if (!e->seed_valid || e->seed_left == 0) return PA_ERR_NO_SEED;
     if (g.n != e->seed_n) return PA_ERR_INVALID_ARG;
+    int crc = note_capture(e, s);
+    if (crc) return crc;
     e->last_chunked = e->last_direct = false;
     if (kr_ready && ((flags & PA_FLAG_EXACT) || g.exact_only))  // these paths read key_rest early
         PA_CUDA(e, cudaStreamWaitEvent(s, kr_ready, 0));
@@ -481,6 +489,8 @@ int pa_set_seed_device(pa_engine* e, const uint32_t* d_seed_words, uint32_t n, i
     if (rc) return rc;
     cudaStream_t s = stream ? (cudaStream_t)stream : e->stream;
     PA_CUDA(e, cudaSetDevice(e->device));
+    rc = note_capture(e, s);
+    if (rc) return rc;
     PA_CUDA(e, cudaMemcpyAsync(e->d_seed, d_seed_words, (size_t)(n / 32u) * 4u, cudaMemcpyDeviceToDevice, s));
     e->pending = true;
     return seed_common(e, n, reuse_seed_amount, s);

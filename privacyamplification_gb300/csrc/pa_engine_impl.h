@@ -86,6 +86,7 @@ struct pa_engine {
     pa::BlockGeom spec_geom{};
     bool count_valid = false;  // short_cnt[1] is the seed's popcount for count_geom
     pa::BlockGeom count_geom{};
+    bool captured = false;  // a call was captured: replays change d_seed and the kept transforms unseen
     int last_cuda = 0;
     bool pending = false;  // device-form work queued and not yet synchronised
     // per-kernel timing ring (pa_set_timing / pa_stage_times)
