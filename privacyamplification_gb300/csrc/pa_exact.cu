@@ -995,6 +995,18 @@ __global__ void __launch_bounds__(1 << (LOWB - 5), LOWB >= 13 ? 2 : 1)
 }
 
 // ------------------------------------------------------------------------------------ host side
+// Allows a kernel the most that any of its launches asks for.  The limit belongs to the function, not to the launch: set
+// to each launch's own size, it could be lowered by another engine's thread before a longer block's launch.
+template <class K>
+void smem_limit(K kernel, size_t most) {
+    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+}
+constexpr int kMaxPoints = 27;  // log2 of the longest transform (2^30 bits, result not compressed)
+constexpr int kMaxTop = 10;     // levels of one pass of k_exact_top
+constexpr size_t kUpperSmem = (size_t(kUpRow + kUpEdge) << kMaxUp) * sizeof(uint32_t);
+constexpr size_t kRowsSmem = (size_t(kBcCols) << (kMaxPoints - 5 - 11)) * sizeof(uint32_t);
+constexpr size_t kTopSmem = (size_t(kTopRow) << kMaxTop) * sizeof(uint32_t);
+
 // l = log2 of the points: 16 P >= h + out_bits, at least 2^16 points (the basis conversion's run).  The low
 // pass takes 2^lowb points per CTA, few enough that the CTAs of a short transform cover the SMs; the levels
 // above go in passes of at most 10 (80 KB of shared memory).
@@ -1009,7 +1021,7 @@ Shape shape_of(const BlockGeom& g) {
     while ((16ull << s.l) < need) ++s.l;
     s.lowb = s.l <= 18 ? 11 : (s.l == 19 ? 12 : 13);
     const int top = s.l - s.lowb;
-    s.passes = top > 10 ? 2 : 1;
+    s.passes = top > kMaxTop ? 2 : 1;
     s.T[0] = s.passes == 2 ? (top + 1) / 2 : top;  // the upper pass first
     s.lo[0] = s.l - s.T[0];
     s.T[1] = top - s.T[0];
@@ -1027,11 +1039,6 @@ struct Chain {
         if (err == cudaSuccess) err = launch_pdl(kernel, grid, block, smem, s, std::forward<A>(args)...);
     }
 };
-
-template <class K>
-void smem_limit(K kernel, size_t bytes) {
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-}
 
 // The basis conversion on `planes` planes in a (b: scratch of the same size); returns where the result is.
 // Up to 2^23 coefficients a plane: the rounds above bit 16 in one pass; longer planes' first Taylor rounds one by one
@@ -1052,7 +1059,7 @@ uint32_t* convert_basis(const Shape& sh, uint32_t* a, uint32_t* b, uint32_t plan
         if (!low) return;
         const int R = 1 << low, W = kUpRow - (R + 31) / 32;
         const size_t smem = (size_t)R * (kUpRow + kUpEdge) * sizeof(uint32_t);
-        smem_limit(k_exact_upper<OP>, smem);
+        smem_limit(k_exact_upper<OP>, kUpperSmem);
         ch.run(k_exact_upper<OP>, dim3((2048u + W - 1u) / W, planes << (up - low)), kUpThreads, smem, a, b, low,
                up == low ? rs : none);
         std::swap(a, b);
@@ -1060,7 +1067,7 @@ uint32_t* convert_basis(const Shape& sh, uint32_t* a, uint32_t* b, uint32_t plan
     auto rows = [&] {
         if (up == low) return;
         const size_t smem = (size_t)(sh.pw / 2048u) * kBcCols * sizeof(uint32_t);
-        smem_limit(k_exact_bc_rows<OP>, smem);
+        smem_limit(k_exact_bc_rows<OP>, kRowsSmem);
         ch.run(k_exact_bc_rows<OP>, dim3(2048u / kBcCols, planes), 256, smem, a, sh.pw, rs);
     };
     auto runs = [&] { ch.run(k_exact_bc16<OP>, dim3(sh.pw / 2048u, planes), kBcThreads, 0, a, sh.pw); };
@@ -1084,7 +1091,7 @@ void top_levels(const Shape& sh, uint32_t* W, Chain& ch) {
         const int p = OP == kT ? sh.passes - 1 - k : k, T = sh.T[p], lo = sh.lo[p];
         if (T == 0) continue;
         const size_t smem = ((size_t)kTopRow << T) * sizeof(uint32_t);
-        smem_limit(k_exact_top<OP>, smem);
+        smem_limit(k_exact_top<OP>, kTopSmem);
         const int nt = std::max(32, std::min(512, 1 << (T - 1)));
         ch.run(k_exact_top<OP>, dim3(2u << (lo - 5), 1u << (sh.l - lo - T)), nt, smem, W, sh.l, lo, T);
     }

@@ -469,7 +469,8 @@ static int pass_c_k(const BlockGeom& g, const PassMaps& maps, const float2* Z, c
     const uint32_t cpt = 8192u >> g.log_n1, ntiles = (1u << LOGL) / cpt;
     const size_t box_bytes = (size_t)(ntiles < 256u ? ntiles : 256u) * cpt * sizeof(float2);
     const size_t smem = exch + (size_t)early * box_bytes;
-    smem_attr(k_pass_c<LOGL, KEEP8>, smem);
+    // the function's limit, not this launch's size: another engine's thread may be about to launch a larger one
+    smem_attr(k_pass_c<LOGL, KEEP8>, early > 0 ? smem_optin_limit() - static_bytes : smem);
     // by the number of early boxes and the box size (pass B's tile width), which fix the shared memory
     static std::atomic<int> resident[33][16];
     std::atomic<int>& known = resident[early][g.log_n1 & 15];
