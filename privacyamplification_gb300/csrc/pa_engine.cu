@@ -470,15 +470,28 @@ static int check_seed_n(pa_engine* e, uint32_t n) {
     return check_n(e, n, 32u, PA_FLAG_COMPRESS, &g);
 }
 
+// Waits for what a call has queued when it returns with an error: the copies and kernels read the caller's buffers.
+struct WaitOnError {
+    cudaStream_t main, side;
+    bool ok = false;
+    ~WaitOnError() {
+        if (ok) return;
+        cudaStreamSynchronize(side);
+        cudaStreamSynchronize(main);
+    }
+};
+
 int pa_set_seed(pa_engine* e, const uint32_t* seed_words, uint32_t n, int32_t reuse_seed_amount) {
     if (!e || !seed_words) return PA_ERR_INVALID_ARG;
     int rc = check_seed_n(e, n);
     if (rc) return rc;
     PA_CUDA(e, cudaSetDevice(e->device));
+    WaitOnError wait{e->stream, e->side};
     PA_CUDA(e, cudaMemcpyAsync(e->d_seed, seed_words, (size_t)(n / 32u) * 4u, cudaMemcpyHostToDevice, e->stream));
     rc = seed_common(e, n, reuse_seed_amount, e->stream);
     if (rc) return rc;
     PA_CUDA(e, cudaStreamSynchronize(e->stream));
+    wait.ok = true;
     return PA_OK;
 }
 
@@ -517,6 +530,7 @@ int pa_process(pa_engine* e, const uint32_t* key_start, const uint32_t* key_rest
     if (n != e->seed_n) return PA_ERR_INVALID_ARG;
     PA_CUDA(e, cudaSetDevice(e->device));
     cudaStream_t s = e->stream;
+    WaitOnError wait{s, e->side};
     // Pinned inputs of up to 256 KB are read where they lie: a copy of any size holds the stream for 11 us (2^16 bits
     // host to host 40 -> 29.5 us a call; longer keys come faster by a copy).  key_rest is first read by the block's last
     // kernel: a long one is copied on the side stream (after whatever the engine stream had queued) while the passes run.
@@ -548,11 +562,7 @@ int pa_process(pa_engine* e, const uint32_t* key_start, const uint32_t* key_rest
     const bool staged = ob <= pa_engine::kStageBytes;
     uint32_t* const d_out = staged ? reinterpret_cast<uint32_t*>(e->h_stage) : e->d_out;
     rc = block_common(e, d_ks, d_kr, g, flags, d_out, s, kr_ready);
-    if (rc) {
-        if (kr_ready) cudaStreamSynchronize(e->side);
-        cudaStreamSynchronize(s);  // the caller's buffers are not read after we return
-        return rc;
-    }
+    if (rc) return rc;
     auto collect = [&](pa_stats* st, float* resid) -> int {
         int prc = pa::launch_publish(e->d_words, e->h_words, sizeof(pa_engine::Words), s);
         if (prc) return cuda_fail(e, (cudaError_t)prc);
@@ -574,6 +584,7 @@ int pa_process(pa_engine* e, const uint32_t* key_start, const uint32_t* key_rest
     }
     if (staged) std::memcpy(out, e->h_stage, ob);
     else PA_CUDA(e, cudaMemcpy(out, e->d_out, ob, cudaMemcpyDeviceToHost));
+    wait.ok = true;
     return PA_OK;
 }
 

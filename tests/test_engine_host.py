@@ -1,0 +1,94 @@
+"""The host side of single blocks (pa_engine.cu), compiled against a fake CUDA runtime (fake_runtime.cpp): what a call does
+when one of the calls below it fails.  No GPU."""
+import ctypes
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from privacyamplification_gb300 import FLAG_EXACT, DEFAULT_FLAGS
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC = os.path.join(ROOT, "privacyamplification_gb300", "csrc")
+PA_ERR_CUDA = -2
+
+
+class Config(ctypes.Structure):
+    _fields_ = [("device_id", ctypes.c_int32), ("max_sample_size", ctypes.c_uint32), ("reduction_exp", ctypes.c_uint32),
+                ("pre_mul_reduction_exp", ctypes.c_uint32), ("residual_limit", ctypes.c_float)]
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    out = tmp_path_factory.mktemp("engine") / "engine.so"
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    r = subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-w", "-I", os.path.join(cuda, "include"), "-I", CSRC,
+                        "-x", "c++", os.path.join(CSRC, "pa_engine.cu"), os.path.join(ROOT, "tests", "fake_runtime.cpp"),
+                        "-o", str(out)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    lib = ctypes.CDLL(str(out))
+    lib.fake_log.restype = ctypes.c_char_p
+    lib.fake_held.restype = ctypes.c_size_t
+    lib.fake_limit.argtypes = [ctypes.c_size_t]
+    lib.fake_residual.argtypes = [ctypes.c_float]
+    return lib
+
+
+class Engine:
+    def __init__(self, lib, n):
+        self.lib, self.ptr = lib, ctypes.c_void_p()
+        lib.fake_reset()
+        self.rc = lib.pa_create(ctypes.byref(Config(0, n, 0, 0, 0.0)), ctypes.byref(self.ptr))
+
+    def close(self):
+        self.lib.pa_destroy(self.ptr)
+
+    def set_seed(self, n, reuse=-1):
+        return self.lib.pa_set_seed(self.ptr, words(n).ctypes.data_as(ctypes.c_void_p), n, reuse)
+
+    def process(self, n, v, flags=DEFAULT_FLAGS):
+        ks, kr, out = words(n), words(v), np.zeros(max(n // 16, v // 8), np.uint8)
+        return self.lib.pa_process(self.ptr, *(a.ctypes.data_as(ctypes.c_void_p) for a in (ks, kr)), n, v, flags,
+                                   out.ctypes.data_as(ctypes.c_void_p), None)
+
+
+def words(bits):
+    return np.zeros(bits // 32, np.uint32)
+
+
+@pytest.mark.parametrize("n,flags,residual,fail,skip", [
+    (1 << 16, DEFAULT_FLAGS, 0.0, "direct", 0),         # the block's own launch
+    (1 << 16, DEFAULT_FLAGS, 0.0, "publish", 0),        # behind a short block
+    (1 << 18, DEFAULT_FLAGS, 0.0, "key", 0),
+    (1 << 18, DEFAULT_FLAGS, 0.0, "publish", 0),        # behind the FP32 passes
+    (1 << 18, DEFAULT_FLAGS, 0.5, "exact_seed", 0),     # the guard's recompute
+    (1 << 18, DEFAULT_FLAGS, 0.5, "exact", 0),
+    (1 << 18, DEFAULT_FLAGS, 0.5, "publish", 1),        # behind the recompute
+    (1 << 18, DEFAULT_FLAGS | FLAG_EXACT, 0.0, "publish", 0),
+    (1 << 24, DEFAULT_FLAGS, 0.0, "copy_async", 1)])    # key_rest's copy, the key's being under way
+def test_process_waits_before_it_returns_an_error(lib, n, flags, residual, fail, skip):
+    """The caller's buffers, pinned ones above all, are not read after the call: whatever it queued has finished."""
+    eng = Engine(lib, n)
+    assert eng.rc == 0 and eng.set_seed(n) == 0
+    lib.fake_reset()
+    lib.fake_residual(residual)
+    lib.fake_fail(fail.encode(), skip)
+    assert eng.process(n, n // 4 + n // 8, flags) == PA_ERR_CUDA
+    calls = lib.fake_log().decode().split("\n")[:-1]
+    failed = [i for i, c in enumerate(calls) if c == fail][skip]
+    assert "sync main" in calls[failed + 1:], calls
+    if fail == "copy_async":
+        assert "sync side" in calls[failed + 1:], calls
+    lib.fake_reset()
+    assert eng.process(n, n // 4 + n // 8, flags) == 0  # the engine goes on
+    eng.close()
+
+
+def test_set_seed_waits_before_it_returns_an_error(lib):
+    eng = Engine(lib, 1 << 18)
+    lib.fake_fail(b"seed", 0)
+    assert eng.set_seed(1 << 18) == PA_ERR_CUDA
+    calls = lib.fake_log().decode().split("\n")[:-1]
+    assert "sync main" in calls[calls.index("seed") + 1:], calls
+    eng.close()
