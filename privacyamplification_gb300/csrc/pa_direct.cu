@@ -154,7 +154,6 @@ __global__ void __launch_bounds__(32 * kWarps, 4) k_direct(const uint32_t* __res
     }
     if (ONE)
         for (uint32_t q = threadIdx.x; q < nwords; q += 32 * kWarps) out[q] = held[q];
-    if (dc.clock && threadIdx.x == 0) clock_end(dc.clock);
     // The placed seed's popcount, once per seed and placement, by up to kCounters CTAs: the last of them to add its share
     // to cnt[2] (arrivals above bit 48) takes the sum and leaves zero.  One CTA took 20 us at 2^20 bits, 270 at 2^24.
     const uint32_t counters = min(gridDim.x, kCounters);
@@ -179,6 +178,7 @@ __global__ void __launch_bounds__(32 * kWarps, 4) k_direct(const uint32_t* __res
             }
         }
     }
+    if (dc.clock && threadIdx.x == 0) clock_end(dc.clock);
 }
 
 template <int M>

@@ -19,18 +19,16 @@ namespace pa {
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// A block's time on the GPU's global timer: its first kernel stores the start and clears the end, every CTA of its last
-// kernel raises the end.  Two timed events around a block took 5.5 us of the stream (2^12 bits 8.5 -> 3.0 us a block)
-// and kept the next block's first kernel from being launched early.
+// A block's time on the GPU's global timer: its first kernel stores the start, every CTA of its last kernel raises the
+// end.  The end is not cleared (the timer only grows, so that a later block's is above it): where first and last kernel are
+// one, a clear could come after another CTA's end.  Two timed events around a block took 5.5 us of the stream (2^12 bits
+// 8.5 -> 3.0 us a block) and kept the next block's first kernel from being launched early.
 __device__ __forceinline__ unsigned long long global_ns() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
     return t;
 }
-__device__ __forceinline__ void clock_start(unsigned long long* clock) {
-    clock[0] = global_ns();
-    clock[1] = 0ull;
-}
+__device__ __forceinline__ void clock_start(unsigned long long* clock) { clock[0] = global_ns(); }
 // By one thread per CTA, after its last stores.
 __device__ __forceinline__ void clock_end(unsigned long long* clock) { atomicMax(clock + 1, global_ns()); }
 
