@@ -84,6 +84,8 @@ pa::Scratch scratch(pa_engine* e) { return {e->d_work, e->d_work2, e->d_planes, 
 
 int build_exact_seed(pa_engine* e, const BlockGeom& g, cudaStream_t s);
 
+constexpr size_t kLaneUnits = 3;  // chunk buffers of lane 1: row pass, column pass, window spectrum
+
 int build_spectrum(pa_engine* e, const BlockGeom& g, cudaStream_t s) {
     if (g.exact_only) return build_exact_seed(e, g, s);
     int rc = ensure_maps(e, g);
@@ -147,12 +149,9 @@ int own_block(pa_engine* e, const uint32_t* d_ks, const uint32_t* d_kr, const Bl
     return rc ? cuda_fail(e, (cudaError_t)rc) : PA_OK;
 }
 
-// Scratch of the exact path: 2 P words beside the P of d_work.  Engines for n > 2^27 take the last two of the chunk
-// buffers, which hold key spectra or row products only.
-uint32_t* exact_scratch(pa_engine* e) {
-    if (!e->d_chunk) return reinterpret_cast<uint32_t*>(e->d_work2);
-    return reinterpret_cast<uint32_t*>(e->d_chunk + (pa::chunk_units(e->cap_log_np) - 2) * (size_t(1) << 26));
-}
+// Scratch of the exact path: 2 P words beside the P of d_work.  Engines for n > 2^27 take the second chunk lane's row-pass
+// and column-pass buffers, which hold nothing from one block to the next.
+uint32_t* exact_scratch(pa_engine* e) { return reinterpret_cast<uint32_t*>(e->d_chunk ? e->d_chunk : e->d_work2); }
 
 int build_exact_seed(pa_engine* e, const BlockGeom& g, cudaStream_t s) {
     int rc = pa::launch_exact_seed(g, e->d_seed, e->d_exact_seed, exact_scratch(e), s, e->d_words->clock);
@@ -163,9 +162,9 @@ int build_exact_seed(pa_engine* e, const BlockGeom& g, cudaStream_t s) {
 }
 
 // n > 2^27: the block in 2^27-bit FP32 transforms (pa_chunk.cu).  Block popcounts are not formed on this path
-// (take_stats reports 0).  Lane 0 has d_work / d_work2 and the block's stream, lane 1 the first two chunk buffers and
-// `side` (free here because the block waited for key_rest's copy).  A seed that is kept has its window spectra kept
-// too, as long as they all fit (up to three rows) and the next block has the same rows and columns.
+// (take_stats reports 0).  Lane 0 has the one-pass path's buffers and the block's stream, lane 1 the first three chunk
+// buffers and `side` (free here because the block waited for key_rest's copy).  A seed that is kept has its window spectra
+// kept too, where they all fit and the next block has the same rows and columns.
 int chunked_block(pa_engine* e, const uint32_t* d_ks, const uint32_t* d_kr, const BlockGeom& g, uint32_t flags,
                   uint32_t* d_out, cudaStream_t s) {
     BlockGeom gc;
@@ -175,26 +174,34 @@ int chunked_block(pa_engine* e, const uint32_t* d_ks, const uint32_t* d_kr, cons
     rc = ensure_maps(e, gc);
     if (rc) return rc;
     const size_t nc = size_t(1) << gc.log_n;  // complex values per buffer
+    float2* const units = e->d_chunk + kLaneUnits * nc;
     if (e->lane_maps_key != pa_host::maps_key(gc)) {
+        e->unit_maps.resize(std::min(e->chunk_count, pa::kChunkCols));
         rc = pa::make_pass_maps(gc, e->d_chunk, e->d_chunk + nc, &e->lane_maps);
+        for (size_t k = 0; k < e->unit_maps.size() && !rc; ++k)
+            rc = pa::make_pass_maps(gc, units + k * nc, e->d_work2, &e->unit_maps[k]);
         if (rc) return cuda_fail(e, (cudaError_t)rc);
         e->lane_maps_key = pa_host::maps_key(gc);
     }
-    const size_t wwords = 2 * (side / 32u);
-    uint32_t* st = e->d_stage;
     pa::ChunkBuffers cb{};
-    cb.lane[0] = {scratch(e), st, s};
-    cb.lane[1] = {{e->d_chunk, e->d_chunk + nc, st + 2 * wwords, e->d_err, &e->lane_maps}, st + wwords, e->side};
+    cb.lane[0].sc = scratch(e);
+    cb.lane[0].spec = e->d_spec;
+    cb.lane[0].s = s;
+    cb.lane[1].sc = {e->d_chunk, e->d_chunk + nc, nullptr, e->d_err, &e->lane_maps};
+    cb.lane[1].spec = e->d_chunk + 2 * nc;
+    cb.lane[1].s = e->side;
+    pa::chunk_staging(e->cap_log_np, e->d_stage, e->d_chunk_cnt, e->d_planes, &cb);
     cb.fork = e->lane_fork;
     cb.join = e->lane_join;
-    cb.units = e->d_chunk + 2 * nc;
-    cb.cnt = reinterpret_cast<unsigned long long*>(st + 3 * wwords + 64);
+    cb.units = units;
+    cb.count = e->chunk_count;
+    cb.unit_maps = e->unit_maps.data();
     const pa::ChunkPlan p = pa::chunk_plan(g);
     const bool ready = e->chunk_valid && e->chunk_rows == p.rows && e->chunk_cols == p.cols;
-    e->chunk_valid = false;
+    e->spec_valid = e->chunk_valid = false;
     rc = pa::launch_chunked_block(g, gc, e->d_seed, d_ks, d_kr, flags, d_out, cb, ready, e->d_resid, e->num_sms, s);
     if (rc) return cuda_fail(e, (cudaError_t)rc);
-    e->chunk_valid = p.slots == p.diagonals;
+    e->chunk_valid = pa::chunk_keeps(p, e->chunk_count);
     e->chunk_rows = p.rows;
     e->chunk_cols = p.cols;
     return PA_OK;
@@ -340,11 +347,7 @@ int pa_kernels_per_block(uint32_t n, uint32_t v, uint32_t flags) {
     BlockGeom g;
     if (make_geom(n, v, flags, nullptr, &g)) return 0;
     if (flags & PA_FLAG_EXACT) return pa::exact_kernel_count(g);
-    if (g.exact_only) {
-        BlockGeom gc;
-        if (make_geom(2u << pa::kChunkLog, 1u << pa::kChunkLog, 0u, nullptr, &gc)) return 0;
-        return pa::chunk_kernel_count(g, gc);
-    }
+    if (g.exact_only) return pa::chunk_kernel_count(g);
     return pa::kernel_count_key_block(g);
 }
 
@@ -404,9 +407,11 @@ int pa_create(const pa_config* cfg, pa_engine** out) {
     if ((err = cudaMalloc(&e->d_work2, (np_fp32 / 2) * sizeof(float2))) != cudaSuccess) return fail(err);
     if ((err = cudaMalloc(&e->d_exact_seed, np / 4 * sizeof(uint32_t))) != cudaSuccess) return fail(err);
     if (np > np_fp32) {
-        const size_t units = pa::chunk_units(e->cap_log_np);
+        e->chunk_count = (uint32_t)pa::chunk_units(e->cap_log_np);
+        const size_t units = kLaneUnits + e->chunk_count, staging = pa::chunk_staging_words(e->cap_log_np);
         if ((err = cudaMalloc(&e->d_chunk, units * (np_fp32 / 2) * sizeof(float2))) != cudaSuccess) return fail(err);
-        if ((err = cudaMalloc(&e->d_stage, pa::chunk_staging_words() * sizeof(uint32_t))) != cudaSuccess) return fail(err);
+        if ((err = cudaMalloc(&e->d_stage, staging * sizeof(uint32_t))) != cudaSuccess) return fail(err);
+        if ((err = cudaMalloc(&e->d_chunk_cnt, pa::kChunkCounts * sizeof(*e->d_chunk_cnt))) != cudaSuccess) return fail(err);
     }
     if ((err = cudaMalloc(&e->d_words, sizeof(pa_engine::Words))) != cudaSuccess) return fail(err);
     cudaMemset(e->d_words, 0, sizeof(pa_engine::Words));
@@ -440,6 +445,7 @@ void pa_destroy(pa_engine* e) {
     cudaFree(e->d_work2);
     cudaFree(e->d_chunk);
     cudaFree(e->d_stage);
+    cudaFree(e->d_chunk_cnt);
     cudaFree(e->d_words);
     cudaFreeHost(e->h_words);
     cudaFree(e->d_planes);

@@ -43,10 +43,13 @@ struct pa_engine {
     pa::BlockGeom exact_geom{};
     pa::PassMaps maps{};        // tensor maps for the geometry maps_key
     int maps_key = -1;
-    // blocks of n > 2^27 (pa_chunk.cu): chunk_units() buffers of 2^26 complex (lane 1's two, seed and key spectra, a row
-    // product), the lanes' seed windows, lane 1's bit planes and the popcounts; the window spectra in place, if any
+    // blocks of n > 2^27 (pa_chunk.cu): buffers of 2^26 complex (lane 1's three, then chunk_count for the key's row passes
+    // and kept window spectra), staging, popcounts, and the window spectra in place, if any
     float2* d_chunk = nullptr;
+    uint32_t chunk_count = 0;
     uint32_t* d_stage = nullptr;
+    unsigned long long* d_chunk_cnt = nullptr;
+    std::vector<pa::PassMaps> unit_maps;  // over the row passes
     bool chunk_valid = false;
     uint32_t chunk_rows = 0, chunk_cols = 0;
     // lane 1: tensor maps over its buffers, its stream is `side`, and the events the lanes fork and join on

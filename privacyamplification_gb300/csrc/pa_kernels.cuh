@@ -149,9 +149,8 @@ int make_group_maps(const BlockGeom& g, const float2* Y, const float2* Z, uint32
 // columns, over `blocks` consecutive blocks.
 int encode_pass_maps(int log_n1, int log_n2, uint32_t cpt, const float2* Y, const float2* Z, CUtensorMap* out,
                      uint32_t blocks = 1);
-// xspec: a seed pass that stores real spectra (columns of 2^12; see pass_b_tiles).
 int launch_pass_b(const BlockGeom& g, bool seed, const PassMaps& maps, float2* Y, float2* Z, float2* spec, int* err,
-                  int num_sms, cudaStream_t s, const Group& gp = kOneBlock, bool xspec = false);
+                  int num_sms, cudaStream_t s, const Group& gp = kOneBlock);
 // A group's pass B with columns of 2^LOGL (pa_group.cu), grid and shared memory as launch_pass_b chose.
 template <int LOGL>
 int launch_pass_b_group(bool seed, dim3 grid, size_t smem, const CUtensorMap& mapY, float2* Y, float2* Z,
@@ -199,32 +198,43 @@ int launch_direct(const BlockGeom& g, const uint32_t* seed, const uint32_t* key_
                   uint32_t flags, uint32_t* out_words, cudaStream_t s, const DirectCounts& dc = kNoCounts);
 int exact_kernel_count(const BlockGeom& g);
 
-// Blocks beyond the single-pass FP32 size (pa_chunk.cu): side x side chunks as transforms of n' = 2 side bits on
-// the FP32 path, summed per row as spectra.  gc: geometry of a chunk transform (n' = 2 side, v' = side, no flags).
-// resid_bits receives the largest residual.
+// Blocks beyond the single-pass FP32 size (pa_chunk.cu): side x side chunks as transforms of n' = 2 side bits on the
+// FP32 path, each rounded by itself.  gc: geometry of a chunk transform (n' = 2 side, v' = side, no flags).
+// resid_bits receives the largest chunk's residual.
 constexpr int kChunkLog = 26;
 struct ChunkPlan {
     uint32_t side, rows, cols, diagonals;
-    uint32_t slots;  // seed spectra held at a time
 };
 ChunkPlan chunk_plan(const BlockGeom& g);
-int chunk_kernel_count(const BlockGeom& g, const BlockGeom& gc);
-// A lane of the chunk transforms: row-pass and column-pass buffers, bit planes, a seed window, a stream.
+int chunk_kernel_count(const BlockGeom& g);
+// One of two lanes that take the diagonals in turn: its row-pass, column-pass and bit-plane buffers with their maps, a
+// seed window (2 side bits) and its spectrum, a chunk's result (side bits), the rows' sums over the lane's chunks (side
+// bits per row), (key, seed) popcount pairs per column, and a stream.
 struct ChunkLane {
     Scratch sc;
-    uint32_t* window;
+    float2* spec;
+    uint32_t *window, *result, *rows;
+    unsigned long long* pairs;
     cudaStream_t s;
 };
 struct ChunkBuffers {
-    ChunkLane lane[2];        // lane 0 runs on the block's stream
-    cudaEvent_t fork, join;   // the lanes synchronise with
-    float2* units;            // seed spectra, key spectra, one row product: N complex each
-    unsigned long long* cnt;  // popcounts: 128 words
+    ChunkLane lane[2];       // lane 0 runs on the block's stream
+    cudaEvent_t fork, join;  // the lanes synchronise with
+    // Buffers of N = 2^26 complex: the row passes of the first key columns, as many as there are; then, where all of
+    // them fit too, the window spectra of a kept seed.
+    float2* units;
+    uint32_t count;
+    const PassMaps* unit_maps;       // over the first units' row passes
+    unsigned long long *key_cnt, *seed_cnt;  // popcounts per column and per kept window
 };
-// Buffers of N = 2^26 complex for blocks of cyclic length up to 2^log_np: lane 1's two and `units`.
-size_t chunk_units(int log_np);
-size_t chunk_staging_words();
-// seed_ready: the spectra of all the block's windows (at most `slots`) are already in place.
+constexpr uint32_t kChunkCols = 1u << (30 - kChunkLog);           // most columns, and rows
+constexpr uint32_t kChunkCounts = 7 * kChunkCols;                 // popcounts: two lanes' pairs, columns' and windows'
+size_t chunk_units(int log_np);                                   // buffers that serve blocks of cyclic length 2^log_np
+size_t chunk_staging_words(int log_np);                           // the lanes' windows, results and rows, lane 1's planes
+void chunk_staging(int log_np, uint32_t* staging, unsigned long long* counts, uint32_t* planes0, ChunkBuffers* cb);
+// The block's window spectra are kept in the units from one block of a seed to the next.
+bool chunk_keeps(const ChunkPlan& p, uint32_t units);
+// seed_ready: they are in place.
 int launch_chunked_block(const BlockGeom& g, const BlockGeom& gc, const uint32_t* seed, const uint32_t* key_start,
                          const uint32_t* key_rest, uint32_t flags, uint32_t* out_words, const ChunkBuffers& cb,
                          bool seed_ready, unsigned int* resid_bits, int num_sms, cudaStream_t s);

@@ -8,7 +8,7 @@
 //   Y        N complex64, row m1 = N2 values in "pair" order: float4 p holds columns p and N2-p
 //            (p = 0 holds 0 and N2/2)                               -- pass A writes, pass B rewrites
 //   spec     N complex64, the seed's packed spectrum (E, A) / (2 Np) in the thread order of pass B, see
-//            spectrum_pair (sums over chunks keep the real spectrum instead)
+//            spectrum_pair
 //   planes   parity bits, [t][m1][N2/32 words], bit m2 of row m1 -- pass C writes
 //   out      v/8 bytes in the reference byte order                  -- k_finish
 // Each pass is one persistent CTA per SM walking rows (A, C) or column tiles (B); the FFT data stay
@@ -282,8 +282,7 @@ struct PassBBases {
 // FUSED: a seed used by this block only.  Every tile is taken twice, first from the seed's row pass output
 // (mapYs) as a seed pass, its spectrum tile parked in this CTA's CPT * L values of `spec` (written and read
 // back by the same CTA a tile later, so it stays in L2), then from the key's (mapY) as a key pass against it.
-// XSPEC (a seed pass): spectra as X = real spectrum instead of the (E, A) form, for sums of products (pa_chunk.cu).
-template <int LOGL, bool SEED, int NT, bool GRP = false, bool FUSED = false, bool XSPEC = false>
+template <int LOGL, bool SEED, int NT, bool GRP = false, bool FUSED = false>
 __device__ __forceinline__ void pass_b_tiles(const CUtensorMap* mapY, const float2* __restrict__ Y,
                                              float2* __restrict__ Z, const BlockGeom& g, float2* __restrict__ spec,
                                              int* err, int early, uint32_t first, uint32_t stride,
@@ -292,7 +291,6 @@ __device__ __forceinline__ void pass_b_tiles(const CUtensorMap* mapY, const floa
     constexpr int L = 1 << LOGL, E = 32, CPT = 32 * NT / L, LR = L / 16, SP = TileStride<L>::value;
     constexpr bool TMA = CPT <= 128;              // box inner extent 2*CPT floats <= 256
     static_assert(!FUSED || (TMA && !GRP && !SEED), "the fused pass is a one-block key pass with TMA tiles");
-    static_assert(!XSPEC || SEED, "only a seed pass stores real spectra");
     constexpr int BOXR = L < 256 ? L : 256;       // rows per box
     using P = Plan<LOGL>;
     using Lin = MapLinear<NT>;
@@ -335,9 +333,8 @@ __device__ __forceinline__ void pass_b_tiles(const CUtensorMap* mapY, const floa
     auto unit_block = [&](int u) { return GRP ? (uint32_t)(u >> tshift) : 0u; };
     const int t = threadIdx.x;
     const int pp = t / LR, jj = t % LR;
-    // Spectrum scale, for transforms of samples at -2 x (pass A): X form 2 (-2 X) sc = -X / (4 Np), (E, A) form
-    // E sc and A sc with 1 / (4 N) = 1 / (2 Np).
-    const float sc = XSPEC ? 1.0f / (float)(16ull << g.log_np) : 1.0f / (float)(2ull << g.log_np);
+    // Spectrum scale, for transforms of samples at -2 x (pass A): E sc and A sc with 1 / (4 N) = 1 / (2 Np).
+    const float sc = 1.0f / (float)(2ull << g.log_np);
     {
         float2 w[4];
         if (P::NSTAGE == 2) {
@@ -567,34 +564,24 @@ __device__ __forceinline__ void pass_b_tiles(const CUtensorMap* mapY, const floa
                         }
                         if (u == 0) {  // DC (dropped) and Nyquist in slot (0, 0); then the self pair N/2
                             float2 z = sm[padk<4>(0)];
-                            const float nyq = XSPEC ? 2.0f * (z.x - z.y) : z.x - z.y;
+                            const float nyq = z.x - z.y;
                             if (sd) {
-                                tspec[spec_index<LR>(0, 0)] = make_float2(XSPEC ? nyq * sc : 0.5f * nyq * sc, 0.f);
+                                tspec[spec_index<LR>(0, 0)] = make_float2(0.5f * nyq * sc, 0.f);
                             } else {
                                 float pn = nyq * tspec[spec_index<LR>(0, 0)].x;
                                 sm[padk<4>(0)] = make_float2(pn, -pn);
                             }
-                            ka = kb = L / 2;
-                            k = n2 * (uint32_t)(L / 2);
-                            if (!XSPEC) {  // w^2 = -1, V = 0: Y = Z Zs, in the pair's one slot
-                                float2* self = &sm[padk<4>(L / 2)];
-                                float2* slot = &tspec[spec_index<LR>(0, L / 2)];
-                                if (sd) *slot = cscale(*self, sc);
-                                else *self = cmul(*self, *slot);
-                                continue;
-                            }
+                            // self pair: w^2 = -1, V = 0: Y = Z Zs, in the pair's one slot
+                            float2* self = &sm[padk<4>(L / 2)];
+                            float2* slot = &tspec[spec_index<LR>(0, L / 2)];
+                            if (sd) *slot = cscale(*self, sc);
+                            else *self = cmul(*self, *slot);
+                            continue;
                         }
                         float2 za = sm[ca * SP + padk<4>(ka)], zb = sm[ca * SP + padk<4>(kb)];
                         int ia = spec_index<LR>(ca, ka), ib = spec_index<LR>(cb, kb);
                         if (sd) {
-                            if (XSPEC) {
-                                float2 xa, xb;
-                                real_split(za, zb, expmi_pi(k, g.log_n), xa, xb);
-                                tspec[ia] = cscale(xa, sc);
-                                tspec[ib] = cscale(xb, sc);
-                            } else {
-                                spectrum_pair(za, zb, sc, tspec[ia], tspec[ib]);
-                            }
+                            spectrum_pair(za, zb, sc, tspec[ia], tspec[ib]);
                         } else {
                             float2 qa, qb;
                             const float2 fb = tspec[ib];
@@ -624,18 +611,7 @@ __device__ __forceinline__ void pass_b_tiles(const CUtensorMap* mapY, const floa
                 const float2* sb = sbase + (2 * pp + 1) * 16 * LR + jj;
                 float2* da = tspec + (2 * pp) * 16 * LR + jj;
                 float2* db = tspec + (2 * pp + 1) * 16 * LR + jj;
-                if (XSPEC) {
-                    // W_2N^{p + N2 (jj + LR r)} = W_2N^{p + N2 jj} * W_32^r
-                    const float2 base = expmi_pi(p + n2 * (uint32_t)jj, g.log_n);
-#pragma unroll
-                    for (int r = 0; r < 16; ++r) {
-                        const float2 w = r ? cmul(base, make_float2(w32(r).x, -w32(r).y)) : base;
-                        float2 xa, xb;
-                        real_split(x[r], x[16 + 15 - r], w, xa, xb);
-                        __stcs(da + r * LR, cscale(xa, sc));
-                        __stcs(db + (15 - r) * LR, cscale(xb, sc));
-                    }
-                } else if (sd) {
+                if (sd) {
 #pragma unroll
                     for (int r = 0; r < 16; ++r) {
                         float2 ea, eb;

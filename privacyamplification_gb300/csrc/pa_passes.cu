@@ -7,7 +7,7 @@
 //   Y        N complex64, row m1 = N2 values in "pair" order: float4 p holds columns p and N2-p
 //            (p = 0 holds 0 and N2/2)                               -- pass A writes, pass B rewrites
 //   spec     N complex64, the seed's packed spectrum (E, A) / (2 Np) in the thread order of pass B, see
-//            spectrum_pair (sums over chunks keep the real spectrum instead)
+//            spectrum_pair
 //   planes   parity bits, [t][m1][N2/32 words], bit m2 of row m1 -- pass C writes
 //   out      v/8 bytes in the reference byte order                  -- k_finish
 // Each pass is one persistent CTA per SM walking rows (A, C) or column tiles (B); the FFT data stay
@@ -187,11 +187,11 @@ __global__ void __launch_bounds__((1 << LOGL) / 32, 1)
 
 // One block (a group's pass B is k_pass_b_group in pa_group.cu: pass B runs at the 128-register limit
 // of two CTAs per SM, and this kernel keeps its pointers in the constant bank instead of registers).
-template <int LOGL, bool SEED, bool XSPEC = false>
+template <int LOGL, bool SEED>
 __global__ void __launch_bounds__(256, 2)
     k_pass_b(const __grid_constant__ CUtensorMap mapY, const float2* __restrict__ Y, float2* __restrict__ Z,
              BlockGeom g, float2* __restrict__ spec, int* err, int early) {
-    pass_b_tiles<LOGL, SEED, 256, false, false, XSPEC>(&mapY, Y, Z, g, spec, err, early, blockIdx.x, gridDim.x);
+    pass_b_tiles<LOGL, SEED, 256>(&mapY, Y, Z, g, spec, err, early, blockIdx.x, gridDim.x);
 }
 
 template <int LOGL, int KEEP8>
@@ -396,7 +396,7 @@ static constexpr size_t pass_b_smem() {
 
 template <int LOGL>
 static int pass_b_l(const BlockGeom& g, bool seed, const PassMaps& maps, float2* Y, float2* Z, float2* spec,
-                    int* err, int num_sms, cudaStream_t s, const Group& gp, bool xspec) {
+                    int* err, int num_sms, cudaStream_t s, const Group& gp) {
     constexpr int L = 1 << LOGL, CPT = 8192 / L;
     const size_t smem = pass_b_smem<LOGL>();
     // a group's CTAs walk all its blocks' tiles (one dimension); one block's walk its own
@@ -424,9 +424,6 @@ static int pass_b_l(const BlockGeom& g, bool seed, const PassMaps& maps, float2*
     const size_t bytes = smem + (size_t)early * box;
     if (gp.e) return launch_pass_b_group<LOGL>(seed, grid, bytes, maps.y, Y, Z, spec, g, err, early, gp, s);
     auto kernel = seed ? k_pass_b<LOGL, true> : k_pass_b<LOGL, false>;
-    if constexpr (LOGL == 12) {  // the columns of the chunk transforms
-        if (xspec) kernel = k_pass_b<LOGL, true, true>;
-    }
     smem_attr(kernel, bytes);
     return (int)launch_pdl(kernel, grid, 256, bytes, s, maps.y, Y, Z, g, spec, err, early);
 }
@@ -550,9 +547,8 @@ int launch_rows_both(const BlockGeom& g, const uint32_t* key, const uint32_t* se
 }
 
 int launch_pass_b(const BlockGeom& g, bool seed, const PassMaps& maps, float2* Y, float2* Z, float2* spec, int* err,
-                  int num_sms, cudaStream_t s, const Group& gp, bool xspec) {
-    if (xspec && (!seed || g.log_n1 != 12)) return (int)cudaErrorInvalidValue;
-#define C(LG) pass_b_l<LG>(g, seed, maps, Y, Z, spec, err, num_sms, s, gp, xspec)
+                  int num_sms, cudaStream_t s, const Group& gp) {
+#define C(LG) pass_b_l<LG>(g, seed, maps, Y, Z, spec, err, num_sms, s, gp)
     PA_COLS_DISPATCH(g.log_n1, C)
 #undef C
 }
