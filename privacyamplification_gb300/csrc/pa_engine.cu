@@ -405,14 +405,8 @@ int pa_create(const pa_config* cfg, pa_engine** out) {
     if ((err = cudaMalloc(&e->d_work, (np_fp32 / 2) * sizeof(float2))) != cudaSuccess) return fail(err);
     if ((err = cudaMalloc(&e->d_spec, (np_fp32 / 2) * sizeof(float2))) != cudaSuccess) return fail(err);
     if ((err = cudaMalloc(&e->d_work2, (np_fp32 / 2) * sizeof(float2))) != cudaSuccess) return fail(err);
-    if ((err = cudaMalloc(&e->d_exact_seed, np / 4 * sizeof(uint32_t))) != cudaSuccess) return fail(err);
-    if (np > np_fp32) {
-        e->chunk_count = (uint32_t)pa::chunk_units(e->cap_log_np);
-        const size_t units = kLaneUnits + e->chunk_count, staging = pa::chunk_staging_words(e->cap_log_np);
-        if ((err = cudaMalloc(&e->d_chunk, units * (np_fp32 / 2) * sizeof(float2))) != cudaSuccess) return fail(err);
-        if ((err = cudaMalloc(&e->d_stage, staging * sizeof(uint32_t))) != cudaSuccess) return fail(err);
-        if ((err = cudaMalloc(&e->d_chunk_cnt, pa::kChunkCounts * sizeof(*e->d_chunk_cnt))) != cudaSuccess) return fail(err);
-    }
+    const size_t exact_words = std::max<size_t>(np / 8, size_t(1) << 16);
+    if ((err = cudaMalloc(&e->d_exact_seed, exact_words * sizeof(uint32_t))) != cudaSuccess) return fail(err);
     if ((err = cudaMalloc(&e->d_words, sizeof(pa_engine::Words))) != cudaSuccess) return fail(err);
     cudaMemset(e->d_words, 0, sizeof(pa_engine::Words));
     e->d_cnt = e->d_words->cnt;
@@ -425,6 +419,21 @@ int pa_create(const pa_config* cfg, pa_engine** out) {
         // one spectrum tile per CTA: two CTAs per SM, at most one per tile of the largest block
         e->park_ctas = std::min<uint32_t>(2u * (uint32_t)e->num_sms, (uint32_t)((np / 2) / 8192u));
         if ((err = cudaMalloc(&e->d_park, e->park_ctas * pa::kParkBytes)) != cudaSuccess) return fail(err);
+    }
+    if (np > np_fp32) {
+        const size_t staging = pa::chunk_staging_words(e->cap_log_np);
+        if ((err = cudaMalloc(&e->d_stage, staging * sizeof(uint32_t))) != cudaSuccess) return fail(err);
+        if ((err = cudaMalloc(&e->d_chunk_cnt, pa::kChunkCounts * sizeof(*e->d_chunk_cnt))) != cudaSuccess) return fail(err);
+        // What is held beside lane 1's buffers only saves repeated transforms (2^29 bits: 14.0 ms a block with all of it,
+        // 16.0 with none): beside other tenants of the memory it is halved until it fits.
+        for (uint32_t count = (uint32_t)pa::chunk_units(e->cap_log_np);; count /= 2u) {
+            e->chunk_count = count;
+            err = cudaMalloc(&e->d_chunk, (kLaneUnits + count) * (np_fp32 / 2) * sizeof(float2));
+            if (err == cudaSuccess) break;
+            cudaGetLastError();  // reported here or not an error
+            e->d_chunk = nullptr;
+            if (err != cudaErrorMemoryAllocation || count == 0) return fail(err);
+        }
     }
     *out = e;
     return PA_OK;

@@ -35,7 +35,7 @@ struct pa_engine {
     float2* d_work2 = nullptr;  // pass B output (tile-major)
     float2* d_spec = nullptr;
     int* d_err = nullptr;       // device error word of the bounded TMA waits (in d_words)
-    uint32_t* d_exact_seed = nullptr;  // the seed's transform (exact path), up to Np / 4 words
+    uint32_t* d_exact_seed = nullptr;  // the seed's transform (exact path), up to Np / 8 words
     bool exact_valid = false;          // d_exact_seed matches the current seed for exact_geom
     bool last_exact = false;           // the last block ran on the exact path
     bool last_direct = false;          // the last block was a short one (pa_direct.cu)

@@ -166,7 +166,7 @@ int launch_exact_block(const BlockGeom&, const uint32_t*, const uint32_t*, const
 ChunkPlan chunk_plan(const BlockGeom&) { return {}; }
 int chunk_kernel_count(const BlockGeom&) { return 1; }
 size_t chunk_units(int log_np) { return 3 * (size_t(1) << (log_np - 27)) + 1; }
-size_t chunk_staging_words(int) { return 1; }
+size_t chunk_staging_words(int log_np) { return ((2 * (3 + (size_t(1) << (log_np - 26))) + 2) << 21) + 64; }
 void chunk_staging(int, uint32_t*, unsigned long long*, uint32_t*, ChunkBuffers*) {}
 bool chunk_keeps(const ChunkPlan&, uint32_t) { return true; }
 int launch_chunked_block(const BlockGeom&, const BlockGeom&, const uint32_t*, const uint32_t*, const uint32_t*, uint32_t,

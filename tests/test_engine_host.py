@@ -92,3 +92,32 @@ def test_set_seed_waits_before_it_returns_an_error(lib):
     calls = lib.fake_log().decode().split("\n")[:-1]
     assert "sync main" in calls[calls.index("seed") + 1:], calls
     eng.close()
+
+
+BUFFER = 1 << 29  # 2^26 complex values
+
+
+@pytest.mark.parametrize("logn,buffers", [(28, 7), (29, 13), (30, 25)])
+def test_large_engine_fits_beside_other_tenants(lib, logn, buffers):
+    """An engine above 2^27 bits needs what one chunk of 2^27 bits at a time takes (`buffers` with everything at the block's
+    own length); more, where it can be had, holds transforms that are otherwise repeated."""
+    n = 1 << logn
+    eng = Engine(lib, n)
+    assert eng.rc == 0
+    most = lib.fake_held()
+    eng.close()
+    assert lib.fake_held() == 0
+    small = 4 * (n // 8 + 256) + (1 << 24) + 256 + 304 * 65536 + 4096  # keys, seed, result, bit planes, park, words
+    for limit in (most, most - 1, buffers * BUFFER + small):
+        eng = Engine(lib, n)
+        eng.close()
+        lib.fake_limit(limit)
+        eng.rc = lib.pa_create(ctypes.byref(Config(0, n, 0, 0, 0.0)), ctypes.byref(eng.ptr))
+        assert eng.rc == 0 and lib.fake_held() <= limit, limit
+        eng.close()
+        assert lib.fake_held() == 0
+    lib.fake_reset()
+    lib.fake_limit(3 * BUFFER)  # not even the passes' own
+    assert lib.pa_create(ctypes.byref(Config(0, n, 0, 0, 0.0)), ctypes.byref(eng.ptr)) == PA_ERR_CUDA
+    assert lib.fake_held() == 0
+    lib.fake_reset()

@@ -105,3 +105,31 @@ def test_padded_block_between_one_pass_blocks(engine):
         out = engine.process(ks, kr, n, v, flags)
         assert engine.last_stats.exact == path
         assert np.array_equal(out, O.ntt(seed, ks, kr, n, v, flags)), (v, flags)
+
+
+@pytest.mark.parametrize("room", [3.85, 4.4, 5.6])
+def test_little_memory(pa_lib, room):
+    """Engines beside a tenant that leaves `room` GB: fewer or no row passes held, the same result.  2^28 bits need 3.7 GB and
+    take 7.4 where they can."""
+    torch = pytest.importorskip("torch")
+    n, v = 1 << 28, (1 << 26) + (1 << 25)
+    seed = seed_of(n, 13)
+    ks, kr = block(n, v, 14)
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    hog = torch.empty(free - int(room * 1e9), dtype=torch.uint8, device="cuda")
+    try:
+        with pa.Engine(max_sample_size=n) as eng:
+            left, _ = torch.cuda.mem_get_info()
+            assert left < room * 1e9 - 3.6e9
+            eng.set_seed(seed, n, -1)
+            outs = [eng.process(ks, kr, n, v) for _ in range(2)]
+            assert eng.last_stats.exact == 2
+            print("room %.2f GB: %.2f ms a block" % (room, eng.last_stats.gpu_ms))
+            exact = eng.process(ks, kr, n, v, DEFAULT | pa.FLAG_EXACT)
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    want = O.ntt(seed, ks, kr, n, v)
+    for out in outs + [exact]:
+        assert np.array_equal(out, want)
