@@ -547,10 +547,15 @@ int pa_process(pa_engine* e, const uint32_t* key_start, const uint32_t* key_rest
     cudaStream_t s = e->stream;
     WaitOnError wait{s, e->side};
     // Pinned inputs of up to 256 KB are read where they lie: a copy of any size holds the stream for 11 us (2^16 bits
-    // host to host 40 -> 29.5 us a call; longer keys come faster by a copy).  key_rest is first read by the block's last
-    // kernel: a long one is copied on the side stream (after whatever the engine stream had queued) while the passes run.
+    // host to host 40 -> 29.5 us a call; longer keys come faster by a copy).  A transform reads the key once (2^18 .. 2^22
+    // bits, keys of 3 to 230 KB: 1 to 4 us a call less than with a copy); a word-by-word block reads it once per cluster
+    // of CTAs, mostly from cache, which is level with a copy or faster up to 32 KB and slower from 64 KB on (128 KB 41 us
+    // against 36, 256 KB 58 against 48).  key_rest is first read by the block's last kernel: a long one is copied on the side stream
+    // (after whatever the engine stream had queued) while the passes run.
+    const bool reread = (flags & PA_FLAG_EXACT) ? pa::direct_geom(g) : pa::short_geom(g);
     const size_t ks_bytes = (size_t)(g.h / 32u + 1u) * 4u;
-    const uint32_t* d_ks = ks_bytes <= pa_engine::kStageBytes ? pinned_view(key_start) : nullptr;
+    const uint32_t* d_ks = ks_bytes <= (reread ? pa_engine::kRereadBytes : pa_engine::kStageBytes) ? pinned_view(key_start)
+                                                                                                   : nullptr;
     if (!d_ks) {
         PA_CUDA(e, cudaMemcpyAsync(e->d_key_start, key_start, ks_bytes, cudaMemcpyHostToDevice, s));
         d_ks = e->d_key_start;

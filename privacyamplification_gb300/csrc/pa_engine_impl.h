@@ -78,6 +78,7 @@ struct pa_engine {
     unsigned int* d_resid = nullptr;      // &d_words->resid
     // pinned: the words, then short results (kStageBytes), which are handed over once the words are read
     static constexpr size_t kStageBytes = size_t(256) << 10;
+    static constexpr size_t kRereadBytes = size_t(48) << 10;  // pinned keys that a block's CTAs read again and again
     Words* h_words = nullptr;
     uint8_t* h_stage = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;

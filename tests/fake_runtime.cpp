@@ -123,8 +123,8 @@ cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cu
 }
 
 namespace pa {
-bool short_geom(const BlockGeom& g) { return g.n <= 1u << 17; }
-bool direct_geom(const BlockGeom& g) { return g.n <= 1u << 17; }
+bool short_geom(const BlockGeom& g) { return (g.h + 1ull) * g.out_bits <= 5ull << 31 && g.h <= 1u << 21; }
+bool direct_geom(const BlockGeom& g) { return (g.h + 1ull) * g.out_bits <= 1ull << 34 && g.h <= 1u << 22; }
 bool direct_overlap(const BlockGeom&, const uint32_t*, const uint32_t*) { return false; }
 int make_pass_maps(const BlockGeom&, const float2*, const float2*, PassMaps*) { return 0; }
 int stage_count_key_block(const BlockGeom&) { return 1; }

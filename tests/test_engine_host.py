@@ -62,9 +62,9 @@ def words(bits):
     (1 << 16, DEFAULT_FLAGS, 0.0, "publish", 0),        # behind a short block
     (1 << 18, DEFAULT_FLAGS, 0.0, "key", 0),
     (1 << 18, DEFAULT_FLAGS, 0.0, "publish", 0),        # behind the FP32 passes
-    (1 << 18, DEFAULT_FLAGS, 0.5, "exact_seed", 0),     # the guard's recompute
-    (1 << 18, DEFAULT_FLAGS, 0.5, "exact", 0),
-    (1 << 18, DEFAULT_FLAGS, 0.5, "publish", 1),        # behind the recompute
+    (1 << 19, DEFAULT_FLAGS, 0.5, "exact_seed", 0),     # the guard's recompute
+    (1 << 19, DEFAULT_FLAGS, 0.5, "exact", 0),
+    (1 << 19, DEFAULT_FLAGS, 0.5, "publish", 1),        # behind the recompute
     (1 << 18, DEFAULT_FLAGS | FLAG_EXACT, 0.0, "publish", 0),
     (1 << 24, DEFAULT_FLAGS, 0.0, "copy_async", 1)])    # key_rest's copy, the key's being under way
 def test_process_waits_before_it_returns_an_error(lib, n, flags, residual, fail, skip):
@@ -82,6 +82,21 @@ def test_process_waits_before_it_returns_an_error(lib, n, flags, residual, fail,
         assert "sync side" in calls[failed + 1:], calls
     lib.fake_reset()
     assert eng.process(n, n // 4 + n // 8, flags) == 0  # the engine goes on
+    eng.close()
+
+
+@pytest.mark.parametrize("h,v,flags,copies", [
+    (393184, 512, DEFAULT_FLAGS, 0), (393216, 512, DEFAULT_FLAGS, 1),    # word by word: 48 KB, one word more
+    (393216, 512, DEFAULT_FLAGS | FLAG_EXACT, 1), (1048576, 512, DEFAULT_FLAGS, 1),
+    (655360, 393216, DEFAULT_FLAGS, 0), (655360, 393216, DEFAULT_FLAGS | FLAG_EXACT, 0),  # transforms: 80 KB
+    (2097120, 1 << 20, DEFAULT_FLAGS, 0), (2097152, 1 << 20, DEFAULT_FLAGS, 1)])          # 256 KB, one word more
+def test_pinned_keys_read_in_place(lib, h, v, flags, copies):
+    """A pinned key that every cluster of CTAs reads again is copied above 48 KB, one that is read once above 256 KB."""
+    eng = Engine(lib, h + v)
+    assert eng.rc == 0 and eng.set_seed(h + v) == 0
+    lib.fake_reset()
+    assert eng.process(h + v, v, flags) == 0
+    assert lib.fake_log().decode().split("\n").count("copy_async") == copies
     eng.close()
 
 
