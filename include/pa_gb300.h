@@ -70,7 +70,8 @@ typedef struct pa_stats {
     uint64_t popcount_key;    /* Hamming weight of key_start (count_one_of_global_key) */
     uint64_t popcount_seed;   /* Hamming weight of the seed (count_one_of_global_seed) */
     float gpu_ms;             /* device time of the block: its first kernel's start to its last one's end on the GPU's
-                                 global timer (CUDA events around a block above 2^27 bits and around a batch) */
+                                 global timer (CUDA events around a block above 2^27 bits, 0 if that was captured,
+                                 and around a batch) */
     int32_t seed_uses_left;   /* remaining blocks for the cached seed, -1 = unlimited */
     int32_t exact;            /* 0: FP32 path, one pass, or a short block, word by word; 2: FP32 path as 2^27-bit chunk blocks (n > 2^27);
                                  1: exact path (guard fallback or PA_FLAG_EXACT).  Popcounts are 0 for 1, 2 */

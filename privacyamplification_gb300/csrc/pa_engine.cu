@@ -327,7 +327,10 @@ int take_stats(pa_engine* e, pa_stats* st, float* resid_out) {
         st->popcount_key = counted ? cnt[0] : 0;
         st->popcount_seed = counted ? cnt[1] : 0;
         float ms = w.clock[1] > w.clock[0] ? (float)((double)(w.clock[1] - w.clock[0]) * 1e-6) : 0.f;
-        if (e->last_chunked) cudaEventElapsedTime(&ms, e->ev0, e->ev1);
+        if (e->last_chunked && cudaEventElapsedTime(&ms, e->ev0, e->ev1) != cudaSuccess) {
+            cudaGetLastError();  // recorded in a captured block: no time, and not an error of the next launch
+            ms = 0.f;
+        }
         st->gpu_ms = ms;
         st->seed_uses_left = e->seed_left < 0 ? -1 : (int32_t)e->seed_left;
         st->exact = e->last_exact ? 1 : (e->last_chunked ? 2 : 0);

@@ -119,3 +119,43 @@ def test_captured_seed(pa_lib, n, v):
             assert eng.sync().popcount_seed == O.popcount(seed, n)
         del graph
         torch.cuda.synchronize()
+
+
+def test_captured_chunks(pa_lib):
+    """A block above 2^27 bits: replays with another seed, statistics behind a replay, and ordinary blocks behind those."""
+    torch = pytest.importorskip("torch")
+    n, v = (1 << 27) + 32, 1 << 26
+    rng = np.random.default_rng(28)
+    words = lambda k: rng.integers(0, 1 << 32, k, dtype=np.uint64).astype(np.uint32)
+    dev = lambda a: torch.from_numpy(a.view(np.int32).copy()).cuda()
+    seeds = [words(n // 32) for _ in range(2)]
+    ks, kr = O.key_split(words(n // 32 + 1), n, v)
+    want = [O.ntt(seed, ks, kr, n, v) for seed in seeds]
+    d_seeds, d_ks, d_kr = [dev(s) for s in seeds], dev(ks), dev(kr)
+    out = torch.zeros(v // 8, dtype=torch.uint8, device="cuda")
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    with pa.Engine(max_sample_size=n) as eng:
+        def block(k):
+            eng.set_seed_device(d_seeds[k].data_ptr(), n, -1, stream=stream.cuda_stream)
+            eng.process_device(d_ks.data_ptr(), d_kr.data_ptr(), n, v, out.data_ptr(), stream=stream.cuda_stream)
+
+        block(0)
+        assert eng.sync().gpu_ms > 0
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream, capture_error_mode="relaxed"):
+            eng.process_device(d_ks.data_ptr(), d_kr.data_ptr(), n, v, out.data_ptr(), stream=stream.cuda_stream)
+        for k in (1, 0):
+            eng.set_seed_device(d_seeds[k].data_ptr(), n, -1, stream=stream.cuda_stream)
+            out.zero_()
+            torch.cuda.synchronize()
+            graph.replay()
+            assert eng.sync().exact == 2
+            assert np.array_equal(out.cpu().numpy(), want[k])
+            out.zero_()
+            torch.cuda.synchronize()
+            block(1 - k)
+            assert eng.sync().gpu_ms > 0
+            assert np.array_equal(out.cpu().numpy(), want[1 - k])
+        del graph
+        torch.cuda.synchronize()
