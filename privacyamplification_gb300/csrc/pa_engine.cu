@@ -176,9 +176,8 @@ int chunked_block(pa_engine* e, const uint32_t* d_ks, const uint32_t* d_kr, cons
     const size_t nc = size_t(1) << gc.log_n;  // complex values per buffer
     float2* const units = e->d_chunk + kLaneUnits * nc;
     if (e->lane_maps_key != pa_host::maps_key(gc)) {
-        e->unit_maps.resize(std::min(e->chunk_count, pa::kChunkCols));
         rc = pa::make_pass_maps(gc, e->d_chunk, e->d_chunk + nc, &e->lane_maps);
-        for (size_t k = 0; k < e->unit_maps.size() && !rc; ++k)
+        for (uint32_t k = 0; k < std::min(e->chunk_count, pa::kChunkCols) && !rc; ++k)
             rc = pa::make_pass_maps(gc, units + k * nc, e->d_work2, &e->unit_maps[k]);
         if (rc) return cuda_fail(e, (cudaError_t)rc);
         e->lane_maps_key = pa_host::maps_key(gc);
@@ -195,7 +194,7 @@ int chunked_block(pa_engine* e, const uint32_t* d_ks, const uint32_t* d_kr, cons
     cb.join = e->lane_join;
     cb.units = units;
     cb.count = e->chunk_count;
-    cb.unit_maps = e->unit_maps.data();
+    cb.unit_maps = e->unit_maps;
     const pa::ChunkPlan p = pa::chunk_plan(g);
     const bool ready = e->chunk_valid && e->chunk_rows == p.rows && e->chunk_cols == p.cols;
     e->spec_valid = e->chunk_valid = false;
@@ -408,7 +407,7 @@ int pa_create(const pa_config* cfg, pa_engine** out) {
     if ((err = cudaMalloc(&e->d_work, (np_fp32 / 2) * sizeof(float2))) != cudaSuccess) return fail(err);
     if ((err = cudaMalloc(&e->d_spec, (np_fp32 / 2) * sizeof(float2))) != cudaSuccess) return fail(err);
     if ((err = cudaMalloc(&e->d_work2, (np_fp32 / 2) * sizeof(float2))) != cudaSuccess) return fail(err);
-    const size_t exact_words = std::max<size_t>(np / 8, size_t(1) << 16);
+    const size_t exact_words = std::max<size_t>(np / 8, std::min<size_t>(np / 4, size_t(1) << 16));  // below 2^18: unused
     if ((err = cudaMalloc(&e->d_exact_seed, exact_words * sizeof(uint32_t))) != cudaSuccess) return fail(err);
     if ((err = cudaMalloc(&e->d_words, sizeof(pa_engine::Words))) != cudaSuccess) return fail(err);
     cudaMemset(e->d_words, 0, sizeof(pa_engine::Words));

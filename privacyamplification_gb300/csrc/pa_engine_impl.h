@@ -49,7 +49,7 @@ struct pa_engine {
     uint32_t chunk_count = 0;
     uint32_t* d_stage = nullptr;
     unsigned long long* d_chunk_cnt = nullptr;
-    std::vector<pa::PassMaps> unit_maps;  // over the row passes
+    pa::PassMaps unit_maps[pa::kChunkCols]{};  // over the row passes
     bool chunk_valid = false;
     uint32_t chunk_rows = 0, chunk_cols = 0;
     // lane 1: tensor maps over its buffers, its stream is `side`, and the events the lanes fork and join on
