@@ -23,8 +23,10 @@ class Config(ctypes.Structure):
 def lib(tmp_path_factory):
     out = tmp_path_factory.mktemp("engine") / "engine.so"
     cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
-    r = subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-w", "-I", os.path.join(cuda, "include"), "-I", CSRC,
-                        "-x", "c++", os.path.join(CSRC, "pa_engine.cu"), os.path.join(ROOT, "tests", "fake_runtime.cpp"),
+    # -Bsymbolic: a CUDA runtime that the process has loaded must not take the fake one's place
+    r = subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-Wl,-Bsymbolic", "-w",
+                        "-I", os.path.join(cuda, "include"), "-I", CSRC, "-x", "c++",
+                        os.path.join(CSRC, "pa_engine.cu"), os.path.join(ROOT, "tests", "fake_runtime.cpp"),
                         "-o", str(out)], capture_output=True, text=True)
     assert r.returncode == 0, r.stderr
     lib = ctypes.CDLL(str(out))
