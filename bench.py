@@ -725,7 +725,7 @@ def run_big29(args, force_exact):
     _line(METRIC, args.steps * n / t / 1e9, UNIT, args.steps, args.warmup, t / args.steps * 1e3,
           "n=2^29 (h=n/2+n/8, v=n/4+n/8), dynamic seed, " + path,
           {"exact": st.exact, "max_residual": st.max_residual, "clocks": clk.summary(),
-           "dtype": "u32 (mod p)" if force_exact else "f32"})
+           "dtype": "GF(2^32) elements, bit-sliced u32" if force_exact else "f32"})
     eng.close()
 
 

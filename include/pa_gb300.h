@@ -20,8 +20,9 @@
  *   - Precision: the FP32 FFT path measures every block's largest distance of an output value to the
  *     nearest integer; above residual_limit pa_process recomputes the block on the exact path, which
  *     forms the product over GF(2) itself (additive FFT).  Single short blocks (up to 1.07e10 bit
- *     products, n = 2^17) are multiplied word by word, which is exact.  Blocks with n > 2^27 (up to 2^30) run as 2^27-bit FP32 chunk blocks
- *     (large-block decomposition) under the same guard.
+ *     products, n = 2^17) are multiplied word by word, which is exact.  Blocks with n > 2^27 (up to 2^30)
+ *     run as 2^27-bit FP32 chunk blocks (large-block decomposition), each rounded by itself, under the
+ *     same guard.
  *
  * All functions return 0 (PA_OK) or a negative PA_ERR_* code; nothing exits the process.
  * An engine is bound to one CUDA device and must be used from one host thread at a time.
@@ -77,7 +78,8 @@ typedef struct pa_stats {
                                  1: exact path (guard fallback or PA_FLAG_EXACT).  Popcounts are 0 for 1, 2 */
 } pa_stats;
 
-/* Creates an engine on cfg->device_id and allocates its HBM working set for n <= max_sample_size.
+/* Creates an engine on cfg->device_id and allocates its HBM working set for n <= max_sample_size (1.8 GB at 2^27; above,
+ * 3.7 / 4.0 / 4.7 GB at 2^28 / 2^29 / 2^30, and up to 7.4 / 11.0 / 18.1 GB where there is room, for faster blocks).
  * Replaces the allocation part of main() (PrivacyAmplification.cu:1536-1606). */
 PA_API int pa_create(const pa_config* cfg, pa_engine** out);
 PA_API void pa_destroy(pa_engine* e);
