@@ -87,11 +87,14 @@ def test_seed_kept_across_lengths(engine):
     n = (1 << 28) + 4096
     seed = seed_of(n, 11)
     engine.set_seed(seed, n, -1)
+    want = {}
     for v in (100663296, 33554432, 100663328, 100663296):
         ks, kr = block(n, v, v)
         out = engine.process(ks, kr, n, v)
         assert engine.last_stats.exact == 2
-        assert np.array_equal(out, O.ntt(seed, ks, kr, n, v)), v
+        if v not in want:
+            want[v] = O.ntt(seed, ks, kr, n, v)
+        assert np.array_equal(out, want[v]), v
 
 
 def test_padded_block_between_one_pass_blocks(engine):
